@@ -34,20 +34,25 @@ __global__ void assign_bins_kernel(int *vox_bin, int *counts, const float *b1map
                                    const float *params, int nparams, long long natoms,
                                    int nblocks, long long nvox) {
     long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (v >= nvox) return;
-    float gt = b1map[v];
-    int best = 0;
-    float best_abs = 10.f;
-    for (int k = 0; k < nblocks; k++) {
-        float b1 = params[(long long)k * natoms * nparams + 3];
-        float d = fabsf(gt - b1);
-        if (d < best_abs) {
-            best_abs = d;
-            best = k;
+    int best = -1;
+    if (v < nvox) {
+        float gt = b1map[v];
+        best = 0;
+        float best_abs = 10.f;
+        for (int k = 0; k < nblocks; k++) {
+            float b1 = params[(long long)k * natoms * nparams + 3];
+            float d = fabsf(gt - b1);
+            if (d < best_abs) {
+                best_abs = d;
+                best = k;
+            }
         }
+        vox_bin[v] = best;
     }
-    vox_bin[v] = best;
-    atomicAdd(&counts[best], 1);
+    // one atomic per warp and bin: neighbouring voxels share bins, and single
+    // atomics queue on a few counters (57,600 voxels, 41 bins: 20 -> 6 us)
+    const unsigned same = __match_any_sync(0xffffffffu, best);
+    if (best >= 0 && (threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&counts[best], __popc(same));
 }
 
 // Exclusive scans of the per-bin voxel counts (slots) and voxel tiles.
@@ -69,9 +74,13 @@ __global__ void scan_bins_kernel(const int *counts, long long *slot_start, long 
 __global__ void scatter_bins_kernel(long long *perm, long long *cursor, const int *vox_bin,
                                     long long nvox) {
     long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (v >= nvox) return;
-    long long pos = atomicAdd((unsigned long long *)&cursor[vox_bin[v]], 1ull);
-    perm[pos] = v;
+    const int bin = v < nvox ? vox_bin[v] : -1, lane = threadIdx.x & 31;
+    const unsigned same = __match_any_sync(0xffffffffu, bin);
+    const int leader = __ffs(same) - 1;
+    unsigned long long pos = 0;
+    if (bin >= 0 && lane == leader) pos = atomicAdd((unsigned long long *)&cursor[bin], (unsigned long long)__popc(same));
+    pos = __shfl_sync(0xffffffffu, pos, leader) + __popc(same & ((1u << lane) - 1));
+    if (bin >= 0) perm[pos] = v;
 }
 
 // Bins that all hold every voxel: slot_start[b] = b*nvox, tile_start[b] = b*vt.

@@ -38,6 +38,7 @@
 
 #include "common.h"
 #include "match_tc.h"
+#include "match_tc_plan.cuh"
 #include "sm100.cuh"
 #include "svd.h"
 
@@ -51,36 +52,7 @@ __global__ void scatter_bins_kernel(long long *perm, long long *cursor, const in
 
 namespace tc {
 
-constexpr int BM = 128;                 // voxels per tile (TMEM lanes)
-constexpr int BA = 128;                 // atoms per tile
-constexpr int BN = 2 * BA;              // B rows per tile
-constexpr int BK = 64;                  // bf16 per 128-byte swizzled row
-constexpr int BK8 = 128;                // e4m3 per 128-byte swizzled row
-constexpr float E4M3_MAX = 448.f;       // largest finite E4M3 value
-constexpr int STAGES = 4;
-constexpr int A_BYTES = BM * BK * 2;    // 16 KB
-constexpr int B_BYTES = BN * BK * 2;    // 32 KB
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int TOPK_MAX = 16;
-constexpr int NLISTS = 2;               // top-k lists per voxel (one per half tile)
-constexpr int THREADS = 320;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;
-constexpr uint32_t TMEM_COLS = 512;
-
 __device__ int g_device_error;
-
-struct Args {
-    const long long *tile_start;  // [nbins + 1]
-    int nbins;
-    long long bin_natoms;
-    int nk;                       // K chunks of BK
-    int tile_stride;              // atom tiles visited in the order (at * tile_stride) % natiles
-    uint32_t idesc;               // tcgen05 instruction descriptor
-    const float *ascale2;         // E4M3: [NATOMS] 1 / (atom scale)^2
-    float *top_s;                 // [slots][TOPK]
-    int *top_i;                   // [slots][TOPK]
-    int *err;
-};
 
 __device__ __forceinline__ int find_bin(const long long *tile_start, int nbins, long long item) {
     int lo = 0, hi = nbins - 1;
@@ -92,19 +64,33 @@ __device__ __forceinline__ int find_bin(const long long *tile_start, int nbins, 
 }
 
 // Insertion into a descending list; strict '>' keeps earlier (lower-index)
-// entries ahead of equal scores.
+// entries ahead of equal scores.  Every slot takes its old entry, the new one
+// or its upper neighbour's, so the slots do not wait for one another.
 template <int TOPK>
 __device__ __forceinline__ void topk_insert(float *ts, int *ti, float s, int i) {
+    bool gt[TOPK];
 #pragma unroll
-    for (int k = 0; k < TOPK; k++) {
-        bool gt = s > ts[k];
-        float t = ts[k];
-        int u = ti[k];
-        ts[k] = gt ? s : t;
-        ti[k] = gt ? i : u;
-        s = gt ? t : s;
-        i = gt ? u : i;
+    for (int k = 0; k < TOPK; k++) gt[k] = s > ts[k];
+#pragma unroll
+    for (int k = TOPK - 1; k > 0; k--) {
+        ts[k] = gt[k - 1] ? ts[k - 1] : gt[k] ? s : ts[k];
+        ti[k] = gt[k - 1] ? ti[k - 1] : gt[k] ? i : ti[k];
     }
+    ts[0] = gt[0] ? s : ts[0];
+    ti[0] = gt[0] ? i : ti[0];
+}
+
+// Stores a held score and its atom where `take` (predicated stores: a branch
+// per score costs the warp its reconvergence); returns the entries added.
+__device__ __forceinline__ int hold_if(bool take, uint32_t addr, float s, int i) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.s32 p, %0, 0;\n\t"
+        "@p st.shared.f32 [%1], %2;\n\t"
+        "@p st.shared.s32 [%1+%4], %3;\n\t}" ::"r"((int)take),
+        "r"(addr), "f"(s), "r"(i), "n"(HOLD * EPI_THREADS * 4)
+        : "memory");
+    return take ? 1 : 0;
 }
 
 // FP8: E4M3 operands on kind::f8f6f4, one 128-byte row holding 128 elements
@@ -115,20 +101,28 @@ __device__ __forceinline__ void topk_insert(float *ts, int *ti, float s, int i) 
 // A tile is 64 voxels x 256 atoms; the two lanes of a voxel swap halves of
 // each 32-column load and keep a top-k each over half the atoms, merged at
 // the end of the item.
-template <int TOPK, bool FP8, bool IMAG>
+// SPLIT: every 64-element row chunk holds 32 elements of K as BF16 pairs,
+// their leading parts first, then the remainders (v = hi + lo to 2^-17): a
+// stage's six MMAs sum hi hi + lo hi + hi lo, a product to about 2^-17 of its
+// size at three times the MMA work, from the same ring as the plain form.
+template <int TOPK, bool FP8, bool IMAG, bool SPLIT = false>
 __global__ void __launch_bounds__(THREADS, 1)
 match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Args p) {
     constexpr int BKE = FP8 ? BK8 : BK;   // K elements per stage
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], tfull[2], tempty[2], mma_done;
     __shared__ uint32_t tmem_base_sh;
+    __shared__ volatile unsigned long long bound_sh[2][BM];  // see insert_held
     unsigned char *smem = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    constexpr int IPT = IMAG ? 2 : 1;       // work items per 128-slot tile
     constexpr int APT = IMAG ? BN : BA;     // atoms per B tile
-    const long long total = p.tile_start[p.nbins] * IPT;
-    const int natiles = (int)((p.bin_natoms + APT - 1) / APT);
+    constexpr int VPT = IMAG ? BM / 2 : BM; // voxels per item
+    constexpr bool HELD = TOPK > 4;         // (four slots insert at once)
+    const int natiles = (p.chunk_natoms + APT - 1) / APT;
+    const long long item0 = p.tile_start[p.bin_lo];
+    const TailPlan plan = tail_plan(p.tile_start[p.bin_hi] - item0, gridDim.x, natiles, p.max_parts);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *p.plan = plan;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) {
@@ -137,9 +131,10 @@ match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         }
         for (int a = 0; a < 2; a++) {
             sm100::mbar_init(&tfull[a], 1);
-            sm100::mbar_init(&tempty[a], 256);
+            sm100::mbar_init(&tempty[a], EPI_THREADS);
         }
         sm100::mbar_init(&mma_done, 1);
+        for (int r = 0; r < 2 * BM; r++) bound_sh[r / BM][r % BM] = ~0ull;  // (no such work unit)
         sm100::fence_mbar_init();
         sm100::prefetch_tmap(&tmA);
         sm100::prefetch_tmap(&tmB);
@@ -161,13 +156,17 @@ match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             int issued[STAGES];
             for (int s = 0; s < STAGES; s++) issued[s] = -1;
             bool ok = true;
-            for (long long item = blockIdx.x; item < total && ok; item += gridDim.x) {
-                const int bin = find_bin(p.tile_start, p.nbins, item / IPT);
+            for (long long w = blockIdx.x; w < plan.work && ok; w += gridDim.x) {
+                const WorkUnit u = work_unit(plan, w, 0);
+                const long long item = item0 + u.item;
+                const int bin = find_bin(p.tile_start, p.nbins, item) - p.bin_lo;
                 const int vrow = (int)(item * BM);
-                for (int at = 0; at < natiles && ok; at++) {
-                    const long long pt = (long long)at * p.tile_stride % natiles;
-                    const int brow = IMAG ? (int)((long long)bin * p.bin_natoms + pt * APT)
-                                          : (int)(2 * ((long long)bin * p.bin_natoms + pt * BA));
+                TileWalk tile(u, p.tile_stride, natiles);
+                const int brow0 = (IMAG ? 1 : 2) * (int)((long long)bin * p.chunk_natoms);
+                for (int at = u.part; at < natiles && ok; at += u.step, tile.next()) {
+                    const int brow = brow0 + tile.at * BN;
+                    // (unrolled like the MMA issuer's loop: 5.70 -> 5.62 ms there)
+#pragma unroll 4
                     for (int kc = 0; kc < p.nk; kc++) {
                         if (!sm100::mbar_wait(&empty[stage], phase ^ 1, p.err, 1)) {
                             ok = false;
@@ -197,33 +196,45 @@ match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             uint32_t phase = 0, aphase = 0;
             bool ok = true;
             const uint32_t idesc = p.idesc;
-            for (long long item = blockIdx.x; item < total && ok; item += gridDim.x) {
-                for (int at = 0; at < natiles && ok; at++) {
+            // (the address field counts 16 bytes and cannot overflow: 227 KB)
+            const uint64_t desc0 = sm100::make_sw128_desc(sm100::smem_u32(smem));
+            for (long long w = blockIdx.x; w < plan.work && ok; w += gridDim.x) {
+                const WorkUnit u = work_unit(plan, w, 0);
+                for (int at = u.part; at < natiles && ok; at += u.step) {
                     if (!sm100::mbar_wait(&tempty[acc], aphase ^ 1, p.err, 2)) {
                         ok = false;
                         break;
                     }
                     sm100::tc_fence_after();
                     const uint32_t d = tmem + (uint32_t)(acc * BN);
+                    // One thread issues every MMA, so what it does between
+                    // two of them can leave the tensor core waiting: the
+                    // descriptors are sums of a constant and the stage's
+                    // offset, and the unrolled loop overlaps a stage's wait
+                    // with the address work of the next (16,384 voxels
+                    // against 111,008 complex atoms, FP16: 6.26 -> 5.69 ms
+                    // from the unrolling alone).
+#pragma unroll 4
                     for (int kc = 0; kc < p.nk; kc++) {
                         if (!sm100::mbar_wait(&full[stage], phase, p.err, 3)) {
                             ok = false;
                             break;
                         }
                         sm100::tc_fence_after();
-                        const uint32_t a_addr = sm100::smem_u32(smem + stage * STAGE_BYTES);
-                        const uint32_t b_addr = a_addr + A_BYTES;
-                        // four MMAs of 32 bytes of K each (16 bf16 / 32 e4m3)
+                        const uint64_t a_desc = desc0 + (uint32_t)stage * (STAGE_BYTES / 16);
+                        const uint64_t b_desc = a_desc + A_BYTES / 16;
+                        // four MMAs of 32 bytes of K each (16 bf16 / 32 e4m3);
+                        // SPLIT: hi hi, lo hi and hi lo, two of 32 bytes each
 #pragma unroll
-                        for (int k = 0; k < 4; k++) {
-                            if (FP8)
-                                sm100::mma_f8f6f4(d, sm100::make_sw128_desc(a_addr + k * 32),
-                                                  sm100::make_sw128_desc(b_addr + k * 32), idesc,
-                                                  (kc > 0 || k > 0) ? 1u : 0u);
+                        for (int k = 0; k < (SPLIT ? 6 : 4); k++) {
+                            const uint32_t acc_in = k > 0 ? 1u : kc > 0 ? 1u : 0u;
+                            if (SPLIT)
+                                sm100::mma_bf16(d, a_desc + (k / 2 == 1 ? 4 : 0) + (k & 1) * 2,
+                                                b_desc + (k / 2 == 2 ? 4 : 0) + (k & 1) * 2, idesc, acc_in);
+                            else if (FP8)
+                                sm100::mma_f8f6f4(d, a_desc + k * 2, b_desc + k * 2, idesc, acc_in);
                             else
-                                sm100::mma_bf16(d, sm100::make_sw128_desc(a_addr + k * 32),
-                                                sm100::make_sw128_desc(b_addr + k * 32), idesc,
-                                                (kc > 0 || k > 0) ? 1u : 0u);
+                                sm100::mma_bf16(d, a_desc + k * 2, b_desc + k * 2, idesc, acc_in);
                         }
                         sm100::mma_commit(&empty[stage]);
                         if (++stage == STAGES) {
@@ -254,9 +265,17 @@ match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         int acc = 0;
         uint32_t aphase = 0;
         bool ok = true;
-        for (long long item = blockIdx.x; item < total && ok; item += gridDim.x) {
+        const int atom_end = p.atom0 + p.chunk_natoms;
+        float *hold_s = reinterpret_cast<float *>(smem + STAGES * STAGE_BYTES) + (threadIdx.x - 64);
+        int *hold_i = reinterpret_cast<int *>(smem + STAGES * STAGE_BYTES) + HOLD * EPI_THREADS + (threadIdx.x - 64);
+        const uint32_t hold_addr = sm100::smem_u32(hold_s);
+        for (long long w = blockIdx.x; w < plan.work && ok; w += gridDim.x) {
+            const WorkUnit u = work_unit(plan, w, p.cap / VPT - item0);
             const float *asc = nullptr;
-            if (FP8) asc = p.ascale2 + (long long)find_bin(p.tile_start, p.nbins, item / IPT) * p.bin_natoms;
+            if (FP8) asc = p.ascale2 + (long long)find_bin(p.tile_start, p.nbins, item0 + u.item) * p.bin_natoms;
+            // this thread's list (of the voxel's two; IMAG: the even lane's)
+            const long long slot = (item0 + u.list_item) * VPT + (IMAG ? row / 2 : row);
+            const long long o = (slot * NLISTS + half) * TOPK_MAX;
             float ts[TOPK];
             int ti[TOPK];
 #pragma unroll
@@ -264,7 +283,63 @@ match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 ts[k] = 0.f;
                 ti[k] = -1;
             }
-            for (int at = 0; at < natiles; at++) {
+            // HELD: scores above thr are held back and inserted together, the lanes'
+            // e-th held scores at a time: an insertion takes 16 dependent
+            // selects for the whole warp however few lanes insert.  C1, BF16
+            // top-16 (1.11 ms without an epilogue): 1.55 -> 1.36 ms with the
+            // held scores, the joint bound below and predicated stores.
+            // thr bounds the voxel's k-th best from below: the k-th best of
+            // any of its lists does (two per voxel, in two warps; IMAG: four,
+            // the lane pair's in each), and so does the smallest of several
+            // lists' n-th best when those make k entries together.  The other
+            // warp's half comes through shared memory, marked with its work
+            // unit (a slot of another unit is another voxel's).
+            float thr = 0.f;
+            int held = 0;
+            auto insert_held = [&]() {
+                const int most = __reduce_max_sync(0xffffffffu, held);
+#pragma unroll 1
+                for (int e = 0; e < most; e++) {
+                    const bool in = e < held;
+                    topk_insert<TOPK>(ts, ti, in ? hold_s[e * EPI_THREADS] : -1.f,
+                                      in ? hold_i[e * EPI_THREADS] : -1);
+                }
+                held = 0;
+                thr = ts[TOPK - 1];
+                float mine = ts[TOPK / 2 - 1];  // k / 2 entries of this half are at least this
+                if (IMAG) {
+                    const float last = __shfl_xor_sync(0xffffffffu, thr, 1);
+                    const float mid = __shfl_xor_sync(0xffffffffu, mine, 1);
+                    const float quart = __shfl_xor_sync(0xffffffffu, ts[TOPK / 4 - 1], 1);
+                    thr = fmaxf(fmaxf(thr, last), fminf(mine, mid));
+                    mine = fmaxf(fminf(ts[TOPK / 4 - 1], quart), fmaxf(mine, mid));
+                }
+                const unsigned long long word =
+                    ((unsigned long long)(unsigned)w << 32) | __float_as_uint(mine);
+                bound_sh[half][row] = word;
+                const unsigned long long theirs = bound_sh[half ^ 1][row];
+                if ((unsigned)(theirs >> 32) == (unsigned)w)
+                    thr = fmaxf(thr, fminf(mine, __uint_as_float((unsigned)theirs)));
+            };
+            // SPLIT: this thread's list instead, appended to in memory: every
+            // atom within the margin of the best score seen so far (by the
+            // lane pair of a voxel in the IMAG form).  An atom left out is
+            // certain to lose to the one that set that best.
+            constexpr int LISTS = split_lists(IMAG), CAPL = LIST_CAP / LISTS;
+            const long long lid = slot * LISTS + (IMAG ? 2 * half + (lane & 1) : half);
+            int ln = 0;
+            float best = 0.f, keep = 0.f, margin = 0.f;
+            if constexpr (SPLIT) {
+                margin = p.margin_rel * sqrtf(__uint_as_float(*p.norm2_bits));
+                if (p.resume) {
+                    ln = p.list_n[lid];
+                    best = p.list_best[lid];
+                    const float low = sqrtf(best) - margin;
+                    keep = low > 0.f ? low * low * (1.f - 0x1p-20f) : 0.f;
+                }
+            }
+            TileWalk tile(u, p.tile_stride, natiles);
+            for (int at = u.part; at < natiles; at += u.step, tile.next()) {
                 // every lane polls, then the warp reconverges and agrees
                 // before the warp-collective tcgen05.ld
                 const bool got = sm100::mbar_wait(&tfull[acc], aphase, p.err, 4);
@@ -274,8 +349,8 @@ match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 }
                 sm100::tc_fence_after();
                 const uint32_t taddr = tmem + (uint32_t)(acc * BN) + ((uint32_t)(lg * 32) << 16);
-                const int abase = (int)((long long)at * p.tile_stride % natiles) * APT;
-                const bool full_tile = (long long)abase + APT <= p.bin_natoms;
+                const int abase = p.atom0 + tile.at * APT;
+                const bool full_tile = abase + APT <= atom_end;
 #pragma unroll 1
                 for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); c++) {
                     float v[32];
@@ -294,8 +369,7 @@ match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                         for (int j = 0; j < 32; j++) am = fmaxf(am, fabsf(v[j]));
                         const float own = am * am;
                         const float bound = (own + __shfl_xor_sync(0xffffffffu, own, 1)) * (1.f + 0x1p-20f);
-                        const float thr = fmaxf(ts[TOPK - 1], __shfl_xor_sync(0xffffffffu, ts[TOPK - 1], 1));
-                        if (!__any_sync(0xffffffffu, bound > thr)) continue;
+                        if (!__any_sync(0xffffffffu, SPLIT ? bound >= keep : bound > thr)) continue;
                     }
                     // the 16 scores of this load, then one test of their
                     // maximum against the current k-th best before any insertion
@@ -317,22 +391,68 @@ match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 #pragma unroll
                         for (int j = 0; j < 16; j++) {
                             sc[j] = fmaf(v[2 * j], v[2 * j], v[2 * j + 1] * v[2 * j + 1]);
-                            if (FP8) sc[j] *= (full_tile || a0 + j < p.bin_natoms) ? __ldg(asc + a0 + j) : 0.f;
+                            if (FP8) sc[j] *= (full_tile || a0 + j < atom_end) ? __ldg(asc + a0 + j) : 0.f;
+                        }
+                    }
+                    if constexpr (SPLIT) {
+                        if (!full_tile) {
+#pragma unroll
+                            for (int j = 0; j < 16; j++)
+                                if (a0 + j >= atom_end) sc[j] = 0.f;
                         }
                     }
                     float mx = sc[0];
 #pragma unroll
                     for (int j = 1; j < 16; j++) mx = fmaxf(mx, sc[j]);
-                    // IMAG: the lane pair keeps two lists of one voxel; each
-                    // list's k-th best bounds the voxel's k-th best from
-                    // below, so a score must beat the larger of the two
-                    float thr = ts[TOPK - 1];
-                    if (IMAG) thr = fmaxf(thr, __shfl_xor_sync(0xffffffffu, thr, 1));
-                    if (mx > thr) {
+                    if constexpr (SPLIT) {
+                        const float both = IMAG ? fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1)) : mx;
+                        if (both > best) {
+                            best = both;
+                            const float low = sqrtf(best) - margin;
+                            keep = low > 0.f ? low * low * (1.f - 0x1p-20f) : 0.f;
+                        }
+                        if (mx >= keep && mx > 0.f) {
+                            float *ls = p.top_s + lid * CAPL;
+                            int *li = p.top_i + lid * CAPL;
 #pragma unroll
-                        for (int j = 0; j < 16; j++)
-                            if (sc[j] > fmaxf(thr, ts[TOPK - 1]) && (full_tile || a0 + j < p.bin_natoms))
-                                topk_insert<TOPK>(ts, ti, sc[j], a0 + j);
+                            for (int j = 0; j < 16; j++) {
+                                if (!(sc[j] >= keep && sc[j] > 0.f) || ln > CAPL) continue;
+                                if (ln == CAPL) {
+                                    // full: entries that the best has left
+                                    // behind go; none left to go: overflow
+                                    int k = 0;
+                                    for (int e = 0; e < CAPL; e++) {
+                                        const float s = ls[e];
+                                        if (s >= keep) {
+                                            ls[k] = s;
+                                            li[k++] = li[e];
+                                        }
+                                    }
+                                    ln = k < CAPL ? k : CAPL + 1;
+                                    if (ln > CAPL) continue;
+                                }
+                                ls[ln] = sc[j];
+                                li[ln++] = a0 + j;
+                            }
+                        }
+                        continue;
+                    }
+                    if constexpr (!HELD) {
+                        if (mx > thr) {
+#pragma unroll
+                            for (int j = 0; j < 16; j++)
+                                if (sc[j] > fmaxf(thr, ts[TOPK - 1]) && (full_tile || a0 + j < atom_end))
+                                    topk_insert<TOPK>(ts, ti, sc[j], a0 + j);
+                            thr = ts[TOPK - 1];
+                        }
+                        if (IMAG) thr = fmaxf(thr, __shfl_xor_sync(0xffffffffu, thr, 1));
+                    } else if (__any_sync(0xffffffffu, mx > thr)) {
+#pragma unroll
+                        for (int j = 0; j < 16; j++) {
+                            if (j % 4 == 0 && __any_sync(0xffffffffu, held > HOLD - 4)) insert_held();
+                            held += hold_if(sc[j] > thr && (full_tile || a0 + j < atom_end),
+                                            hold_addr + held * (EPI_THREADS * 4), sc[j], a0 + j);
+                        }
                     }
                 }
                 sm100::tc_fence_before();
@@ -340,6 +460,13 @@ match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 acc ^= 1;
                 if (acc == 0) aphase ^= 1;
             }
+            if constexpr (SPLIT) {
+                p.list_n[lid] = ln;
+                p.list_best[lid] = best;
+                __syncwarp();
+                continue;
+            }
+            if constexpr (HELD) insert_held();
             if (IMAG) {
                 // the odd lane's list into the even lane's: the top-k of the union
                 float os[TOPK];
@@ -356,8 +483,6 @@ match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 }
             }
             if (!IMAG || !(lane & 1)) {
-                const long long slot = IMAG ? item * (BM / 2) + row / 2 : item * BM + row;
-                const long long o = (slot * NLISTS + half) * TOPK_MAX;
 #pragma unroll
                 for (int k = 0; k < TOPK_MAX; k++) {
                     p.top_s[o + k] = k < TOPK ? ts[k] : 0.f;
@@ -374,23 +499,24 @@ match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
 }
 
-// Padded bin layout: every B1 block's voxel slots start on a multiple of BM.
-__global__ void scan_padded_kernel(const int *counts, long long *tile_start, long long *cursor, int nbins) {
+// Padded bin layout: every B1 block's voxel slots start on a multiple of vt,
+// the voxels of an item.
+__global__ void scan_padded_kernel(const int *counts, long long *tile_start, long long *cursor, int nbins, int vt) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     long long t = 0;
     for (int b = 0; b < nbins; b++) {
         tile_start[b] = t;
-        cursor[b] = t * BM;
-        t += (counts[b] + BM - 1) / BM;
+        cursor[b] = t * vt;
+        t += (counts[b] + vt - 1) / vt;
     }
     tile_start[nbins] = t;
 }
 
-__global__ void global_bin_kernel(long long *tile_start, long long *perm, long long nvox, long long cap) {
+__global__ void global_bin_kernel(long long *tile_start, long long *perm, long long nvox, long long cap, int vt) {
     long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (s == 0) {
         tile_start[0] = 0;
-        tile_start[1] = (nvox + BM - 1) / BM;
+        tile_start[1] = (nvox + vt - 1) / vt;
     }
     if (s < cap) perm[s] = s < nvox ? s : -1;
 }
@@ -704,172 +830,203 @@ __global__ void pack_atoms_e4m3_kernel(unsigned char *B, float *ascale2, const f
     }
 }
 
+// Sums of NV values over the warp (NV a power of two <= 32), each in the
+// order of a butterfly over 16, 8, 4, 2, 1: at each level a lane hands the
+// half of its values that it does not keep to its partner, so NV values take
+// NV - 1 + log2(32 / NV) exchanges instead of 5 NV.  Returns value (lane * NV
+// / 32), the same on the 32 / NV lanes that hold it.
+template <int NV>
+__device__ __forceinline__ float warp_sums(float (&v)[NV], int lane) {
+    int n = NV;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (n > 1) {
+            n /= 2;
+            const bool up = lane & o;
+#pragma unroll
+            for (int i = 0; i < NV / 2; i++)
+                if (i < n) {
+                    const float got = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + n], o);
+                    v[i] = (up ? v[i + n] : v[i]) + got;
+                }
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+    return v[0];
+}
+
 // Exact FP32 rescoring of the top-k per voxel; one warp per slot.  The
 // scoring kernel leaves NLISTS lists of TOPK (by approximate score) per
-// voxel, one per half of the atom tiles; their TOPK best (ties to the lower
-// atom index) are rescored.  The map gets the candidate with the largest |s| (lowest
+// voxel and part of its item, one per half of the atom tiles; their TOPK
+// best (ties to the lower atom index) are rescored.  The map gets the candidate with the largest |s| (lowest
 // atom index on ties, nothing unless |s| > 0, like generate_maps' strict '>'
 // from 0).  VEC: two samples per 16-byte load (strides even, rows aligned).
 // ROWS: the atoms are Im rows of purely imaginary atoms, [NATOMS][atom_stride]
 // float (SNAPMRF_DICT_IMAG_ROWS); VEC then reads four samples per 16 bytes.
+// 16 candidates' rows and sums at once took 126 registers, 16 warps per SM,
+// and waited on latency (L2 at 12 % of its peak).  In batches of eight, 24 warps
+// per SM, the lanes' sums exchanged in 16 steps per batch instead of 80 and the
+// best found by the lanes together: 57,600 voxels x 16 candidates of T = 1000
+// 478 -> 424 us, which is 4.7 GB of rows from L2 at 11 TB/s.
+constexpr int kRescoreThreads = 256;
 template <int TOPK, bool VEC, bool ROWS = false>
-__global__ void rescore_kernel(float *maps, long long *index_out, const float *top_s, const int *top_i,
-                               const long long *perm, const long long *tile_start, int nbins, const int *vox_bin,
-                               const float2 *atoms, long long atom_stride, const float2 *img, long long img_stride,
-                               long long nreps, const float *params, int nparams, long long bin_natoms,
-                               const int *err, const float *atom_norms) {
+__global__ void __launch_bounds__(kRescoreThreads, 3)
+rescore_kernel(float *maps, long long *index_out, Lists lists, const long long *perm, const long long *tile_start,
+               int nbins, const int *vox_bin, const float2 *atoms, long long atom_stride, const float2 *img,
+               long long img_stride, long long nreps, const float *params, int nparams, long long bin_natoms,
+               const int *err, const float *atom_norms) {
+    __shared__ int scand[kRescoreThreads / 32][TOPK];
+    __shared__ float sscore[kRescoreThreads / 32][TOPK];
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const long long slot = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / 32;
-    const int lane = threadIdx.x % 32;
-    if (slot >= tile_start[nbins] * BM) return;
+    if (slot >= tile_start[nbins] * lists.vt) return;
     const long long v = perm[slot];
     if (v < 0) return;
     const long long bin = vox_bin ? vox_bin[v] : 0;
     static_assert(NLISTS * TOPK <= 32, "one lane per listed candidate");
-    const bool listed = lane < NLISTS * TOPK;
-    const long long o = (slot * NLISTS + lane / TOPK) * TOPK_MAX + lane % TOPK;
-    const int li = listed ? top_i[o] : -1;
-    const float ls = listed && li >= 0 ? top_s[o] : -1.f;
-    int rank = 0;
-#pragma unroll
-    for (int j = 0; j < NLISTS * TOPK; j++) {
-        const float sj = __shfl_sync(0xffffffffu, ls, j);
-        const int ij = __shfl_sync(0xffffffffu, li, j);
-        rank += sj > ls || (sj == ls && (ij < li || (ij == li && j < lane)));
-    }
-    int cand = -1;
-#pragma unroll
-    for (int k = 0; k < TOPK; k++) {
-        const unsigned m = __ballot_sync(0xffffffffu, listed && rank == k);
-        const int ik = __shfl_sync(0xffffffffu, li, m ? __ffs(m) - 1 : 0);
-        if (lane == k) cand = m ? ik : -1;
-    }
-    int ci[TOPK];
-    const float2 *row[TOPK];
-#pragma unroll
-    for (int k = 0; k < TOPK; k++) {
-        ci[k] = __shfl_sync(0xffffffffu, cand, k);
-        row[k] = atoms + (bin * bin_natoms + (ci[k] >= 0 ? ci[k] : 0)) * atom_stride;
-    }
-    float re[TOPK], im[TOPK];
-#pragma unroll
-    for (int k = 0; k < TOPK; k++) {
-        re[k] = 0.f;
-        im[k] = 0.f;
-    }
-    // Atoms as generated (atom_norms): 1 / ||d|| per candidate, formed as the
-    // dictionary's normalisation forms it, loaded ahead of the inner products
-    // so that the loads' latency is hidden.  Top-16: every lane loads and
-    // forms all 16; top-4 / 8: lane k loads candidate k's norm and forms its
-    // inverse after the inner products (each the faster on C1).
-    float inv[TOPK];
-    if constexpr (TOPK == 16) {
-#pragma unroll
-        for (int k = 0; k < TOPK; k++) {
-            inv[k] = 1.f;
-            if (atom_norms && ci[k] >= 0) {
-                const float n = atom_norms[bin * bin_natoms + ci[k]];
-                inv[k] = n > 0.f ? 1.f / n : 0.f;
-            }
+    const ListSlots at = list_slots(lists, slot);
+    // the TOPK best of the first list slot's two lists, then (a split item)
+    // joined with those of one more list at a time
+#pragma unroll 1
+    for (int l = NLISTS - 1; l < at.n * NLISTS; l++) {
+        const bool first = l == NLISTS - 1;  // both lists of the slot at once
+        const int q = first ? lane : lane - TOPK;
+        const bool listed = q >= 0 && q < (first ? NLISTS * TOPK : TOPK);
+        const long long ps = at.first + (long long)(l / NLISTS) * lists.vt;
+        const long long o = (ps * NLISTS + (first ? q / TOPK : l % NLISTS)) * TOPK_MAX + q % TOPK;
+        int li = listed ? lists.top_i[o] : -1;
+        float ls = listed && li >= 0 ? lists.top_s[o] : -1.f;
+        if (!first && lane < TOPK) {
+            li = scand[warp][lane];
+            ls = sscore[warp][lane];
         }
+        int rank = 0;
+#pragma unroll
+        for (int j = 0; j < NLISTS * TOPK; j++) {
+            const float sj = __shfl_sync(0xffffffffu, ls, j);
+            const int ij = __shfl_sync(0xffffffffu, li, j);
+            rank += sj > ls || (sj == ls && (ij < li || (ij == li && j < lane)));
+        }
+        __syncwarp();
+        if (lane < NLISTS * TOPK && rank < TOPK) {
+            scand[warp][rank] = li;
+            sscore[warp][rank] = ls;
+        }
+        __syncwarp();
     }
-    const bool scaled = TOPK != 16 && atom_norms && lane < TOPK && cand >= 0;
-    const float my_norm = scaled ? atom_norms[bin * bin_natoms + cand] : 1.f;
     const float2 *x = img + v * img_stride;
-    if (ROWS) {
-        // s = i d: conj(s) x = (d xi, -d xr)
-        const float *rowf[TOPK];
+    // one batch of NB candidates at a time
+    constexpr int NB = TOPK < 8 ? TOPK : 8, LPC = 32 / NB;  // lanes per candidate after the sums
+    int best = -1;
+    float bs = 0.f, bre = 0.f, bim = 0.f;
+#pragma unroll 1
+    for (int k0 = 0; k0 < TOPK; k0 += NB) {
+        float acc[2 * NB];  // Re, Im of each candidate
 #pragma unroll
-        for (int k = 0; k < TOPK; k++)
-            rowf[k] = reinterpret_cast<const float *>(atoms) + (bin * bin_natoms + (ci[k] >= 0 ? ci[k] : 0)) * atom_stride;
-        if (VEC) {
-            const long long n4 = nreps / 4;
-            for (long long t = lane; t < n4; t += 32) {
-                const float4 x0 = reinterpret_cast<const float4 *>(x)[2 * t];
-                const float4 x1 = reinterpret_cast<const float4 *>(x)[2 * t + 1];
+        for (int k = 0; k < 2 * NB; k++) acc[k] = 0.f;
+        // (a missing candidate reads atom 0's row; its sums are dropped)
+        const int ci = scand[warp][k0 + lane / LPC];
+        // Atoms as generated (atom_norms): 1 / ||d|| as the dictionary's
+        // normalisation forms it, its load ahead of the inner products
+        const float norm = atom_norms && ci >= 0 ? atom_norms[bin * bin_natoms + ci] : 1.f;
+        if (ROWS) {
+            // s = i d: conj(s) x = (d xi, -d xr)
+            const float *row[NB];
 #pragma unroll
-                for (int k = 0; k < TOPK; k++) {
-                    if (ci[k] < 0) continue;
-                    const float4 d = reinterpret_cast<const float4 *>(rowf[k])[t];
-                    re[k] += d.x * x0.y + d.y * x0.w;
-                    im[k] -= d.x * x0.x + d.y * x0.z;
-                    re[k] += d.z * x1.y + d.w * x1.w;
-                    im[k] -= d.z * x1.x + d.w * x1.z;
+            for (int k = 0; k < NB; k++)
+                row[k] = reinterpret_cast<const float *>(atoms) +
+                         (bin * bin_natoms + max(scand[warp][k0 + k], 0)) * atom_stride;
+            if (VEC) {
+                const int n4 = (int)(nreps / 4);
+                for (int t = lane; t < n4; t += 32) {
+                    const float4 x0 = reinterpret_cast<const float4 *>(x)[2 * t];
+                    const float4 x1 = reinterpret_cast<const float4 *>(x)[2 * t + 1];
+#pragma unroll
+                    for (int k = 0; k < NB; k++) {
+                        const float4 d = reinterpret_cast<const float4 *>(row[k])[t];
+                        float &re = acc[2 * k], &im = acc[2 * k + 1];
+                        re += d.x * x0.y + d.y * x0.w;
+                        im -= d.x * x0.x + d.y * x0.z;
+                        re += d.z * x1.y + d.w * x1.w;
+                        im -= d.z * x1.x + d.w * x1.z;
+                    }
+                }
+            } else {
+                for (long long t = lane; t < nreps; t += 32) {
+                    const float2 xv = x[t];
+#pragma unroll
+                    for (int k = 0; k < NB; k++) {
+                        const float d = row[k][t];
+                        acc[2 * k] += d * xv.y;
+                        acc[2 * k + 1] -= d * xv.x;
+                    }
                 }
             }
         } else {
-            for (long long t = lane; t < nreps; t += 32) {
-                const float2 xv = x[t];
+            const float2 *row[NB];
 #pragma unroll
-                for (int k = 0; k < TOPK; k++) {
-                    if (ci[k] < 0) continue;
-                    const float d = rowf[k][t];
-                    re[k] += d * xv.y;
-                    im[k] -= d * xv.x;
+            for (int k = 0; k < NB; k++)
+                row[k] = atoms + (bin * bin_natoms + max(scand[warp][k0 + k], 0)) * atom_stride;
+            if (VEC) {
+                const int n2 = (int)(nreps / 2);
+                for (int t = lane; t < n2; t += 32) {
+                    const float4 xv = reinterpret_cast<const float4 *>(x)[t];
+#pragma unroll
+                    for (int k = 0; k < NB; k++) {
+                        const float4 d = reinterpret_cast<const float4 *>(row[k])[t];
+                        float &re = acc[2 * k], &im = acc[2 * k + 1];
+                        re += d.x * xv.x + d.y * xv.y;
+                        im += d.x * xv.y - d.y * xv.x;
+                        re += d.z * xv.z + d.w * xv.w;
+                        im += d.z * xv.w - d.w * xv.z;
+                    }
+                }
+            } else {
+                for (long long t = lane; t < nreps; t += 32) {
+                    const float2 xv = x[t];
+#pragma unroll
+                    for (int k = 0; k < NB; k++) {
+                        const float2 d = row[k][t];
+                        float &re = acc[2 * k], &im = acc[2 * k + 1];
+                        re += d.x * xv.x + d.y * xv.y;
+                        im += d.x * xv.y - d.y * xv.x;
+                    }
                 }
             }
         }
-    } else if (VEC) {
-        const long long n2 = nreps / 2;
-        for (long long t = lane; t < n2; t += 32) {
-            const float4 xv = reinterpret_cast<const float4 *>(x)[t];
-#pragma unroll
-            for (int k = 0; k < TOPK; k++) {
-                if (ci[k] < 0) continue;
-                const float4 d = reinterpret_cast<const float4 *>(row[k])[t];
-                re[k] += d.x * xv.x + d.y * xv.y;
-                im[k] += d.x * xv.y - d.y * xv.x;
-                re[k] += d.z * xv.z + d.w * xv.w;
-                im[k] += d.z * xv.w - d.w * xv.z;
-            }
+        // candidate lane / LPC: Re on the first half of its lanes, Im on the rest
+        const float sum = warp_sums<2 * NB>(acc, lane);
+        const float other = __shfl_xor_sync(0xffffffffu, sum, LPC / 2);
+        const bool low = (lane & (LPC / 2)) == 0;
+        float re = low ? sum : other, im = low ? other : sum;
+        if (atom_norms && ci >= 0) {
+            const float inv = norm > 0.f ? 1.f / norm : 0.f;
+            re *= inv;
+            im *= inv;
         }
-    } else {
-        for (long long t = lane; t < nreps; t += 32) {
-            const float2 xv = x[t];
-#pragma unroll
-            for (int k = 0; k < TOPK; k++) {
-                if (ci[k] < 0) continue;
-                const float2 d = row[k][t];
-                re[k] += d.x * xv.x + d.y * xv.y;
-                im[k] += d.x * xv.y - d.y * xv.x;
-            }
+        const float sc = re * re + im * im;
+        if (ci >= 0 && sc > 0.f && (sc > bs || (sc == bs && best >= 0 && ci < best))) {
+            bs = sc;
+            best = ci;
+            bre = re;
+            bim = im;
         }
     }
+    // the best of the candidates (each lane: its own of every batch)
 #pragma unroll
-    for (int k = 0; k < TOPK; k++) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            re[k] += __shfl_xor_sync(0xffffffffu, re[k], o);
-            im[k] += __shfl_xor_sync(0xffffffffu, im[k], o);
+    for (int o = 16; o >= LPC; o >>= 1) {
+        const float os = __shfl_xor_sync(0xffffffffu, bs, o);
+        const int ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const float ore = __shfl_xor_sync(0xffffffffu, bre, o), oim = __shfl_xor_sync(0xffffffffu, bim, o);
+        if (ob >= 0 && (os > bs || (os == bs && (best < 0 || ob < best)))) {
+            bs = os;
+            best = ob;
+            bre = ore;
+            bim = oim;
         }
-    }
-    if constexpr (TOPK != 16) {
-        const float my_inv = scaled ? (my_norm > 0.f ? 1.f / my_norm : 0.f) : 1.f;
-#pragma unroll
-        for (int k = 0; k < TOPK; k++) inv[k] = __shfl_sync(0xffffffffu, my_inv, k);
     }
     if (lane != 0) return;
-    if (atom_norms) {
-#pragma unroll
-        for (int k = 0; k < TOPK; k++) {
-            re[k] *= inv[k];
-            im[k] *= inv[k];
-        }
-    }
-    int best = -1;
-    float bs = 0.f, bre = 0.f, bim = 0.f;
-#pragma unroll
-    for (int k = 0; k < TOPK; k++) {
-        if (ci[k] < 0) continue;
-        const float sc = re[k] * re[k] + im[k] * im[k];
-        if (sc > bs || (sc == bs && best >= 0 && ci[k] < best)) {
-            if (sc > 0.f) {
-                bs = sc;
-                best = ci[k];
-                bre = re[k];
-                bim = im[k];
-            }
-        }
-    }
     const long long g = bin * bin_natoms + (best >= 0 ? best : 0);
     const float *pr = params + g * nparams;
     float *m = maps + v * 5;
@@ -934,7 +1091,41 @@ int make_map(CUtensorMap *m, const void *base, long long rows, long long Kp, int
     return SNAPMRF_OK;
 }
 
-inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
+// (grid: one CTA per SM; the epilogue's list layout depends on it)
+int launch_scores(ScoreLaunch &l, int grid, cudaStream_t st) {
+    CUtensorMap mA, mB;
+    int rc = make_map(&mA, l.A, l.arows, l.Kp, BM, l.fmt);
+    if (rc) return rc;
+    rc = make_map(&mB, l.B, l.brows, l.Kp, BN, l.fmt);
+    if (rc) return rc;
+    const bool fp8 = l.fmt == 2, half = l.fmt == 1;
+    auto pick = [&](auto k16, auto k8, auto k4) { return l.topk > 8 ? k16 : l.topk > 4 ? k8 : k4; };
+    auto kern = l.split ? (l.imag ? match_bf16_kernel<16, false, true, true> : match_bf16_kernel<16, false, false, true>)
+                : fp8   ? pick(match_bf16_kernel<16, true, false>, match_bf16_kernel<8, true, false>,
+                               match_bf16_kernel<4, true, false>)
+                : l.imag ? pick(match_bf16_kernel<16, false, true>, match_bf16_kernel<8, false, true>,
+                                match_bf16_kernel<4, false, true>)
+                         : pick(match_bf16_kernel<16, false, false>, match_bf16_kernel<8, false, false>,
+                                match_bf16_kernel<4, false, false>);
+    SNAPMRF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+    l.a.nk = (int)(l.Kp / (fp8 ? BK8 : BK));
+    // Atom tiles in a golden-ratio stride order (coprime to their count):
+    // the dictionary's (T1, T2) order makes consecutive tiles' scores rise
+    // smoothly toward a voxel's best, so visiting tiles spread over the grid
+    // first raises the k-th best early and saves top-k insertions.
+    {
+        const int apt = l.imag ? BN : BA;
+        const long long natiles = ((long long)l.a.chunk_natoms + apt - 1) / apt;
+        long long st_ = std::max(1ll, (long long)std::llround(0.618034 * (double)natiles));
+        while (std::gcd(st_, natiles) != 1) st_++;
+        l.a.tile_stride = natiles > 1 ? (int)(st_ % natiles) : 1;
+        if (l.a.tile_stride == 0) l.a.tile_stride = 1;
+    }
+    l.a.idesc = fp8 ? sm100::make_idesc_e4m3(BM, BN) : half ? sm100::make_idesc_f16(BM, BN) : sm100::make_idesc_bf16(BM, BN);
+    kern<<<grid, THREADS, SMEM_BYTES, st>>>(mA, mB, l.a);
+    SNAPMRF_LAUNCH_CHECK();
+    return SNAPMRF_OK;
+}
 
 }  // namespace tc
 
@@ -956,7 +1147,12 @@ int match_bf16(const TcMatchRequest &q, cudaStream_t st) {
     // BF16 / FP16 compressed operands are split into hi + lo parts (K = 3L)
     const bool split = comp && !fp8;
     const long long Kp = (((imag ? 1 : 2) * kn * (split ? 3 : 1) + bke - 1) / bke) * bke;
-    const long long cap = ((nvox + BM - 1) / BM + nbins) * BM;  // padded slots, upper bound
+    const int vt = imag ? BM / 2 : BM;    // voxels per work item
+    const long long cap = ((nvox + vt - 1) / vt + nbins) * vt;  // padded slots, upper bound
+    int num_sms = 0, dev = 0;
+    SNAPMRF_CUDA(cudaGetDevice(&dev));
+    SNAPMRF_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
+    const long long lslots = cap + split_slots(cap / vt, num_sms) * vt;  // list slots
     const long long brows = (imag ? 1 : 2) * q.NATOMS;
     const long long arows = (imag ? 2 : 1) * cap;
     if (arows > 0x7fffffffll || brows > 0x7fffffffll || Kp > 0x7fffffffll)
@@ -971,10 +1167,10 @@ int match_bf16(const TcMatchRequest &q, cudaStream_t st) {
     const bool prepacked = imag && q.packed;
     const size_t oA = take((size_t)arows * Kp * eb), oB = take(prepacked ? 0 : (size_t)brows * Kp * eb);
     const size_t oSc = take(fp8 ? (size_t)q.NATOMS * 4 : 0);
-    const size_t oTs = take((size_t)cap * NLISTS * TOPK_MAX * 4), oTi = take((size_t)cap * NLISTS * TOPK_MAX * 4);
+    const size_t oTs = take((size_t)lslots * NLISTS * TOPK_MAX * 4), oTi = take((size_t)lslots * NLISTS * TOPK_MAX * 4);
     const size_t oPerm = take((size_t)cap * 8), oTile = take((size_t)(nbins + 1) * 8);
     const size_t oCur = take((size_t)(nbins + 1) * 8), oVb = take((size_t)nvox * 4);
-    const size_t oCnt = take((size_t)nbins * 4), oErr = take(4);
+    const size_t oCnt = take((size_t)nbins * 4), oErr = take(4), oPlan = take(sizeof(TailPlan));
     const size_t oCimg = take(comp ? (size_t)nvox * rs * sizeof(float2) : 0);
     DeviceScratch s;
     SNAPMRF_CUDA(s.alloc(bytes, st));
@@ -1005,12 +1201,12 @@ int match_bf16(const TcMatchRequest &q, cudaStream_t st) {
         assign_bins_kernel<<<nblk(nvox, 256), 256, 0, st>>>(vox_bin, counts, q.b1map, q.params, q.nparams,
                                                             q.natoms, nbins, nvox);
         SNAPMRF_LAUNCH_CHECK();
-        scan_padded_kernel<<<1, 32, 0, st>>>(counts, tile_start, cursor, nbins);
+        scan_padded_kernel<<<1, 32, 0, st>>>(counts, tile_start, cursor, nbins, vt);
         SNAPMRF_LAUNCH_CHECK();
         scatter_bins_kernel<<<nblk(nvox, 256), 256, 0, st>>>(perm, cursor, vox_bin, nvox);
         SNAPMRF_LAUNCH_CHECK();
     } else {
-        global_bin_kernel<<<nblk(cap, 256), 256, 0, st>>>(tile_start, perm, nvox, cap);
+        global_bin_kernel<<<nblk(cap, 256), 256, 0, st>>>(tile_start, perm, nvox, cap, vt);
         SNAPMRF_LAUNCH_CHECK();
     }
     if (comp) {
@@ -1083,48 +1279,40 @@ int match_bf16(const TcMatchRequest &q, cudaStream_t st) {
                                                                                  kn, Kp);
         SNAPMRF_LAUNCH_CHECK();
     }
-    CUtensorMap mA, mB;
-    int rc = make_map(&mA, A, arows, Kp, BM, fmt);
-    if (rc) return rc;
-    rc = make_map(&mB, B, brows, Kp, BN, fmt);
-    if (rc) return rc;
-
-    int num_sms = 0, dev = 0;
-    SNAPMRF_CUDA(cudaGetDevice(&dev));
-    SNAPMRF_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
-    auto pick = [&](auto k16, auto k8, auto k4) { return q.topk > 8 ? k16 : q.topk > 4 ? k8 : k4; };
-    auto kern = fp8    ? pick(match_bf16_kernel<16, true, false>, match_bf16_kernel<8, true, false>,
-                              match_bf16_kernel<4, true, false>)
-                : imag ? pick(match_bf16_kernel<16, false, true>, match_bf16_kernel<8, false, true>,
-                              match_bf16_kernel<4, false, true>)
-                       : pick(match_bf16_kernel<16, false, false>, match_bf16_kernel<8, false, false>,
-                              match_bf16_kernel<4, false, false>);
-    SNAPMRF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-    Args a;
+    ScoreLaunch sl;
+    sl.A = A;
+    sl.B = B;
+    sl.arows = arows;
+    sl.brows = brows;
+    sl.Kp = Kp;
+    sl.fmt = fmt;
+    sl.imag = imag;
+    sl.split = false;
+    sl.topk = q.topk;
+    Args &a = sl.a;
     a.tile_start = tile_start;
     a.nbins = nbins;
+    a.bin_lo = 0;
+    a.bin_hi = nbins;
     a.bin_natoms = bin_natoms;
-    a.nk = (int)(Kp / bke);
-    // Atom tiles in a golden-ratio stride order (coprime to their count):
-    // the dictionary's (T1, T2) order makes consecutive tiles' scores rise
-    // smoothly toward a voxel's best, so visiting tiles spread over the grid
-    // first raises the k-th best early and saves top-k insertions.
-    {
-        const long long natiles = (bin_natoms + (imag ? BN : BA) - 1) / (imag ? BN : BA);
-        long long st_ = std::max(1ll, (long long)std::llround(0.618034 * (double)natiles));
-        while (std::gcd(st_, natiles) != 1) st_++;
-        a.tile_stride = natiles > 1 ? (int)(st_ % natiles) : 1;
-        if (a.tile_stride == 0) a.tile_stride = 1;
-    }
-    a.idesc = fp8 ? sm100::make_idesc_e4m3(BM, BN) : half ? sm100::make_idesc_f16(BM, BN) : sm100::make_idesc_bf16(BM, BN);
+    a.atom0 = 0;
+    a.chunk_natoms = (int)bin_natoms;
+    a.max_parts = MAX_PARTS;
+    a.plan = reinterpret_cast<TailPlan *>(b + oPlan);
     a.ascale2 = fp8 ? ascale2 : nullptr;
+    a.cap = cap;
     a.top_s = top_s;
     a.top_i = top_i;
     a.err = err;
-    const long long max_items = (imag ? 2 : 1) * cap / BM;
-    const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>(num_sms, max_items));
-    kern<<<grid, THREADS, SMEM_BYTES, st>>>(mA, mB, a);
-    SNAPMRF_LAUNCH_CHECK();
+    int rc = launch_scores(sl, num_sms, st);
+    if (rc) return rc;
+    auto pick = [&](auto k16, auto k8, auto k4) { return q.topk > 8 ? k16 : q.topk > 4 ? k8 : k4; };
+    Lists lists;
+    lists.top_s = top_s;
+    lists.top_i = top_i;
+    lists.plan = a.plan;
+    lists.cap = cap;
+    lists.vt = vt;
     // two samples per 16-byte load when every row starts 16-byte aligned
     // rescoring operands: the atoms and samples, or (compressed, no atoms)
     // the coordinates and projected voxels
@@ -1141,7 +1329,7 @@ int match_bf16(const TcMatchRequest &q, cudaStream_t st) {
                                  rescore_kernel<4, false, true>))
                    : vec ? pick(rescore_kernel<16, true>, rescore_kernel<8, true>, rescore_kernel<4, true>)
                          : pick(rescore_kernel<16, false>, rescore_kernel<8, false>, rescore_kernel<4, false>);
-    rk<<<nblk(cap * 32, 256), 256, 0, st>>>(q.maps, q.index_out, top_s, top_i, perm, tile_start, nbins,
+    rk<<<nblk(cap * 32, kRescoreThreads), kRescoreThreads, 0, st>>>(q.maps, q.index_out, lists, perm, tile_start, nbins,
                                             q.b1map ? vox_bin : nullptr, ratoms, ras, rimg, ris, rn, q.params,
                                             q.nparams, bin_natoms, err, rfull ? q.atom_norms : nullptr);
     SNAPMRF_LAUNCH_CHECK();
