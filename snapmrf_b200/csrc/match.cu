@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "common.h"
+#include "match_fp32_tc.h"
 #include "match_kernels.cuh"
 #include "match_tc.h"
 #include "svd.h"
@@ -183,6 +184,11 @@ __global__ void poison_maps_kernel(float *maps, long long *index_out, long long 
 namespace tc {
 // Copies a call's error code into the library's device error word (match_tc.cu).
 __global__ void publish_error_kernel(const int *err);
+}
+
+// Whether the FP32 form's screen pays for its launches.
+static bool screen_pays(long long nvox, long long bin_natoms, long long nreps) {
+    return nvox * bin_natoms * nreps >= (1ll << 24);
 }
 
 static inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -557,15 +563,58 @@ extern "C" int snapmrf_mrf_match(float *d_maps, const float *img, int img_on_hos
         }
         return SNAPMRF_OK;
     };
+    // Screened on the tensor cores where that applies (see match_fp32_tc.cu):
+    // not for compressed scores, blocks with several B1 values, or calls too
+    // small to pay for its launches.
+    const bool screen = !comp && !general && screen_pays(nvox, (long long)(d_b1 ? natoms : NATOMS), (long long)nreps);
+    auto range = [&](long long v0, long long n) -> int {
+        float *maps = d_maps + 5 * v0;
+        int64_t *index = d_index ? d_index + v0 : nullptr;
+        const float2 *x = d_img + v0 * istride;
+        const float *b1 = d_b1 ? d_b1 + v0 : nullptr;
+        if (screen) {
+            ScreenRequest q;
+            q.maps = maps;
+            q.index_out = (long long *)index;
+            q.img = x;
+            q.img_stride = istride;
+            q.atoms = reinterpret_cast<const float2 *>(d_atoms);
+            q.atom_stride = (long long)atom_stride;
+            q.params = d_params;
+            q.nparams = nparams;
+            q.nreps = (long long)nreps;
+            q.NATOMS = (long long)NATOMS;
+            q.natoms = (long long)natoms;
+            q.nvox = n;
+            q.nblocks = (int)nblocks;
+            q.b1map = b1;
+            q.imag = (flags & SNAPMRF_MATCH_IMAG_ATOMS) != 0;
+            bool done = false;
+            int rc = match_fp32_screened(q, st, &done);
+            if (rc || done) return rc;
+        }
+        return fp32_range(v0, n, maps, index, x, b1);
+    };
     if (!img_on_host || up.nchunks <= 1 || comp || general) {
         if (img_on_host) SNAPMRF_CUDA(cudaStreamWaitEvent(st, up.done(), 0));
-        return fp32_range(0, nvox, d_maps, d_index, d_img, d_b1);
+        return range(0, nvox);
+    }
+    if (screen) {
+        // (each range packs the dictionary again: two, as the other
+        // tensor-core forms, all but the last two chunks first)
+        const long long vA = up.nchunks >= 4 ? up.first(up.nchunks - 2) : 0;
+        if (vA) {
+            SNAPMRF_CUDA(cudaStreamWaitEvent(st, up.ev[up.nchunks - 3], 0));
+            int rc = range(0, vA);
+            if (rc) return rc;
+        }
+        SNAPMRF_CUDA(cudaStreamWaitEvent(st, up.done(), 0));
+        return range(vA, nvox - vA);
     }
     for (int c = 0; c < up.nchunks; c++) {
         const long long v0 = up.first(c), n = up.first(c + 1) - v0;
         SNAPMRF_CUDA(cudaStreamWaitEvent(st, up.ev[c], 0));
-        int rc = fp32_range(v0, n, d_maps + 5 * v0, d_index ? d_index + v0 : nullptr, d_img + v0 * istride,
-                            d_b1 ? d_b1 + v0 : nullptr);
+        int rc = range(v0, n);
         if (rc) return rc;
     }
     return SNAPMRF_OK;

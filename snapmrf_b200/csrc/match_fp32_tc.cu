@@ -1,0 +1,596 @@
+// FP32 matching screened on the tensor cores.
+//
+// The FP32 form's answer is the first argmax of |s|^2 over the atoms of a
+// voxel's block, s being the FP32 sums of match_fp32_kernel in its own order.
+// Nearly all of its work goes into atoms that are far from the best.  Here
+// tcgen05 scores every pair from BF16 pairs (v = hi + lo, three products each,
+// FP32 accumulation), the epilogue lists every atom whose approximate |s| is
+// within twice the error bound of the best one, and
+//   - the listed atoms are scored again in FP32, in match_fp32_kernel's order
+//     (the same chain of FMAs, bit for bit), and their first argmax wins;
+//   - a voxel with more such atoms than a list holds, or whose input is not
+//     finite or out of range, goes to match_fp32_kernel itself.
+// So the approximate scores only decide what need not be looked at, and the
+// chosen atom is the one that the FP32 kernel alone chooses: maps and indices
+// are the same bit for bit (tests/test_match_screen_gpu.py).
+//
+// The bound, relative to ||d|| ||x|| (the voxels are scaled to unit norm, the
+// largest ||d|| of the dictionary stands for all), of the difference between
+// the two scores: the FP32 chain's n FMAs, 2^-24 each of a partial sum that
+// Cauchy and Schwarz keep below ||d|| ||x||; the BF16 pairs, 3 2^-18; the
+// tensor core's accumulation, 1.25 2^-23 (a truncated last bit and a quarter)
+// per MMA.  Measured, the scores differ by at most 1.6e-5 at T = 1000 (complex
+// atoms; 1.2e-5 imaginary, 4e-6 at T = 200 .. 300), where the bound is 2.1e-4
+// (1.0e-4, 3e-5).
+//
+// 57,600 voxels, 284,458 imaginary atoms in 41 blocks, T = 1000: 36.3 -> 4.9
+// ms (packing 0.68, scores 2.9 = three BF16 products at 1.68 PFLOP/s, about
+// eight candidates per voxel in FP32 0.88, maps 0.11; the FP32 kernel alone
+// runs at 0.61 of the FP32 FMA peak); 4,096 voxels, 837 complex atoms: 0.80 ->
+// 0.23 ms.
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+
+#include "common.h"
+#define SNAPMRF_MATCH_KERNEL_DECLARATION_ONLY
+#include "match_kernels.cuh"
+#undef SNAPMRF_MATCH_KERNEL_DECLARATION_ONLY
+#include "match_fp32_tc.h"
+#include "match_tc_plan.cuh"
+
+namespace snapmrf {
+
+// Kernels of the FP32 matching path (match.cu).
+__global__ void assign_bins_kernel(int *vox_bin, int *counts, const float *b1map, const float *params,
+                                   int nparams, long long natoms, int nblocks, long long nvox);
+__global__ void scatter_bins_kernel(long long *perm, long long *cursor, const int *vox_bin,
+                                    long long nvox);
+__global__ void finalize_maps_kernel(float *maps, long long *index_out, const unsigned long long *keys,
+                                     const long long *perm, const int *vox_bin, const float2 *atoms,
+                                     long long atom_stride, const float2 *img, long long img_stride,
+                                     long long nreps, const float *params, int nparams,
+                                     long long natoms_per_bin, long long nslots);
+__global__ void poison_maps_kernel(float *maps, long long *index_out, long long nvox, const int *err);
+
+namespace screen {
+
+constexpr int KB = 32;               // elements of K per 64-element row chunk (hi, then lo)
+constexpr float kMaxAbs = 1e15f;     // larger samples (or not finite) are left to the FP32 kernel
+constexpr float kMinNorm2 = 1e-30f;  // smaller norms too (of either side or their product): squares would lose bits
+constexpr float kMaxNorm2 = 1e30f;
+// Operand memory of one pass: larger dictionaries are screened in chunks of
+// atoms, larger images in ranges of voxels.
+constexpr size_t kAtomBytes = 2ull << 30, kVoxelBytes = 1ull << 30;
+
+struct State {
+    int err;                 // error word of the scoring kernel, or 7
+    int bad_atoms;           // an atom is not finite or out of range: the FP32 kernel takes every voxel
+    unsigned norm2_bits;     // largest squared atom norm
+    int nfall;               // voxels left to the FP32 kernel
+};
+
+__global__ void init_kernel(unsigned long long *keys, long long nkeys, long long *perm, long long nperm, int *counts,
+                            int *fall_counts, int nbins, State *st) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i < nkeys) keys[i] = 0ull;
+    if (i < nperm) perm[i] = -1;
+    if (i < nbins) counts[i] = fall_counts[i] = 0;
+    if (i == 0) *st = State{0, 0, 0u, 0};
+}
+
+// hi and lo of two neighbouring elements, packed.
+__device__ __forceinline__ void split2(float a, float b, uint32_t *hi, uint32_t *lo) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    const float2 f = __bfloat1622float2(h);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(a - f.x, b - f.y);
+    *hi = *reinterpret_cast<const uint32_t *>(&h);
+    *lo = *reinterpret_cast<const uint32_t *>(&l);
+}
+
+// Eight elements k0 .. k0 + 7 of a row (k0 a multiple of 8): 16 bytes of hi
+// and, 64 bytes further, 16 bytes of lo.
+__device__ __forceinline__ void store8(__nv_bfloat16 *row, long long k0, const float *v) {
+    uint4 h, l;
+    split2(v[0], v[1], &h.x, &l.x);
+    split2(v[2], v[3], &h.y, &l.y);
+    split2(v[4], v[5], &h.z, &l.z);
+    split2(v[6], v[7], &h.w, &l.w);
+    __nv_bfloat16 *p = row + (k0 / KB) * (2 * KB) + k0 % KB;
+    *reinterpret_cast<uint4 *>(p) = h;
+    *reinterpret_cast<uint4 *>(p + KB) = l;
+}
+
+// N samples from t of a row, zeros past nreps (VEC: 16-byte loads).
+template <int N, bool VEC>
+__device__ __forceinline__ void load_samples(const float2 *x, long long t, long long nreps, float2 *s) {
+    if (VEC && t + N <= nreps) {
+#pragma unroll
+        for (int u = 0; u < N / 2; u++) {
+            const float4 q = __ldg(reinterpret_cast<const float4 *>(x + t) + u);
+            s[2 * u] = make_float2(q.x, q.y);
+            s[2 * u + 1] = make_float2(q.z, q.w);
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < N; u++) s[u] = t + u < nreps ? __ldg(x + t + u) : make_float2(0.f, 0.f);
+    }
+}
+
+// A rows: the slot's voxel at unit norm, two rows (Re, Im) for purely
+// imaginary atoms, else one interleaved row.  vnorm2[slot]: its squared norm, 0
+// when every sample is 0 (no atom scores above 0), -1 when the FP32 kernel has
+// to take it.  One warp per slot.
+template <bool IMAG, bool VEC>
+__global__ void pack_voxels_kernel(__nv_bfloat16 *A, float *vnorm2, const float2 *img, long long img_stride,
+                                   const long long *perm, long long nslots, long long nreps, long long Kp) {
+    const long long slot = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / 32;
+    const int lane = threadIdx.x % 32;
+    if (slot >= nslots) return;
+    const long long v = perm[slot];
+    const float2 *x = img + (v >= 0 ? v : 0) * img_stride;
+    float n = 0.f, mx = 0.f;
+    if (v >= 0)
+        for (long long t = 4 * lane; t < nreps; t += 128) {
+            float2 s[4];
+            load_samples<4, VEC>(x, t, nreps, s);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                n += s[u].x * s[u].x + s[u].y * s[u].y;
+                mx = fmaxf(mx, fmaxf(fabsf(s[u].x), fabsf(s[u].y)));
+            }
+        }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        n += __shfl_xor_sync(0xffffffffu, n, o);
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    const bool fit = n >= kMinNorm2 && mx <= kMaxAbs && n <= kMaxNorm2;  // (false for NaN)
+    const float inv = fit ? rsqrtf(n) : 0.f;
+    if (lane == 0) vnorm2[slot] = fit ? n : (n == 0.f && mx == 0.f) ? 0.f : -1.f;
+    const long long K = IMAG ? Kp / 2 : Kp / 4;  // samples, padded
+    __nv_bfloat16 *row = A + (IMAG ? 2 * slot : slot) * Kp;
+    for (long long t = (IMAG ? 8 : 4) * lane; t < K; t += (IMAG ? 256 : 128)) {
+        float2 s[IMAG ? 8 : 4];
+        if (inv > 0.f) {
+            load_samples<IMAG ? 8 : 4, VEC>(x, t, nreps, s);
+        } else {
+#pragma unroll
+            for (int u = 0; u < (IMAG ? 8 : 4); u++) s[u] = make_float2(0.f, 0.f);
+        }
+        float a[8], b[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            if (IMAG) {
+                a[u] = s[u].x * inv;
+                b[u] = s[u].y * inv;
+            } else {
+                a[u] = (u & 1 ? s[u / 2].y : s[u / 2].x) * inv;
+            }
+        }
+        store8(row, IMAG ? t : 2 * t, a);
+        if (IMAG) store8(row + Kp, t, b);
+    }
+}
+
+// B rows of atoms [a0, a0 + n) (row r of the operand: atom a0 + r): one row
+// (Im d) for purely imaginary atoms (a real part sets the error word to 7),
+// else two, (Re d, Im d) and (-Im d, Re d); the largest squared norm and
+// whether every sample is finite and in range.  One warp per atom.  Bound by
+// its traffic: C1's 284,458 atoms (2.28 GB read, 1.17 GB written) 0.6 ms.
+template <bool IMAG, bool VEC>
+__global__ void pack_atoms_kernel(__nv_bfloat16 *B, const float2 *atoms, long long atom_stride, long long n,
+                                  long long nreps, long long Kp, State *st) {
+    const long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / 32;
+    const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+    __shared__ float smax[8];
+    float n2 = 0.f, mx = 0.f;
+    bool real_part = false, bad = false;
+    if (r < n) {
+        const float2 *src = atoms + r * atom_stride;
+        __nv_bfloat16 *row = B + (IMAG ? r : 2 * r) * Kp;
+        const long long K = IMAG ? Kp / 2 : Kp / 4;
+        for (long long t = (IMAG ? 8 : 4) * lane; t < K; t += (IMAG ? 256 : 128)) {
+            float2 s[IMAG ? 8 : 4];
+            load_samples<IMAG ? 8 : 4, VEC>(src, t, nreps, s);
+            float a[8], b[8];
+#pragma unroll
+            for (int u = 0; u < (IMAG ? 8 : 4); u++) {
+                n2 += s[u].x * s[u].x + s[u].y * s[u].y;
+                bad |= !(fabsf(s[u].x) <= kMaxAbs && fabsf(s[u].y) <= kMaxAbs);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                if (IMAG) {
+                    real_part |= s[u].x != 0.f;
+                    a[u] = s[u].y;
+                } else {
+                    a[u] = u & 1 ? s[u / 2].y : s[u / 2].x;
+                    b[u] = u & 1 ? s[u / 2].x : -s[u / 2].y;
+                }
+            }
+            store8(row, IMAG ? t : 2 * t, a);
+            if (!IMAG) store8(row + Kp, 2 * t, b);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+    bad |= !(n2 <= kMaxNorm2);
+    if (IMAG && __any_sync(0xffffffffu, real_part) && lane == 0) atomicCAS(&st->err, 0, 7);
+    if (__any_sync(0xffffffffu, bad)) {
+        n2 = 0.f;
+        if (lane == 0) atomicExch(&st->bad_atoms, 1);
+    }
+    if (lane == 0) smax[warp] = n2;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 0; w < (int)blockDim.x / 32; w++) mx = fmaxf(mx, smax[w]);
+        // (one atomic per CTA, and only while it raises the value)
+        const unsigned bits = __float_as_uint(mx);
+        if (bits > *reinterpret_cast<volatile unsigned *>(&st->norm2_bits)) atomicMax(&st->norm2_bits, bits);
+    }
+}
+
+// The voxels' winners: FP32 scores of every listed atom within the bound, in
+// match_fp32_kernel's order, or the voxel goes to the fall list.  One warp per
+// slot; lane c carries candidate c's chain (kBatch of them at a time) through
+// samples that cp.async stages kDepth steps of kSteps ahead.  The chain is
+// serial by definition: 57,600 voxels of about eight candidates 0.88 ms, their
+// rows 3.7 GB from L2 (waiting for each candidate's load in turn: 2.4 ms).
+constexpr int kRescoreWarps = 4, kMaxCand = 96, kBatch = 16, kSteps = 16, kDepth = 3;
+struct RescoreSmem {
+    float2 d[kDepth][kBatch][kSteps + 1];  // (rows padded: the lanes' reads differ in bank)
+    float2 x[kDepth][kSteps];
+    int cand[kMaxCand];
+};
+
+__device__ __forceinline__ void copy8(float2 *dst, const float2 *src, bool in) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(in ? 8 : 0)
+                 : "memory");
+}
+
+template <bool IMAG>
+__global__ void __launch_bounds__(kRescoreWarps * 32)
+rescore_kernel(unsigned long long *keys, tc::Lists lists, const int *list_n, const float *list_best,
+               const long long *perm, const float *vnorm2, const long long *tile_start, int nbins,
+               const int *vox_bin, const float2 *atoms, long long atom_stride, const float2 *img,
+               long long img_stride, int nreps, long long bin_natoms, float margin_rel, State *st, int *fall,
+               int *fall_counts) {
+    __shared__ RescoreSmem smem[kRescoreWarps];
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    RescoreSmem &sm = smem[warp];
+    const long long slot = blockIdx.x * (long long)kRescoreWarps + warp;
+    if (slot >= tile_start[nbins] * lists.vt) return;
+    const long long v = perm[slot];
+    const float xn2 = vnorm2[slot];
+    if (v < 0 || xn2 == 0.f) return;
+    const int bin = vox_bin ? vox_bin[v] : 0;
+    auto leave = [&]() {
+        if (lane == 0) {
+            fall[atomicAdd(&st->nfall, 1)] = (int)v;
+            atomicAdd(&fall_counts[bin], 1);
+        }
+    };
+    const float norm2 = __uint_as_float(st->norm2_bits);
+    if (xn2 < 0.f || st->bad_atoms || norm2 < kMinNorm2 || norm2 * xn2 < kMinNorm2 || norm2 * xn2 > kMaxNorm2)
+        return leave();
+    // the slot's lists: counts and best scores, one list per lane
+    constexpr int LISTS = tc::split_lists(IMAG), CAPL = tc::LIST_CAP / LISTS;
+    const tc::ListSlots at = tc::list_slots(lists, slot);
+    const int nl = at.n * LISTS;
+    static_assert(tc::MAX_PARTS * 4 <= 32, "a lane per list");
+    long long lid = 0;
+    int n = 0;
+    float best = 0.f;
+    if (lane < nl) {
+        lid = (at.first + (long long)(lane / LISTS) * lists.vt) * LISTS + lane % LISTS;
+        n = list_n[lid];
+        best = list_best[lid];
+    }
+    const bool over = n > CAPL;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
+    const float low = sqrtf(best) - margin_rel * sqrtf(norm2);
+    if (__any_sync(0xffffffffu, over) || !(low > 0.f)) return leave();
+    const float thr = low * low * (1.f - 0x1p-20f);
+    int count = 0;
+    for (int l = 0; l < nl; l++) {
+        const long long base = __shfl_sync(0xffffffffu, lid, l) * CAPL;
+        const int nn = __shfl_sync(0xffffffffu, n, l);
+        for (int e0 = 0; e0 < nn; e0 += 32) {
+            const bool in = e0 + lane < nn && lists.top_s[base + e0 + lane] >= thr;
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            const int pos = count + __popc(m & ((1u << lane) - 1));
+            if (in && pos < kMaxCand) sm.cand[pos] = lists.top_i[base + e0 + lane];
+            count += __popc(m);
+        }
+    }
+    if (count > kMaxCand) return leave();
+    __syncwarp();
+    if (count == 1) {
+        // no other atom can win (|s| > 0: it is above the bound)
+        if (lane == 0) keys[v] = pack_key(best, (unsigned)sm.cand[0]);
+        return;
+    }
+    const float2 *x = img + v * img_stride;
+    const float2 *d0 = atoms + (long long)bin * bin_natoms * atom_stride;
+    const int steps = (nreps + kSteps - 1) / kSteps, sub = lane % kSteps, which = lane / kSteps;
+    float bs = 0.f;
+    int bi = -1;
+    for (int c0 = 0; c0 < count; c0 += kBatch) {
+        const int nb = min(kBatch, count - c0);
+        // (two candidates' samples per copy instruction)
+        const float2 *row[kBatch / 2];
+#pragma unroll
+        for (int q = 0; q < kBatch / 2; q++)
+            row[q] = d0 + (long long)sm.cand[min(c0 + 2 * q + which, count - 1)] * atom_stride + sub;
+        auto stage = [&](int s) {
+            if (s < steps) {
+                const int t0 = s * kSteps, b = s % kDepth;
+                const bool in = t0 + sub < nreps;
+                if (which == 0) copy8(&sm.x[b][sub], in ? x + t0 + sub : x, in);
+#pragma unroll
+                for (int q = 0; q < kBatch / 2; q++)
+                    if (2 * q < nb) copy8(&sm.d[b][2 * q + which][sub], in ? row[q] + t0 : row[q] - sub, in);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        for (int s = 0; s < kDepth - 1; s++) stage(s);
+        float ar = 0.f, ai = 0.f;
+        for (int s = 0; s < steps; s++) {
+            stage(s + kDepth - 1);
+            asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");
+            __syncwarp();
+            const float2 *dr = sm.d[s % kDepth][lane % kBatch], *xr = sm.x[s % kDepth];
+            // (samples past nreps are zeros: their products add exact zeros)
+#pragma unroll
+            for (int u = 0; u < kSteps; u++) {
+                const float2 d = dr[u], xv = xr[u];
+                if (IMAG) {
+                    ar = fmaf(d.y, xv.y, ar);
+                    ai = fmaf(-d.y, xv.x, ai);
+                } else {
+                    ar = fmaf(d.x, xv.x, ar);
+                    ar = fmaf(d.y, xv.y, ar);
+                    ai = fmaf(d.x, xv.y, ai);
+                    ai = fmaf(-d.y, xv.x, ai);
+                }
+            }
+            __syncwarp();
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        const float sc = ar * ar + ai * ai;
+        if (lane < nb && sc > 0.f && beats(sc, sm.cand[c0 + lane], bs, bi)) {
+            bs = sc;
+            bi = sm.cand[c0 + lane];
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float os = __shfl_xor_sync(0xffffffffu, bs, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (beats(os, oi, bs, bi)) {
+            bs = os;
+            bi = oi;
+        }
+    }
+    if (lane == 0 && bi >= 0) keys[v] = pack_key(bs, (unsigned)bi);
+}
+
+// Slots and tiles of the voxels left to the FP32 kernel, by bin.  One CTA:
+// usually there are none.
+__global__ void __launch_bounds__(1024) fall_bins_kernel(const State *st, const int *fall, const int *fall_counts,
+                                                         const int *vox_bin, long long *slot_start,
+                                                         long long *tile_start, long long *cursor, long long *perm,
+                                                         int nbins) {
+    const int n = st->nfall;
+    if (threadIdx.x == 0) {
+        long long s = 0, t = 0;
+        if (n)
+            for (int b = 0; b < nbins; b++) {
+                slot_start[b] = cursor[b] = s;
+                tile_start[b] = t;
+                s += fall_counts[b];
+                t += (fall_counts[b] + kMatchVT - 1) / kMatchVT;
+            }
+        slot_start[nbins] = s;
+        tile_start[nbins] = t;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const int v = fall[i], b = vox_bin ? vox_bin[v] : 0;
+        perm[atomicAdd(reinterpret_cast<unsigned long long *>(&cursor[b]), 1ull)] = v;
+    }
+}
+
+inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
+
+}  // namespace screen
+
+int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
+    using namespace screen;
+    *done = false;
+    const int nbins = q.b1map ? q.nblocks : 1;
+    const long long bin_natoms = q.b1map ? q.natoms : q.NATOMS;
+    const int vt = q.imag ? tc::BM / 2 : tc::BM, apt = q.imag ? tc::BN : tc::BA, rows = q.imag ? 1 : 2;
+    const long long K = (q.imag ? 1 : 2) * q.nreps, nk = (K + KB - 1) / KB, Kp = nk * 2 * KB;
+    if (Kp > 0x7fffffffll / 4) return SNAPMRF_OK;
+    // atoms per pass: whole bins, or a chunk of one bin's tiles
+    const long long row_bytes = rows * Kp * 2, fit = std::max<long long>(apt, (long long)kAtomBytes / row_bytes);
+    const int bins_per = (int)std::min<long long>(nbins, std::max(1ll, fit / bin_natoms));
+    const long long chunk = bin_natoms <= fit ? bin_natoms : fit / apt * apt;
+    // voxels per pass
+    const long long nv_fit = std::max<long long>(vt, (long long)kVoxelBytes / ((q.imag ? 2 : 1) * Kp * 2));
+    const long long nv_max = std::min(q.nvox, nv_fit);
+    const long long cap = ((nv_max + vt - 1) / vt + nbins) * vt;
+    const long long arows = (q.imag ? 2 : 1) * cap, brows = rows * chunk * bins_per;
+    if (arows > 0x7fffffffll || brows > 0x7fffffffll) return SNAPMRF_OK;
+    int num_sms = 0, dev = 0;
+    SNAPMRF_CUDA(cudaGetDevice(&dev));
+    SNAPMRF_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
+    // (items are split only when one launch covers the whole dictionary)
+    const bool one = bins_per == nbins && chunk == bin_natoms;
+    const long long lslots = cap + (one ? tc::split_slots(cap / vt, num_sms) * vt : 0);
+
+    size_t bytes = 0;
+    auto take = [&](size_t n) {
+        size_t off = bytes;
+        bytes += (n + 255) & ~size_t(255);
+        return off;
+    };
+    const size_t oA = take((size_t)arows * Kp * 2), oB = take((size_t)brows * Kp * 2);
+    const size_t lb = (size_t)lslots * tc::LIST_CAP * 4, hb = (size_t)lslots * tc::split_lists(q.imag) * 4;
+    const size_t oTs = take(lb), oTi = take(lb), oLn = take(hb), oLb = take(hb), oPlan = take(sizeof(tc::TailPlan));
+    const size_t oKey = take((size_t)nv_max * 8);
+    const size_t oPerm = take((size_t)cap * 8), oFperm = take((size_t)nv_max * 8), oFall = take((size_t)nv_max * 4);
+    const size_t oVb = take((size_t)nv_max * 4), oKind = take((size_t)cap * 4);
+    const size_t oBin = take(5 * (size_t)(nbins + 1) * 8), oCnt = take(2 * (size_t)nbins * 4), oSt = take(sizeof(State));
+    DeviceScratch s;
+    const cudaError_t ae = s.alloc(bytes, st);
+    if (ae == cudaErrorMemoryAllocation) {
+        // without room for the operands the FP32 kernel takes the whole call
+        cudaGetLastError();
+        return SNAPMRF_OK;
+    }
+    SNAPMRF_CUDA(ae);
+    unsigned char *b = s.as<unsigned char>();
+    __nv_bfloat16 *A = reinterpret_cast<__nv_bfloat16 *>(b + oA), *B = reinterpret_cast<__nv_bfloat16 *>(b + oB);
+    unsigned long long *keys = reinterpret_cast<unsigned long long *>(b + oKey);
+    long long *perm = reinterpret_cast<long long *>(b + oPerm), *fperm = reinterpret_cast<long long *>(b + oFperm);
+    int *fall = reinterpret_cast<int *>(b + oFall), *vox_bin = reinterpret_cast<int *>(b + oVb);
+    float *vnorm2 = reinterpret_cast<float *>(b + oKind);
+    long long *tile_start = reinterpret_cast<long long *>(b + oBin), *cursor = tile_start + nbins + 1;
+    long long *fslot = cursor + nbins + 1, *ftile = fslot + nbins + 1, *fcursor = ftile + nbins + 1;
+    int *counts = reinterpret_cast<int *>(b + oCnt), *fall_counts = counts + nbins;
+    State *state = reinterpret_cast<State *>(b + oSt);
+    *done = true;
+
+    const float eps = 0x1p-24f, n = (float)K;
+    const float delta = n * eps + 3.f * 0x1p-18f + 1.25f * 6.f * (float)nk * 0x1p-23f + 0x1p-20f;
+    const float margin_rel = 2.f * delta * (1.f + 0x1p-16f);
+    auto aligned = [](const void *p, long long stride) {
+        return stride % 2 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0;
+    };
+    const bool avec = aligned(q.atoms, q.atom_stride);
+
+    for (long long v0 = 0; v0 < q.nvox; v0 += nv_max) {
+        const long long nv = std::min(nv_max, q.nvox - v0);
+        const float2 *img = q.img + v0 * q.img_stride;
+        const float *b1 = q.b1map ? q.b1map + v0 : nullptr;
+        const long long ninit = std::max<long long>(std::max(nv, q.b1map ? cap : 0), nbins);
+        init_kernel<<<nblk(ninit, 256), 256, 0, st>>>(keys, nv, perm, q.b1map ? cap : 0, counts, fall_counts, nbins,
+                                                      state);
+        SNAPMRF_LAUNCH_CHECK();
+        if (b1) {
+            assign_bins_kernel<<<nblk(nv, 256), 256, 0, st>>>(vox_bin, counts, b1, q.params, q.nparams, q.natoms,
+                                                              nbins, nv);
+            SNAPMRF_LAUNCH_CHECK();
+            tc::scan_padded_kernel<<<1, 32, 0, st>>>(counts, tile_start, cursor, nbins, vt);
+            SNAPMRF_LAUNCH_CHECK();
+            scatter_bins_kernel<<<nblk(nv, 256), 256, 0, st>>>(perm, cursor, vox_bin, nv);
+        } else {
+            tc::global_bin_kernel<<<nblk(cap, 256), 256, 0, st>>>(tile_start, perm, nv, cap, vt);
+        }
+        SNAPMRF_LAUNCH_CHECK();
+        const bool ivec = aligned(img, q.img_stride);
+        auto pv = q.imag ? (ivec ? pack_voxels_kernel<true, true> : pack_voxels_kernel<true, false>)
+                         : (ivec ? pack_voxels_kernel<false, true> : pack_voxels_kernel<false, false>);
+        pv<<<nblk(cap * 32, 256), 256, 0, st>>>(A, vnorm2, img, q.img_stride, perm, cap, q.nreps, Kp);
+        SNAPMRF_LAUNCH_CHECK();
+
+        tc::ScoreLaunch sl;
+        sl.A = A;
+        sl.B = B;
+        sl.arows = arows;
+        sl.Kp = Kp;
+        sl.fmt = 0;
+        sl.imag = q.imag;
+        sl.split = true;
+        sl.topk = 16;
+        tc::Args &a = sl.a;
+        a.tile_start = tile_start;
+        a.nbins = nbins;
+        a.bin_natoms = bin_natoms;
+        a.max_parts = one ? tc::MAX_PARTS : 1;
+        a.ascale2 = nullptr;
+        a.cap = cap;
+        a.top_s = reinterpret_cast<float *>(b + oTs);
+        a.top_i = reinterpret_cast<int *>(b + oTi);
+        a.plan = reinterpret_cast<tc::TailPlan *>(b + oPlan);
+        a.margin_rel = margin_rel;
+        a.norm2_bits = &state->norm2_bits;
+        a.list_n = reinterpret_cast<int *>(b + oLn);
+        a.list_best = reinterpret_cast<float *>(b + oLb);
+        a.err = &state->err;
+        auto pa = q.imag ? (avec ? pack_atoms_kernel<true, true> : pack_atoms_kernel<true, false>)
+                         : (avec ? pack_atoms_kernel<false, true> : pack_atoms_kernel<false, false>);
+        for (int b0 = 0; b0 < nbins; b0 += bins_per) {
+            const int nb = std::min(bins_per, nbins - b0);
+            for (long long a0 = 0; a0 < bin_natoms; a0 += chunk) {
+                // (several bins only with chunk == bin_natoms)
+                const long long ca = std::min(chunk, bin_natoms - a0);
+                const long long na = nb * ca;
+                pa<<<nblk(na * 32, 256), 256, 0, st>>>(B, q.atoms + (b0 * bin_natoms + a0) * q.atom_stride,
+                                                       q.atom_stride, na, q.nreps, Kp, state);
+                SNAPMRF_LAUNCH_CHECK();
+                sl.brows = rows * na;
+                a.bin_lo = b0;
+                a.bin_hi = b0 + nb;
+                a.atom0 = (int)a0;
+                a.chunk_natoms = (int)ca;
+                a.resume = a0 > 0;
+                int rc = tc::launch_scores(sl, num_sms, st);
+                if (rc) return rc;
+            }
+        }
+        tc::Lists lists;
+        lists.top_s = a.top_s;
+        lists.top_i = a.top_i;
+        lists.plan = a.plan;
+        lists.cap = cap;
+        lists.vt = vt;
+        auto rk = q.imag ? rescore_kernel<true> : rescore_kernel<false>;
+        rk<<<nblk(cap, kRescoreWarps), kRescoreWarps * 32, 0, st>>>(
+            keys, lists, a.list_n, a.list_best, perm, vnorm2, tile_start, nbins, b1 ? vox_bin : nullptr, q.atoms,
+            q.atom_stride, img, q.img_stride, (int)q.nreps, bin_natoms, margin_rel, state, fall, fall_counts);
+        SNAPMRF_LAUNCH_CHECK();
+        fall_bins_kernel<<<1, 1024, 0, st>>>(state, fall, fall_counts, b1 ? vox_bin : nullptr, fslot, ftile, fcursor,
+                                             fperm, nbins);
+        SNAPMRF_LAUNCH_CHECK();
+        MatchArgs m;
+        m.atoms = q.atoms;
+        m.atom_stride = q.atom_stride;
+        m.img = img;
+        m.img_stride = q.img_stride;
+        m.nreps = q.nreps;
+        m.nbins = nbins;
+        m.bin_natoms = bin_natoms;
+        m.nvox = nv;
+        m.keys = keys;
+        m.key_by_voxel = 1;
+        m.err = nullptr;  // (a real part was looked for while packing)
+        m.slot_start = fslot;
+        m.tile_start = ftile;
+        m.perm = fperm;
+        m.perm_mod = 0;
+        m.atiles_per_split = 0;
+        SNAPMRF_CUDA(launch_match_fp32(m, dim3(2 * num_sms), q.imag, st));
+        float *maps = q.maps + v0 * 5;
+        long long *index = q.index_out ? q.index_out + v0 : nullptr;
+        finalize_maps_kernel<<<nblk(nv * 32, 256), 256, 0, st>>>(
+            maps, index, keys, nullptr, b1 ? vox_bin : nullptr, q.atoms, q.atom_stride, img, q.img_stride, q.nreps,
+            q.params, q.nparams, bin_natoms, nv);
+        SNAPMRF_LAUNCH_CHECK();
+        // a timed-out wait or an atom with a real part: NaN maps, indices -1
+        poison_maps_kernel<<<nblk(nv, 256), 256, 0, st>>>(maps, index, nv, &state->err);
+        SNAPMRF_LAUNCH_CHECK();
+        tc::publish_error_kernel<<<1, 1, 0, st>>>(&state->err);
+        SNAPMRF_LAUNCH_CHECK();
+    }
+    return SNAPMRF_OK;
+}
+
+}  // namespace snapmrf

@@ -28,7 +28,8 @@ struct MatchArgs {
     long long perm_mod;
     long long nvox;
     unsigned long long *keys;    // [slots] packed (|s|^2 bits << 32 | ~atom)
-    int atiles_per_split;
+    int key_by_voxel;            // 1: keys are indexed by voxel instead of slot
+    int atiles_per_split;        // 0: chosen on the device for the launch's grid
     int *err;                    // imaginary form: set to 7 when an atom has a real part
 };
 
@@ -64,8 +65,10 @@ struct MatchSmem {
 template <bool IMAG, bool VEC>
 __global__ void __launch_bounds__(kMatchThreads, 2) match_fp32_kernel(MatchArgs m);
 #else
-// One CTA: a tile of kMatchVT voxel slots of one bin against
-// atiles_per_split tiles of kMatchAT atoms of that bin.  Warp w covers atoms
+// One work item: a tile of kMatchVT voxel slots of one bin against
+// atiles_per_split tiles of kMatchAT atoms of that bin; a CTA takes the items
+// blockIdx.x, blockIdx.x + gridDim.x, ..  (the number of tiles is only known
+// on the device).  Warp w covers atoms
 // 32 (w / 2) .. + 31 and voxels 32 (w % 2) .. + 31; lane (ag, vg) = (lane / 8,
 // lane % 8) accumulates atoms 8 ag .. 8 ag + 7 of its warp's rows against
 // voxels vg + 8 j (j < 4).  Scores s = sum_t conj(d_t) x_t:
@@ -93,8 +96,14 @@ __global__ void __launch_bounds__(kMatchThreads, 2) match_fp32_kernel(MatchArgs 
     static_assert(kVoxPasses >= 1 && kMatchVT % kRowsPerPass == 0, "stage geometry");
     const int q = tid % kLanesPerRow, lrow = tid / kLanesPerRow;
     bool real_part = false;
+    const long long atiles = (m.bin_natoms + kMatchAT - 1) / kMatchAT;
+    // atom tiles per item: as launched, or about eight items per CTA
+    int aps = m.atiles_per_split;
+    if (aps == 0) aps = (int)max(1ll, min(atiles, total_tiles * atiles / (8ll * gridDim.x)));
+    const long long splits = (atiles + aps - 1) / aps;
 
-    for (long long tile = blockIdx.y; tile < total_tiles; tile += gridDim.y) {
+    for (long long it = blockIdx.x; it < total_tiles * splits; it += gridDim.x) {
+        const long long tile = it / splits, split = it - tile * splits;
         // bin of this tile (binary search over the tile prefix)
         int lo = 0, hi = m.nbins - 1;
         while (lo < hi) {
@@ -106,8 +115,8 @@ __global__ void __launch_bounds__(kMatchThreads, 2) match_fp32_kernel(MatchArgs 
         const long long s_end = m.slot_start[bin + 1];
         const long long a_bin0 = (long long)bin * m.bin_natoms;
         // atom positions within the bin fit an int (fewer than 2^31 atoms per bin)
-        const int at_begin = (int)min((long long)blockIdx.x * m.atiles_per_split * kMatchAT, m.bin_natoms);
-        const int at_end = (int)min(m.bin_natoms, (long long)at_begin + (long long)m.atiles_per_split * kMatchAT);
+        const int at_begin = (int)min(split * aps * kMatchAT, m.bin_natoms);
+        const int at_end = (int)min(m.bin_natoms, (long long)at_begin + (long long)aps * kMatchAT);
         __syncthreads();
         if (tid < kMatchVT) {
             long long s = s0 + tid;
@@ -275,7 +284,8 @@ __global__ void __launch_bounds__(kMatchThreads, 2) match_fp32_kernel(MatchArgs 
                 }
             }
             const int vcol = vcol0 + 8 * j;
-            if (ag == 0 && bi >= 0 && sm.vox[vcol] >= 0) atomicMax(&m.keys[s0 + vcol], pack_key(bs, (unsigned)bi));
+            if (ag == 0 && bi >= 0 && sm.vox[vcol] >= 0)
+                atomicMax(&m.keys[m.key_by_voxel ? sm.vox[vcol] : s0 + vcol], pack_key(bs, (unsigned)bi));
         }
     }
     if (IMAG && m.err && __any_sync(0xffffffffu, real_part) && lane == 0) atomicCAS(m.err, 0, 7);
@@ -286,9 +296,9 @@ inline size_t match_fp32_smem(bool imag) {
     return imag ? sizeof(MatchSmem<true>) : sizeof(MatchSmem<false>);
 }
 
-// Grid of the FP32 kernel: y walks the voxel tiles (bin-major, so CTAs that
-// run together share a bin's atoms in L2), x splits each bin's atom tiles so
-// that about 16 waves of two resident CTAs per SM keep the last wave's idle
+// Grid of the FP32 kernel: one CTA per item, the splits of a voxel tile
+// first (bin-major, so CTAs that run together share a bin's atoms in L2); each
+// bin's atom tiles are split so that about 16 waves of two resident CTAs per SM keep the last wave's idle
 // share small.  Sets m.atiles_per_split.  tiles_est: voxel tiles the grid
 // covers; max_tiles: an upper bound of the tile count.
 inline dim3 fp32_match_grid(MatchArgs &m, long long tiles_est, long long max_tiles) {
@@ -303,7 +313,8 @@ inline dim3 fp32_match_grid(MatchArgs &m, long long tiles_est, long long max_til
     long long splits = std::max(1ll, std::min(atiles, (target + tiles_est - 1) / std::max(1ll, tiles_est)));
     m.atiles_per_split = (int)((atiles + splits - 1) / splits);
     splits = (atiles + m.atiles_per_split - 1) / m.atiles_per_split;
-    return dim3((unsigned)splits, (unsigned)std::min(max_tiles, 65535ll));
+    m.key_by_voxel = 0;
+    return dim3((unsigned)std::min(splits * max_tiles, 0x7fffffffll));
 }
 
 // Launches the imaginary-atom or complex form; 16-byte loads when every atom

@@ -1,0 +1,117 @@
+"""The FP32 form screened on the tensor cores chooses the atoms that the FP32
+kernel alone chooses.  snapmrf_mrf_match_noalloc always runs that kernel over
+every atom, so maps and indices of the two are compared bit for bit: at the
+edges of the screen's tiles (64 / 128 voxels, 256 / 128 atoms, 32 elements of
+K), with purely imaginary and complex atoms, odd strides, a B1 map with empty
+and one-voxel blocks, atoms of very different norms, exact duplicates, and
+voxels and atoms that the screen must leave to the FP32 kernel (zero, tiny,
+huge, infinite, NaN; a grid so fine that more atoms than a list holds lie
+within the screen's bound)."""
+import numpy as np
+import pytest
+
+from gpu_util import torch_cuda
+
+pytestmark = pytest.mark.gpu
+
+
+def _both(snap, img, atoms, params, nreps, natoms, b1map=None, imag=False):
+    torch = torch_cuda()
+    N, stride = atoms.shape
+    nvox = img.shape[0]
+    d_atoms = torch.from_numpy(np.ascontiguousarray(atoms).view(np.float32)).cuda()
+    d_img = torch.from_numpy(np.ascontiguousarray(img).view(np.float32)).cuda()
+    d_p = torch.from_numpy(params).cuda()
+    d_b1 = None if b1map is None else torch.from_numpy(b1map).cuda()
+    out = []
+    for call in ("screened", "plain"):
+        maps = torch.full((nvox, 5), -3.0, device="cuda")
+        idx = torch.full((nvox,), -9, dtype=torch.int64, device="cuda")
+        if call == "screened":
+            snap.MRF_match(maps, d_img, d_atoms, d_p, stride, nreps, N, natoms, nvox, in_b1map=d_b1, d_index=idx,
+                           img_stride=img.shape[1], flags=snap.MATCH_IMAG_ATOMS if imag else 0)
+        else:
+            snap.MRF_match_noalloc(maps, d_img, d_atoms, d_p, stride, nreps, N, natoms, nvox, d_b1map=d_b1,
+                                   img_stride=img.shape[1], d_index=idx)
+        torch.cuda.synchronize()
+        out.append((maps.cpu().numpy(), idx.cpu().numpy()))
+    assert snap.device_error(reset=True) == 0
+    return out
+
+
+def _inputs(nvox, natoms, T, nb, imag, seed, smooth=40.0):
+    """Atoms along a smooth two-parameter family (neighbours correlate as a
+    dictionary's do) and voxels near them."""
+    rng = np.random.default_rng(seed)
+    t = np.arange(T)[None, :] / T
+    u = np.arange(natoms)[:, None] / smooth
+    atoms = []
+    for b in range(nb):
+        f = 0.1 * np.sin(6 * t * (1 + u) + 0.2 * b) * np.exp(-t * u) + 0.05 * np.cos(25 * t + u)
+        atoms.append(1j * f if imag else f * np.exp(1j * (3 * t * u + 0.1 * b)))
+    atoms = np.concatenate(atoms)
+    atoms /= np.linalg.norm(atoms, axis=1, keepdims=True)
+    s = atoms[rng.integers(0, len(atoms), nvox)] + 0.2 * atoms[rng.integers(0, len(atoms), nvox)]
+    s = s * (rng.uniform(0.5, 1, nvox) * np.exp(6.28j * rng.uniform(size=nvox)))[:, None]
+    s = s + 0.02 / np.sqrt(T) * (rng.standard_normal(s.shape) + 1j * rng.standard_normal(s.shape))
+    params = rng.uniform(1, 100, (len(atoms), 4)).astype(np.float32)
+    params[:, 3] = np.repeat(0.8 + 0.1 * np.arange(nb), natoms)
+    return atoms.astype(np.complex64), s.astype(np.complex64), params
+
+
+@pytest.mark.parametrize("nvox,natoms,T,nb,use_map,imag,pad", [
+    (4096, 837, 100, 1, False, False, 0), (1025, 129, 257, 1, False, True, 0), (63, 4097, 128, 1, False, True, 1),
+    (129, 1283, 333, 1, False, False, 3), (1, 30000, 1000, 1, False, True, 0), (30011, 7, 97, 1, False, False, 0),
+    (2500, 300, 200, 5, True, True, 0), (1500, 257, 161, 6, True, False, 1), (20000, 1999, 64, 3, True, True, 2)])
+def test_screened_match_equals_the_fp32_kernel(snap, nvox, natoms, T, nb, use_map, imag, pad):
+    atoms, img, params = _inputs(nvox, natoms, T, nb, imag, seed=nvox + T)
+    nreps = T - pad
+    b1map = None
+    if use_map:
+        b1map = np.random.default_rng(1).uniform(0.78, 0.82 + 0.1 * (nb - 1), nvox).astype(np.float32)
+        b1map[np.abs(b1map - 0.9) < 0.05] = 0.8      # block 1: one voxel
+        b1map[5] = 0.9
+    a, b = _both(snap, img, atoms, params, nreps, natoms, b1map, imag)
+    np.testing.assert_array_equal(a[1], b[1])
+    np.testing.assert_array_equal(a[0], b[0])
+
+
+@pytest.mark.parametrize("imag", [True, False])
+def test_inputs_left_to_the_fp32_kernel(snap, imag):
+    atoms, img, params = _inputs(700, 1500, 150, 1, imag, seed=3)
+    atoms[700] = atoms[11]                        # duplicates: the lower index wins
+    atoms[1499] = atoms[1498]
+    atoms *= np.float32(10.0) ** np.random.default_rng(4).integers(-3, 4, (1500, 1))
+    img[0] = 0
+    img[1, 7] = np.nan
+    img[2, 9] = np.inf
+    img[3] = 1e-20
+    img[4] *= np.float32(1e-25)
+    img[5] *= np.float32(1e17)
+    img[6] = atoms[11]
+    img[7, 1:] = 0
+    # (an infinite voxel: the complex form's products of the zero real parts
+    # are NaN, the imaginary form has no such products and scores inf; the
+    # comparison call is the complex form)
+    same = np.arange(700) != 2 if imag else slice(None)
+    a, b = _both(snap, img, atoms, params, 150, 1500, None, imag)
+    np.testing.assert_array_equal(a[1][same], b[1][same])
+    np.testing.assert_array_equal(a[0][same], b[0][same])
+    for value in (np.inf, np.nan, 1e25, 1e-22):   # an atom out of the screen's range
+        bad = atoms.copy()
+        bad[77, 5] = complex(0.0, value)
+        a, b = _both(snap, img, bad, params, 150, 1500, None, imag)
+        np.testing.assert_array_equal(a[1][same], b[1][same])
+        np.testing.assert_array_equal(a[0][same], b[0][same])
+    a, b = _both(snap, img, atoms * np.float32(1e-19), params, 150, 1500, None, imag)
+    np.testing.assert_array_equal(a[1][same], b[1][same])
+    np.testing.assert_array_equal(a[0][same], b[0][same])
+
+
+@pytest.mark.parametrize("imag", [True, False])
+def test_more_near_ties_than_a_list_holds(snap, imag):
+    """20,000 atoms along one slow curve: hundreds lie within the bound."""
+    atoms, img, params = _inputs(300, 20000, 120, 1, imag, seed=8, smooth=20000.0)
+    a, b = _both(snap, img, atoms, params, 120, 20000, None, imag)
+    np.testing.assert_array_equal(a[1], b[1])
+    np.testing.assert_array_equal(a[0], b[0])
