@@ -602,22 +602,61 @@ __global__ void reduce_gram_kernel(typename Ty<REAL>::d *G, const typename Ty<RE
 // or below 1e-18 of the trace; the iteration stops after a sweep that
 // rotates nothing (at most 40 sweeps).  Output: eigenvalues descending
 // (lam[b][i]) and eigenvectors as columns (W[b][a][i]).
+// One rotated pair, x_p <- c x_p - s e x_q, x_q <- s x_p + c e x_q.
+struct Rot {
+    int p, q;
+    double c, s, er, ei;
+};
+// A round's pairs, an array per field (the lanes of a warp read neighbours).
+struct Rots {
+    int p[KMAX / 2], q[KMAX / 2];
+    double c[KMAX / 2], s[KMAX / 2], er[KMAX / 2], ei[KMAX / 2];
+    __device__ __forceinline__ Rot get(int i) const { return {p[i], q[i], c[i], s[i], er[i], ei[i]}; }
+};
 template <bool REAL>
-__global__ void __launch_bounds__(THREADS) jacobi_kernel(const typename Ty<REAL>::d *G, typename Ty<REAL>::d *W,
-                                                         double *lam, int k) {
+__device__ __forceinline__ void rotate(const Rot &j, double ei, double &pr, double &pi, double &qr, double &qi) {
+    const double xpr = pr, xqr = qr;
+    if constexpr (REAL) {
+        const double eq = j.er * xqr;
+        pr = j.c * xpr - j.s * eq;
+        qr = j.s * xpr + j.c * eq;
+    } else {
+        const double xpi = pi, xqi = qi;
+        const double eqr = j.er * xqr - ei * xqi, eqi = j.er * xqi + ei * xqr;
+        pr = j.c * xpr - j.s * eqr;
+        pi = j.c * xpi - j.s * eqi;
+        qr = j.s * xpr + j.c * eqr;
+        qi = j.s * xpi + j.c * eqi;
+    }
+}
+
+// A round is two phases: the angles of its pairs (a thread each, a chain of
+// FP64 divisions and roots) while the other warps apply the round before to V,
+// and then A, one 2 x 2 block (rows of pair i, columns of pair j) at a time:
+// columns and rows in one pass over shared memory, a thread keeping its
+// column pair's angle.  The operations on every entry are those of separate
+// column and row passes.  Bound by the angles' chain (a root, two divisions
+// and a root one after the other, FP64) and the phases' barriers.  Five blocks
+// of 72 vectors: the atoms' first Gram matrix 6.36 -> 2.65 ms, all eight
+// problems of a compression 15.0 -> 6.3 ms (256 threads, an integer division
+// per entry, three passes and three barriers per round before).
+constexpr int JACOBI_THREADS = 1024, ANGLE_THREADS = 64;
+template <bool REAL>
+__global__ void __launch_bounds__(JACOBI_THREADS) jacobi_kernel(const typename Ty<REAL>::d *G,
+                                                                typename Ty<REAL>::d *W, double *lam, int k) {
     using D = typename Ty<REAL>::d;
     extern __shared__ double jsm[];
     const int n = k + (k & 1), ld = n + 1, h = n / 2;
     double *Ar = jsm, *Vr = Ar + n * ld;
     double *Ai = REAL ? nullptr : Vr + n * ld;
     double *Vi = REAL ? nullptr : Ai + n * ld;
-    __shared__ int sp[KMAX / 2], sq[KMAX / 2];
-    __shared__ double sc[KMAX / 2], ss[KMAX / 2], ser[KMAX / 2], sei[KMAX / 2];
-    __shared__ double red_off[1];
+    __shared__ Rots rot[2];
+    __shared__ double trace;
     __shared__ int done;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+    static_assert(KMAX / 2 <= ANGLE_THREADS, "a thread per pair");
     const D *g = G + (long long)blockIdx.x * k * k;
-    for (int e = tid; e < n * n; e += THREADS) {
+    for (int e = tid; e < n * n; e += JACOBI_THREADS) {
         const int r = e / n, c = e % n;
         const D v = (r < k && c < k) ? g[r * k + c] : zero_<D>();
         if constexpr (REAL) {
@@ -634,116 +673,114 @@ __global__ void __launch_bounds__(THREADS) jacobi_kernel(const typename Ty<REAL>
     if (tid == 0) {
         double tr = 0.0;
         for (int a = 0; a < n; a++) tr += fabs(Ar[a * ld + a]);
-        red_off[0] = tr;
+        trace = tr;
     }
     __syncthreads();
-    const double floor_abs = 1e-18 * red_off[0];
+    const double floor_abs = 1e-18 * trace;
     const double tol = 2.2e-16 * n;
+    // V <- V J of one round, a pair per warp from warp `first` on
+    auto turn_v = [&](const Rots &rt, int first) {
+        for (int i = warp - first; i < h; i += JACOBI_THREADS / 32 - first) {
+            const Rot j = rt.get(i);
+            if (j.s == 0.0) continue;
+            for (int row = lane; row < n; row += 32) {
+                double pi = 0.0, qi = 0.0, pr = Vr[row * ld + j.p], qr = Vr[row * ld + j.q];
+                if constexpr (!REAL) {
+                    pi = Vi[row * ld + j.p];
+                    qi = Vi[row * ld + j.q];
+                }
+                rotate<REAL>(j, j.ei, pr, pi, qr, qi);
+                Vr[row * ld + j.p] = pr;
+                Vr[row * ld + j.q] = qr;
+                if constexpr (!REAL) {
+                    Vi[row * ld + j.p] = pi;
+                    Vi[row * ld + j.q] = qi;
+                }
+            }
+        }
+    };
+    // this thread's column pair and first row pair of A
+    const int bj = tid % h, bi0 = tid / h, bstep = JACOBI_THREADS / h;
+    int it = 0;  // rounds so far: round it's angles are in rot[it & 1]
     for (int sweep = 0; sweep < 40; sweep++) {
         if (tid == 0) done = 1;
         __syncthreads();
-        for (int r = 0; r < n - 1; r++) {
-            if (tid < h) {
-                auto idx = [&](int pos) { return pos == 0 ? 0 : 1 + (pos - 1 + r) % (n - 1); };
-                int p = idx(tid), q = idx(n - 1 - tid);
-                if (p > q) {
-                    const int t = p;
-                    p = q;
-                    q = t;
+        for (int r = 0; r < n - 1; r++, it++) {
+            Rots &rt = rot[it & 1];
+            if (tid < ANGLE_THREADS) {
+                if (tid < h) {
+                    auto idx = [&](int pos) { return pos == 0 ? 0 : 1 + (pos - 1 + r) % (n - 1); };
+                    int p = idx(tid), q = idx(n - 1 - tid);
+                    if (p > q) {
+                        const int t = p;
+                        p = q;
+                        q = t;
+                    }
+                    const double app = Ar[p * ld + p], aqq = Ar[q * ld + q];
+                    const double apr = Ar[p * ld + q], api = REAL ? 0.0 : Ai[p * ld + q];
+                    const double mag = REAL ? fabs(apr) : hypot(apr, api);
+                    // rotate unless |a_pq| is negligible against the diagonal
+                    // (relative) or against the whole matrix (null directions)
+                    const double theta = (aqq - app) / (2.0 * mag);  // (beside the test's root)
+                    const bool turn = mag > floor_abs && mag > tol * sqrt(fabs(app * aqq));
+                    Rot j = {p, q, 1.0, 0.0, 1.0, 0.0};
+                    if (turn) {
+                        const double t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+                        j.c = 1.0 / sqrt(t * t + 1.0);
+                        j.s = t * j.c;
+                        // e^{-i phi} = conj(a_pq) / |a_pq| (real: exactly +-1)
+                        j.er = REAL ? copysign(1.0, apr) : apr / mag;
+                        j.ei = REAL ? 0.0 : -api / mag;
+                    }
+                    rt.p[tid] = j.p;
+                    rt.q[tid] = j.q;
+                    rt.c[tid] = j.c;
+                    rt.s[tid] = j.s;
+                    rt.er[tid] = j.er;
+                    rt.ei[tid] = j.ei;
+                    if (turn) done = 0;
                 }
-                const double app = Ar[p * ld + p], aqq = Ar[q * ld + q];
-                const double apr = Ar[p * ld + q], api = REAL ? 0.0 : Ai[p * ld + q];
-                const double mag = REAL ? fabs(apr) : hypot(apr, api);
-                double c = 1.0, s = 0.0, er = 1.0, ei = 0.0;
-                // rotate unless |a_pq| is negligible against the diagonal
-                // (relative) or against the whole matrix (null directions)
-                if (mag > floor_abs && mag > tol * sqrt(fabs(app * aqq))) {
-                    const double theta = (aqq - app) / (2.0 * mag);
-                    const double t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-                    c = 1.0 / sqrt(t * t + 1.0);
-                    s = t * c;
-                    er = apr / mag;   // e^{-i phi} = conj(a_pq) / |a_pq|
-                    ei = -api / mag;
-                    done = 0;
-                }
-                sp[tid] = p;
-                sq[tid] = q;
-                sc[tid] = c;
-                ss[tid] = s;
-                ser[tid] = er;
-                sei[tid] = ei;
+            } else if (it > 0) {
+                turn_v(rot[(it & 1) ^ 1], ANGLE_THREADS / 32);
             }
             __syncthreads();
-            // columns: X <- X J for A and V (X_rp, X_rq) -> (c X_rp - s e X_rq, s X_rp + c e X_rq)
-            for (int e = tid; e < n * h; e += THREADS) {
-                const int row = e / h, i = e % h;
-                if (ss[i] == 0.0) continue;
-                const int p = sp[i], q = sq[i];
-                const double c = sc[i], s = ss[i], er = ser[i], ei = sei[i];
-                {
-                    const double xpr = Ar[row * ld + p], xqr = Ar[row * ld + q];
-                    if constexpr (REAL) {
-                        const double eq = er * xqr;
-                        Ar[row * ld + p] = c * xpr - s * eq;
-                        Ar[row * ld + q] = s * xpr + c * eq;
-                    } else {
-                        const double xpi = Ai[row * ld + p], xqi = Ai[row * ld + q];
-                        const double eqr = er * xqr - ei * xqi, eqi = er * xqi + ei * xqr;
-                        Ar[row * ld + p] = c * xpr - s * eqr;
-                        Ai[row * ld + p] = c * xpi - s * eqi;
-                        Ar[row * ld + q] = s * xpr + c * eqr;
-                        Ai[row * ld + q] = s * xpi + c * eqi;
+            // A <- J^H A J: columns (X_rp, X_rq) -> (c X_rp - s e X_rq, s X_rp
+            // + c e X_rq), then rows with conj(e); the rotated pair's
+            // off-diagonal entries are set to 0 and its diagonal made real
+            const Rot rj = rt.get(bj);
+            for (int bi = bi0; bi < h && bi0 < bstep; bi += bstep) {
+                const Rot ri = rt.get(bi);
+                if (ri.s == 0.0 && rj.s == 0.0) continue;
+                // [row p_i / q_i][column p_j / q_j]
+                const int at[2][2] = {{ri.p * ld + rj.p, ri.p * ld + rj.q}, {ri.q * ld + rj.p, ri.q * ld + rj.q}};
+                double xr[2][2], xi[2][2];
+#pragma unroll
+                for (int u = 0; u < 2; u++)
+#pragma unroll
+                    for (int v = 0; v < 2; v++) {
+                        xr[u][v] = Ar[at[u][v]];
+                        xi[u][v] = REAL ? 0.0 : Ai[at[u][v]];
+                    }
+                if (rj.s != 0.0) {
+#pragma unroll
+                    for (int u = 0; u < 2; u++) rotate<REAL>(rj, rj.ei, xr[u][0], xi[u][0], xr[u][1], xi[u][1]);
+                }
+                if (ri.s != 0.0) {
+#pragma unroll
+                    for (int v = 0; v < 2; v++) rotate<REAL>(ri, -ri.ei, xr[0][v], xi[0][v], xr[1][v], xi[1][v]);
+                    if (bi == bj) {
+                        xr[0][1] = xi[0][1] = 0.0;  // A_pq
+                        xr[1][0] = xi[1][0] = 0.0;  // A_qp
+                        xi[0][0] = xi[1][1] = 0.0;  // A_pp, A_qq real
                     }
                 }
-                {
-                    const double xpr = Vr[row * ld + p], xqr = Vr[row * ld + q];
-                    if constexpr (REAL) {
-                        const double eq = er * xqr;
-                        Vr[row * ld + p] = c * xpr - s * eq;
-                        Vr[row * ld + q] = s * xpr + c * eq;
-                    } else {
-                        const double xpi = Vi[row * ld + p], xqi = Vi[row * ld + q];
-                        const double eqr = er * xqr - ei * xqi, eqi = er * xqi + ei * xqr;
-                        Vr[row * ld + p] = c * xpr - s * eqr;
-                        Vi[row * ld + p] = c * xpi - s * eqi;
-                        Vr[row * ld + q] = s * xpr + c * eqr;
-                        Vi[row * ld + q] = s * xpi + c * eqi;
+#pragma unroll
+                for (int u = 0; u < 2; u++)
+#pragma unroll
+                    for (int v = 0; v < 2; v++) {
+                        Ar[at[u][v]] = xr[u][v];
+                        if constexpr (!REAL) Ai[at[u][v]] = xi[u][v];
                     }
-                }
-            }
-            __syncthreads();
-            // rows: A <- J^H A, (A_pc, A_qc) -> (c A_pc - s conj(e) A_qc, s A_pc + c conj(e) A_qc);
-            // the rotated pair's off-diagonal entries are set to 0 and its
-            // diagonal made real
-            for (int e = tid; e < h * n; e += THREADS) {
-                const int i = e / n, col = e % n;
-                if (ss[i] == 0.0) continue;
-                const int p = sp[i], q = sq[i];
-                const double c = sc[i], s = ss[i], er = ser[i], ei = -sei[i];
-                const double xpr = Ar[p * ld + col], xqr = Ar[q * ld + col];
-                double npr, nqr, npi = 0.0, nqi = 0.0;
-                if constexpr (REAL) {
-                    const double eq = er * xqr;
-                    npr = c * xpr - s * eq;
-                    nqr = s * xpr + c * eq;
-                } else {
-                    const double xpi = Ai[p * ld + col], xqi = Ai[q * ld + col];
-                    const double eqr = er * xqr - ei * xqi, eqi = er * xqi + ei * xqr;
-                    npr = c * xpr - s * eqr;
-                    npi = c * xpi - s * eqi;
-                    nqr = s * xpr + c * eqr;
-                    nqi = s * xpi + c * eqi;
-                }
-                if (col == q) npr = npi = 0.0;  // A_pq
-                if (col == p) nqr = nqi = 0.0;  // A_qp
-                if (col == p) npi = 0.0;        // A_pp real
-                if (col == q) nqi = 0.0;        // A_qq real
-                Ar[p * ld + col] = npr;
-                Ar[q * ld + col] = nqr;
-                if constexpr (!REAL) {
-                    Ai[p * ld + col] = npi;
-                    Ai[q * ld + col] = nqi;
-                }
             }
             __syncthreads();
         }
@@ -752,6 +789,8 @@ __global__ void __launch_bounds__(THREADS) jacobi_kernel(const typename Ty<REAL>
         __syncthreads();
         if (finished) break;
     }
+    if (it > 0) turn_v(rot[(it & 1) ^ 1], 0);
+    __syncthreads();
     // descending order (ties by index)
     if (tid < k) {
         const double v = Ar[tid * ld + tid];
@@ -1047,7 +1086,7 @@ int compress(const float2 *atoms, long long astride, long long nreps, long long 
         SNAPMRF_LAUNCH_CHECK();
         reduce_gram_kernel<REAL><<<nblk(nb * k * k, 256), 256, 0, st>>>(G, Gp, nb, g.splits, k, atom_side ? 1 : 0);
         SNAPMRF_LAUNCH_CHECK();
-        jacobi_kernel<REAL><<<(unsigned)nb, THREADS, jac_smem, st>>>(G, W, lam, k);
+        jacobi_kernel<REAL><<<(unsigned)nb, JACOBI_THREADS, jac_smem, st>>>(G, W, lam, k);
         SNAPMRF_LAUNCH_CHECK();
         return SNAPMRF_OK;
     };
