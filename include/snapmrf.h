@@ -137,7 +137,10 @@ void snapmrf_ra_free(snapmrf_ra *a);
  * only epg_ssfp and roa_ssfp, src/functions.cu:1268, 1297). */
 #define SNAPMRF_DICT_NORMALIZE 0x2u
 /* Use the reference's operation order (complex state, separate relaxation
- * and RF steps) even where the real-valued fast recursion applies. */
+ * and RF steps) even where a faster recursion applies: the real-valued one,
+ * and for epg_ssfp the one in the frame of the RF phase (which
+ * SNAPMRF_DICT_SEPARATE_RELAX turns off too; its atoms differ by rounding,
+ * about 2e-6 of their peak). */
 #define SNAPMRF_DICT_REFERENCE_ORDER 0x4u
 /* Real-valued recursion (FISP / SR with every RF phase 0) with the
  * reference's two relaxations per step, bit-identical to the complex

@@ -21,6 +21,7 @@
 
 #include "common.h"
 #include "epg_kernels.cuh"
+#include "epg_ssfp_kernel.cuh"
 
 namespace snapmrf {
 
@@ -175,6 +176,22 @@ static cudaError_t launch_epg_ref(const EpgArgs &a, dim3 grid, cudaStream_t st) 
     k<<<grid, kEpgThreads, smem, st>>>(a);
     note_launches(1);
     return cudaGetLastError();
+}
+
+template <int S>
+static cudaError_t launch_ssfp(const EpgArgs &a, dim3 grid, cudaStream_t st) {
+    auto k = a.L * S - a.nstates <= 3 ? epg_ssfp_kernel<S, true> : epg_ssfp_kernel<S, false>;
+    k<<<grid, 32, epg_ssfp_smem_bytes(a.L), st>>>(a);
+    note_launches(1);
+    return cudaGetLastError();
+}
+
+template <int S = kSsfpMaxStates>
+static cudaError_t dispatch_ssfp(const EpgArgs &a, int states, dim3 grid, cudaStream_t st) {
+    if constexpr (S > 1) {
+        if (states < S) return dispatch_ssfp<S - 1>(a, states, grid, st);
+    }
+    return launch_ssfp<S>(a, grid, st);
 }
 
 template <int ECHO>
@@ -478,12 +495,27 @@ static int dict_impl(float *d_atoms, const float *d_params, const float *h_mrf, 
         a.packed_pitch = (long long)snapmrf_packed_pitch(nreps);
     }
     int L, S;
-    if (real_path)
+    // bSSFP in the frame of the RF phase, unless the reference's order of
+    // operations is asked for
+    const bool ssfp_path = echo == ECHO_SSFP && !(flags & (SNAPMRF_DICT_REFERENCE_ORDER | SNAPMRF_DICT_SEPARATE_RELAX));
+    if (real_path) {
         choose_layout(nstates, kMaxRealStatesPerLane, 2, &L, &S);
-    else
+    } else if (ssfp_path) {
+        choose_layout(nstates, kSsfpMaxStates, 1, &L, &S);
+        // few atoms: more lanes per atom, for at least two warps per scheduler
+        // (a step is a chain that more lanes shorten)
+        int dev = 0, sms = 0;
+        SNAPMRF_CUDA(cudaGetDevice(&dev));
+        SNAPMRF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        while (L < 32 && S > 1 && gen_blocks * natoms * L < (size_t)sms * 8 * 32) {
+            L *= 2;
+            S = (nstates + L - 1) / L;
+        }
+    } else {
         choose_layout(nstates, kMaxStatesPerLane, 1, &L, &S);
+    }
     a.L = L;
-    const int apc = (real_path ? kRealThreads : kEpgThreads) / L;
+    const int apc = (real_path ? kRealThreads : ssfp_path ? 32 : kEpgThreads) / L;
     dim3 grid((unsigned)((natoms + apc - 1) / apc), (unsigned)gen_blocks);
     if (grid.x > 0x7fffffffu) SNAPMRF_FAIL(SNAPMRF_ERR_UNSUPPORTED, "MRF_dict: grid too large");
     if (real_path) {
@@ -509,6 +541,8 @@ static int dict_impl(float *d_atoms, const float *d_params, const float *h_mrf, 
             pack_operand_kernel<<<(unsigned)blocks, 256, 0, st>>>(a, total);
             SNAPMRF_LAUNCH_CHECK();
         }
+    } else if (ssfp_path) {
+        SNAPMRF_CUDA(dispatch_ssfp(a, S, grid, st));
     } else {
         SNAPMRF_CUDA(launch_epg(echo, a, S, grid, st));
     }
