@@ -24,6 +24,7 @@
 #include "common.h"
 #define SNAPMRF_EPG_DEVICE_HELPERS_ONLY
 #include "epg_kernels.cuh"
+#include "epg_ssfp_kernel.cuh"
 
 namespace snapmrf {
 namespace ssfpgrad {
@@ -32,14 +33,14 @@ constexpr int kThreads = 32;   // one warp per CTA: no CTA barrier couples voxel
 constexpr int kStepChunk = 16; // time steps staged per chunk
 
 // Per-(voxel, step) constants staged in shared memory.
-struct Step {
-    float E1a, E2a, E1b, E2b;      // relaxation over TE and over TR - TE
-    float dE1a, dE2a, dE1b, dE2b;  // their derivatives by T1 / T2
-    float2 ea, eb;                 // B0 phasors over TE and TR - TE
-    float tha, thb;                // d(phase)/dB0 over TE and TR - TE (rad / Hz)
-    float ca, sa, fa;              // cos, sin of alpha_t * B1; alpha_t (d alpha / dB1)
-    float2 z;                      // (cos phi_t, sin phi_t)
-    float2 x;                      // voxel sample
+struct alignas(16) Step {
+    float C, S, E1, rec;       // cos, sin of alpha_t * B1; Z's relaxation over the TR before, its recovery
+    float2 w;                  // the TR's factor on F+ (see gn_ssfp_kernel)
+    float kappa, theta;        // d log w / dT2 and / dB0 (/ i) over TR
+    float dE1, fa;             // dE1/dT1; alpha_t (d alpha / dB1)
+    float R, kappa_e;          // |r|^2 of the readout factor r = E2 e^{i theta} z over TE; d log r / dT2
+    float2 x;                  // conj(r) x_t
+    float theta_e, pad;        // d log r / dB0 (/ i)
 };
 
 struct Args {
@@ -103,71 +104,6 @@ __device__ __forceinline__ void zero(LaneState<S> &s) {
     for (int j = 0; j < S; j++) s.fp[j] = s.fm[j] = s.zz[j] = make_float2(0.f, 0.f);
 }
 
-// d <- T d (+ g dT s when WITH_S)
-template <int S, bool WITH_S>
-__device__ __forceinline__ void rf_apply(LaneState<S> &d, const float2 *T, const float2 *dT, float g,
-                                         const LaneState<S> &s) {
-#pragma unroll
-    for (int j = 0; j < S; j++) {
-        const float2 o0 = d.fp[j], o1 = d.fm[j], o2 = d.zz[j];
-        float2 r0 = rf_row(T[0], T[1], T[2], o0, o1, o2);
-        float2 r1 = rf_row(T[3], T[4], T[5], o0, o1, o2);
-        float2 r2 = rf_row(T[6], T[7], T[8], o0, o1, o2);
-        if (WITH_S) {
-            const float2 q0 = rf_row(dT[0], dT[1], dT[2], s.fp[j], s.fm[j], s.zz[j]);
-            const float2 q1 = rf_row(dT[3], dT[4], dT[5], s.fp[j], s.fm[j], s.zz[j]);
-            const float2 q2 = rf_row(dT[6], dT[7], dT[8], s.fp[j], s.fm[j], s.zz[j]);
-            r0.x = fmaf(g, q0.x, r0.x); r0.y = fmaf(g, q0.y, r0.y);
-            r1.x = fmaf(g, q1.x, r1.x); r1.y = fmaf(g, q1.y, r1.y);
-            r2.x = fmaf(g, q2.x, r2.x); r2.y = fmaf(g, q2.y, r2.y);
-        }
-        d.fp[j] = r0;
-        d.fm[j] = r1;
-        d.zz[j] = r2;
-    }
-}
-
-// Tangent relaxation: d <- E d + dE s on the channels that depend on the
-// parameter (which = 0: T1, Z and the recovery; 1: T2, F+ and F-; else none).
-template <int S>
-__device__ __forceinline__ void relax_tangent(LaneState<S> &d, const LaneState<S> &s, float E1, float E2, float dE1,
-                                              float dE2, int which, bool lane0) {
-#pragma unroll
-    for (int j = 0; j < S; j++) {
-        if (which == 1) {
-            d.fp[j] = make_float2(fmaf(dE2, s.fp[j].x, E2 * d.fp[j].x), fmaf(dE2, s.fp[j].y, E2 * d.fp[j].y));
-            d.fm[j] = make_float2(fmaf(dE2, s.fm[j].x, E2 * d.fm[j].x), fmaf(dE2, s.fm[j].y, E2 * d.fm[j].y));
-        } else {
-            d.fp[j] = c_scale(d.fp[j], E2);
-            d.fm[j] = c_scale(d.fm[j], E2);
-        }
-        if (which == 0)
-            d.zz[j] = make_float2(fmaf(dE1, s.zz[j].x, E1 * d.zz[j].x), fmaf(dE1, s.zz[j].y, E1 * d.zz[j].y));
-        else
-            d.zz[j] = c_scale(d.zz[j], E1);
-    }
-    if (which == 0 && lane0) d.zz[0].x -= dE1;  // d(1 - E1)
-}
-
-// Tangent B0 precession after the signal's: d <- e d (+ i th s_new on F+,
-// - i th s_new on F- for the B0 tangent).
-template <int S>
-__device__ __forceinline__ void b0_tangent(LaneState<S> &d, const LaneState<S> &s_new, float2 e, float th, bool b0) {
-    const float2 ec = c_conj(e);
-#pragma unroll
-    for (int j = 0; j < S; j++) {
-        float2 p = c_mul(e, d.fp[j]), m = c_mul(ec, d.fm[j]);
-        if (b0) {
-            p.x = fmaf(-th, s_new.fp[j].y, p.x);
-            p.y = fmaf(th, s_new.fp[j].x, p.y);
-            m.x = fmaf(th, s_new.fm[j].y, m.x);
-            m.y = fmaf(-th, s_new.fm[j].x, m.y);
-        }
-        d.fp[j] = p;
-        d.fm[j] = m;
-    }
-}
-
 // Cholesky solve of the NT x NT system A d = b (A symmetric positive
 // definite up to a relative diagonal jitter); false when it is not.
 template <int NT>
@@ -214,25 +150,109 @@ __device__ __forceinline__ bool solve_spd(float (&A)[NT][NT], float (&b)[NT], fl
     return true;
 }
 
+// EPG states of one stream in the frame of the RF phase (epg_ssfp_kernel.cuh):
+// p = conj(z) F+, m = z F-, y = -i Z.
+template <int S>
+struct Frame {
+    float2 p[S], m[S], y[S];
+};
+
+struct FrameRF {
+    float2 c, s, S, h, C;  // (1 + cos)/2, (1 - cos)/2, E1 sin, -sin/2, E1 cos
+};
+
+__device__ __forceinline__ float2 dup(float v) { return make_float2(v, v); }
+
+// The pulse, the interval's relaxation of Z folded in.  SRC (the T1 tangent):
+// Z gains dE1 times the signal's before the pulse, S2 = dE1 sin, C2 = dE1 cos.
+template <int S, bool SRC>
+__device__ __forceinline__ void frame_rf(Frame<S> &x, const FrameRF &k, const float2 *src, float2 S2, float2 C2) {
+    const float2 minus = make_float2(-1.f, -1.f);
+#pragma unroll
+    for (int j = 0; j < S; j++) {
+        const float2 u = x.p[j], v = x.m[j], q = x.y[j];
+        float2 np = __ffma2_rn(k.S, q, __ffma2_rn(k.s, v, __fmul2_rn(k.c, u)));
+        float2 ny = __ffma2_rn(k.C, q, __fmul2_rn(k.h, __ffma2_rn(v, minus, u)));
+        if (SRC) {
+            np = __ffma2_rn(S2, src[j], np);
+            ny = __ffma2_rn(C2, src[j], ny);
+        }
+        x.m[j] = __ffma2_rn(np, minus, __fadd2_rn(u, v));
+        x.p[j] = np;
+        x.y[j] = ny;
+    }
+}
+
+// The interval's factor on F+ (its conjugate on F-) and the dephasing shift.
+// src_up / src_dn: the neighbouring lanes of the group.  padded: slot w exists
+// and is cleared.
+template <int S>
+__device__ __forceinline__ void frame_shift(Frame<S> &x, float2 w, int gl, int L, int nstates, int src_up, int src_dn,
+                                            bool padded) {
+    const unsigned full = 0xffffffffu;
+    const float2 up = make_float2(__shfl_sync(full, x.p[S - 1].x, src_up), __shfl_sync(full, x.p[S - 1].y, src_up));
+    float2 dn = make_float2(__shfl_sync(full, x.m[0].x, src_dn), __shfl_sync(full, x.m[0].y, src_dn));
+    const float2 m0 = x.m[0];
+    if (gl == L - 1) dn = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int j = S - 1; j >= 1; j--) x.p[j] = c_mul_fma(w, x.p[j - 1]);
+    x.p[0] = c_mul_fma(w, up);
+#pragma unroll
+    for (int j = 0; j < S - 1; j++) x.m[j] = c_mul_conj(w, x.m[j + 1]);
+    x.m[S - 1] = c_mul_conj(w, dn);
+    if (gl == 0) x.p[0] = nstates == 1 ? c_conj(c_mul_conj(w, m0)) : c_conj(x.m[0]);
+    if (padded) {
+#pragma unroll
+        for (int j = 0; j < S; j++)
+            if (gl * S + j == nstates) x.p[j] = make_float2(0.f, 0.f);
+    }
+}
+
+// Sums of one voxel: <s,s>, <s,x>, <s,J_j>, <J_j,x>, Re<J_j,J_k> (j <= k).
+__host__ __device__ constexpr int gn_sums(int nt) { return 3 + 4 * nt + nt * (nt + 1) / 2; }
+
 // One Gauss-Newton iteration per voxel of the list (NT = 3: T1, T2, B0 with
 // B1 from the map; NT = 4: B1 refined too) or, with NT = 0, the value-only
-// evaluation of PD and M0.  L lanes per voxel, S complex states per lane.
+// evaluation of PD and M0.  L lanes per voxel (any number: 32 / L voxels per
+// warp, the remaining lanes idle), S complex states per lane.
+//
+// The signal and its tangents run in the frame of the RF phase: 24 operations
+// per state and step for each stream, and for the tangents
+//   T1  dE1 times the signal's Y through the pulse             4 more
+//   T2  w (d + kappa s), kappa = TR / T2^2                     4 more
+//   B0  w (d +- i theta' s), theta' = 2 pi TR / 1000           8 more
+//   B1  alpha_t G s after the pulse (dM/da = G M, G its
+//       generator: (Y, -Y, -(F+ - F-)/2))                      8 more
+// instead of 64 and more for each in the reference's order.  The readout's
+// factor r is common to the signal and the tangents, so it goes to the sample
+// (conj(r) x) and the weight |r|^2; the readouts are staged and the sums taken
+// for a chunk at once, one step per lane, in shared memory (29 registers of
+// every lane otherwise).  16,384 voxels, T = 500, w = 50, T1, T2, B0 and B1: a pass
+// 7.97 -> 3.12 ms (1.6 of it the 144 operations at the measured FP32 peak; 3
+// voxels per warp, 8 warps per SM at 234 registers).
 template <int S, int NT>
 __global__ void __launch_bounds__(kThreads) gn_ssfp_kernel(Args a) {
     extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int NS = gn_sums(NT), NJ = NT + 1;
     const int L = a.L, apc = kThreads / L;
-    const int tid = threadIdx.x, g = tid / L, gl = tid % L;
-    const bool lane0 = gl == 0;
-    Step *sQ = reinterpret_cast<Step *>(smem);                      // [apc][kStepChunk]
-    float *sV = reinterpret_cast<float *>(sQ + apc * kStepChunk);   // [apc][6]: T1 T2 B0 B1 ok pad
-    long long *sI = reinterpret_cast<long long *>(sV + apc * 6);    // [apc]
+    const int lane = threadIdx.x, gl = lane % L;
+    const bool idle = lane >= apc * L, lane0 = gl == 0;
+    const int g = min(lane / L, apc - 1);
+    const int src_up = gl == 0 ? lane : lane - 1, src_dn = lane + 1 < 32 ? lane + 1 : lane;
+    Step *sQ = reinterpret_cast<Step *>(smem);                                  // [apc][kStepChunk]
+    float2 *sJ = reinterpret_cast<float2 *>(sQ + apc * kStepChunk);             // [apc][kStepChunk][NJ]
+    float *sA = reinterpret_cast<float *>(sJ + apc * kStepChunk * NJ);          // [NS][32]
+    float2 *sZ = reinterpret_cast<float2 *>(sA + NS * 32);                      // [kStepChunk + 1] frames
+    float *sV = reinterpret_cast<float *>(sZ + kStepChunk + 1);                 // [apc][6]: T1 T2 B0 B1 ok pad
+    long long *sI = reinterpret_cast<long long *>(sV + ((apc * 6 + 1) & ~1));   // [apc]
     const long long vox0 = (long long)blockIdx.x * apc;
     const long long nlist = a.list_in ? (long long)*a.count_in : a.nvox;
-    for (int i = tid; i < apc; i += kThreads) {
-        const long long slot = vox0 + i;
+    bool any = false;
+    if (lane < apc) {
+        const long long slot = vox0 + lane;
         long long v = -1;
         if (slot < nlist) v = a.list_in ? (long long)a.list_in[slot] : slot;
-        sI[i] = v;
+        sI[lane] = v;
         float T1 = 2.f, T2 = 1.f, B0 = 0.f, B1 = 1.f, ok = 0.f;
         if (v >= 0) {
             const float *mp = a.maps + v * a.nmaps;
@@ -244,137 +264,217 @@ __global__ void __launch_bounds__(kThreads) gn_ssfp_kernel(Args a) {
                 B0 = b0;
                 B1 = b1;
                 ok = 1.f;
+                any = true;
             }
         }
-        sV[6 * i] = T1;
-        sV[6 * i + 1] = T2;
-        sV[6 * i + 2] = B0;
-        sV[6 * i + 3] = B1;
-        sV[6 * i + 4] = ok;
+        sV[6 * lane] = T1;
+        sV[6 * lane + 1] = T2;
+        sV[6 * lane + 2] = B0;
+        sV[6 * lane + 3] = B1;
+        sV[6 * lane + 4] = ok;
     }
-    if (!__syncthreads_or(tid < apc && sV[6 * tid + 4] != 0.f)) return;
+#pragma unroll
+    for (int k = 0; k < NS; k++) sA[k * 32 + lane] = 0.f;
+    __syncwarp();
+    if (!__any_sync(0xffffffffu, any)) return;
     const long long v = sI[g];
-    const bool active = sV[6 * g + 4] != 0.f;
+    const bool active = !idle && sV[6 * g + 4] != 0.f;
     const int T = a.nreps, w = a.w;
     const float T1 = sV[6 * g], T2 = sV[6 * g + 1];
+    const bool padded = L * S > w;
 
-    LaneState<S> s;
-    LaneState<S> d[NT > 0 ? NT : 1];
-    // inversion (init_rf_pulse, src/functions.cu:456-481) with the signal's
-    // float expressions of st_init; its tangents by T1 and T2
-    st_init<S>(s, lane0, T1, T2, 180.f, 0.f, a.TI);
+    Frame<S> s, d[NT > 0 ? NT : 1];
 #pragma unroll
-    for (int p = 0; p < NT; p++) zero<S>(d[p]);
-    if constexpr (NT > 0) {
-        if (lane0) {
-            const float alpha = (float)(180.f * M_PI / 180.f);
-            float sa0, ca0;
-            __sincosf(alpha, &sa0, &ca0);
-            const float e1 = expf(-a.TI / T1), e2 = expf(-a.TI / T2);
-            const float de1 = e1 * a.TI / (T1 * T1), de2 = e2 * a.TI / (T2 * T2);
-            d[0].zz[0] = make_float2(de1 * (ca0 - 1.f), 0.f);
-            const float2 q = make_float2(0.f, de2 * sa0);  // d/dT2 of e2 sa (sin 0 + i cos 0)
-            d[1].fp[0] = c_conj(q);
-            d[1].fm[0] = q;
+    for (int j = 0; j < S; j++) s.p[j] = s.m[j] = s.y[j] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < NT; q++)
+#pragma unroll
+        for (int j = 0; j < S; j++) d[q].p[j] = d[q].m[j] = d[q].y[j] = make_float2(0.f, 0.f);
+    {
+        // inversion (init_rf_pulse, src/functions.cu:456-481) with the
+        // signal's float expressions of st_init; its tangents by T1 and T2
+        LaneState<1> s0;
+        st_init<1>(s0, lane0, T1, T2, 180.f, 0.f, a.TI);
+        float2 z0;
+        sincosf(a.phi[0], &z0.y, &z0.x);
+        s.p[0] = c_mul_conj(z0, s0.fp[0]);
+        s.m[0] = c_mul_fma(z0, s0.fm[0]);
+        s.y[0] = make_float2(s0.zz[0].y, -s0.zz[0].x);
+        if constexpr (NT > 0) {
+            if (lane0) {
+                const float alpha = (float)(180.f * M_PI / 180.f);
+                float sa0, ca0;
+                __sincosf(alpha, &sa0, &ca0);
+                const float e1 = expf(-a.TI / T1), e2 = expf(-a.TI / T2);
+                const float de1 = e1 * a.TI / (T1 * T1), de2 = e2 * a.TI / (T2 * T2);
+                d[0].y[0] = make_float2(0.f, -(de1 * (ca0 - 1.f)));
+                const float2 q = make_float2(0.f, de2 * sa0);  // d/dT2 of e2 sa (sin 0 + i cos 0)
+                d[1].p[0] = c_mul_conj(z0, c_conj(q));
+                d[1].m[0] = c_mul_fma(z0, q);
+            }
         }
     }
 
-    // inner products on the first lane: Ss = <s,s>, P = <s,x>, G_j = <s,J_j>,
-    // H_jk = Re<J_j,J_k>, Q_j = <J_j,x>
-    float Ss = 0.f;
-    float2 P = make_float2(0.f, 0.f);
-    float2 G[NT > 0 ? NT : 1], Q[NT > 0 ? NT : 1];
-    float H[NT > 0 ? NT : 1][NT > 0 ? NT : 1];
-#pragma unroll
-    for (int j = 0; j < NT; j++) {
-        G[j] = Q[j] = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int k = 0; k < NT; k++) H[j][k] = 0.f;
-    }
     for (int t0 = 0; t0 < T; t0 += kStepChunk) {
         const int nch = min(kStepChunk, T - t0);
-        __syncthreads();
-        for (int idx = tid; idx < apc * nch; idx += kThreads) {
+        __syncwarp();
+        if (lane <= nch) {
+            float2 z = make_float2(1.f, 0.f);
+            if (t0 + lane < T) sincosf(a.phi[t0 + lane], &z.y, &z.x);
+            sZ[lane] = z;
+        }
+        __syncwarp();
+        for (int idx = lane; idx < apc * nch; idx += kThreads) {
             const int ga = idx / nch, i = idx - ga * nch;
             const float t1 = sV[6 * ga], t2 = sV[6 * ga + 1], b0 = sV[6 * ga + 2], b1 = sV[6 * ga + 3];
             const int t = t0 + i;
             Step q;
-            const float tr = a.TR[t], te = a.TE[t];
-            const float ta = te, tb = tr - te;
-            q.E1a = expf(-ta / t1);
-            q.E2a = expf(-ta / t2);
-            q.E1b = expf(-tb / t1);
-            q.E2b = expf(-tb / t2);
-            q.dE1a = q.E1a * ta / (t1 * t1);
-            q.dE2a = q.E2a * ta / (t2 * t2);
-            q.dE1b = q.E1b * tb / (t1 * t1);
-            q.dE2b = q.E2b * tb / (t2 * t2);
-            q.ea = b0_phasor(b0, ta);
-            q.eb = b0_phasor(b0, tb);
-            q.tha = (float)(2 * M_PI * ta / 1000.0);
-            q.thb = (float)(2 * M_PI * tb / 1000.0);
+            const float tr = a.TR[t], ta = a.TE[t], tb = tr - ta;
             q.fa = a.alpha[t];
-            __sincosf(q.fa * b1, &q.sa, &q.ca);
-            float sp, cp;
-            __sincosf(a.phi[t], &sp, &cp);
-            q.z = make_float2(cp, sp);
+            __sincosf(q.fa * b1, &q.S, &q.C);
+            q.E1 = 1.f;
+            q.rec = q.dE1 = 0.f;
+            if (t > 0) {
+                const float trp = a.TR[t - 1], tep = a.TE[t - 1];
+                const float e1a = expf(-tep / t1), e1b = expf(-(trp - tep) / t1);
+                q.E1 = e1a * e1b;
+                q.rec = fmaf(1 - e1a, e1b, 1 - e1b);
+                q.dE1 = q.E1 * trp / (t1 * t1);
+            }
+            const float E2a = expf(-ta / t2), E2 = E2a * expf(-tb / t2);
+            const float2 ea = b0_phasor(b0, ta), eb = b0_phasor(b0, tb);
+            const float2 z = sZ[i], zn = sZ[i + 1];
+            q.w = c_scale(c_mul_fma(c_mul_fma(ea, eb), c_mul_conj(zn, z)), E2);
+            q.kappa = tr / (t2 * t2);
+            q.theta = (float)(2 * M_PI * tr / 1000.0);
+            q.kappa_e = ta / (t2 * t2);
+            q.theta_e = (float)(2 * M_PI * ta / 1000.0);
+            const float2 r = c_scale(c_mul_fma(ea, z), E2a);
+            q.R = fmaf(r.x, r.x, r.y * r.y);
             const long long vv = sI[ga];
-            q.x = vv >= 0 ? a.img[vv * a.img_stride + t] : make_float2(0.f, 0.f);
+            q.x = c_mul_conj(r, vv >= 0 ? a.img[vv * a.img_stride + t] : make_float2(0.f, 0.f));
+            q.pad = 0.f;
             sQ[ga * kStepChunk + i] = q;
         }
-        __syncthreads();
+        __syncwarp();
         const Step *qs = sQ + g * kStepChunk;
+        float2 *js = sJ + g * kStepChunk * NJ;
         for (int i = 0; i < nch; i++) {
             const Step q = qs[i];
-            float2 Tm[9], dT[9];
-            rf_and_derivative(q.ca, q.sa, q.z, Tm, dT);
-            // RF: tangents from the signal before the pulse, then the signal
+            FrameRF k;
+            k.c = dup((1 + q.C) / 2);
+            k.s = dup((1 - q.C) / 2);
+            k.S = dup(q.S * q.E1);
+            k.h = dup(-0.5f * q.S);
+            k.C = dup(q.C * q.E1);
+            // RF: the tangents, the T1 one from the signal before the pulse
 #pragma unroll
             for (int p = 0; p < NT; p++) {
-                if (p == 3) rf_apply<S, true>(d[p], Tm, dT, q.fa, s);
-                else rf_apply<S, false>(d[p], Tm, dT, 0.f, s);
+                if (p == 0) frame_rf<S, true>(d[p], k, s.y, dup(q.S * q.dE1), dup(q.C * q.dE1));
+                else frame_rf<S, false>(d[p], k, nullptr, k.c, k.c);
             }
-            rf_apply<S, false>(s, Tm, dT, 0.f, s);
-            // relaxation over TE
-#pragma unroll
-            for (int p = 0; p < NT; p++) relax_tangent<S>(d[p], s, q.E1a, q.E2a, q.dE1a, q.dE2a, p, lane0);
-            st_relax<S>(s, q.E1a, q.E2a, lane0);
-            // B0 over TE: the signal, then its tangents
-            st_b0<S>(s, q.ea);
-#pragma unroll
-            for (int p = 0; p < NT; p++) b0_tangent<S>(d[p], s, q.ea, q.tha, p == 2);
+            frame_rf<S, false>(s, k, nullptr, k.c, k.c);
             if (lane0) {
-                const float2 sv = s.fp[0], x = q.x;
-                Ss = fmaf(sv.x, sv.x, fmaf(sv.y, sv.y, Ss));
-                P.x = fmaf(sv.x, x.x, fmaf(sv.y, x.y, P.x));
-                P.y = fmaf(sv.x, x.y, fmaf(-sv.y, x.x, P.y));
-#pragma unroll
-                for (int j = 0; j < NT; j++) {
-                    const float2 J = d[j].fp[0];
-                    G[j].x = fmaf(sv.x, J.x, fmaf(sv.y, J.y, G[j].x));
-                    G[j].y = fmaf(sv.x, J.y, fmaf(-sv.y, J.x, G[j].y));
-                    Q[j].x = fmaf(J.x, x.x, fmaf(J.y, x.y, Q[j].x));
-                    Q[j].y = fmaf(J.x, x.y, fmaf(-J.y, x.x, Q[j].y));
-#pragma unroll
-                    for (int k = j; k < NT; k++) {
-                        const float2 K = d[k].fp[0];
-                        H[j][k] = fmaf(J.x, K.x, fmaf(J.y, K.y, H[j][k]));
-                    }
+                // Z0's recovery -i rec and its T1 derivative +i dE1
+                s.p[0].y = fmaf(-q.S, q.rec, s.p[0].y);
+                s.m[0].y = fmaf(q.S, q.rec, s.m[0].y);
+                s.y[0].y = fmaf(-q.C, q.rec, s.y[0].y);
+                if constexpr (NT > 0) {
+                    d[0].p[0].y = fmaf(q.S, q.dE1, d[0].p[0].y);
+                    d[0].m[0].y = fmaf(-q.S, q.dE1, d[0].m[0].y);
+                    d[0].y[0].y = fmaf(q.C, q.dE1, d[0].y[0].y);
                 }
             }
-            // B0 over TR - TE, shift, relaxation over TR - TE
-            st_b0<S>(s, q.eb);
+            if constexpr (NT > 3) {
+                const float2 fa = dup(q.fa), nfa = dup(-q.fa), hfa = dup(-0.5f * q.fa), minus = dup(-1.f);
 #pragma unroll
-            for (int p = 0; p < NT; p++) b0_tangent<S>(d[p], s, q.eb, q.thb, p == 2);
-            st_shift<S>(s, gl, L, w);
+                for (int j = 0; j < S; j++) {
+                    d[3].p[j] = __ffma2_rn(fa, s.y[j], d[3].p[j]);
+                    d[3].m[j] = __ffma2_rn(nfa, s.y[j], d[3].m[j]);
+                    d[3].y[j] = __ffma2_rn(hfa, __ffma2_rn(s.m[j], minus, s.p[j]), d[3].y[j]);
+                }
+            }
+            if (lane0 && !idle) {
+                js[i * NJ] = s.p[0];
 #pragma unroll
-            for (int p = 0; p < NT; p++) st_shift<S>(d[p], gl, L, w);
+                for (int p = 0; p < NT; p++) js[i * NJ + 1 + p] = d[p].p[0];
+            }
+            // the interval: what T2 and B0 change in the signal's factor ..
+            if constexpr (NT > 0) {
+                const float2 kp = dup(q.kappa);
 #pragma unroll
-            for (int p = 0; p < NT; p++) relax_tangent<S>(d[p], s, q.E1b, q.E2b, q.dE1b, q.dE2b, p, lane0);
-            st_relax<S>(s, q.E1b, q.E2b, lane0);
+                for (int j = 0; j < S; j++) {
+                    d[1].p[j] = __ffma2_rn(kp, s.p[j], d[1].p[j]);
+                    d[1].m[j] = __ffma2_rn(kp, s.m[j], d[1].m[j]);
+                    d[2].p[j].x = fmaf(-q.theta, s.p[j].y, d[2].p[j].x);
+                    d[2].p[j].y = fmaf(q.theta, s.p[j].x, d[2].p[j].y);
+                    d[2].m[j].x = fmaf(q.theta, s.m[j].y, d[2].m[j].x);
+                    d[2].m[j].y = fmaf(-q.theta, s.m[j].x, d[2].m[j].y);
+                }
+            }
+            // .. and the factor with the shift
+            frame_shift<S>(s, q.w, gl, L, w, src_up, src_dn, padded);
+#pragma unroll
+            for (int p = 0; p < NT; p++) frame_shift<S>(d[p], q.w, gl, L, w, src_up, src_dn, padded);
+        }
+        __syncwarp();
+        // this chunk's sums, a step per lane of the group
+        for (int i = gl; i < nch && !idle; i += L) {
+            const Step q = qs[i];
+            const float2 sv = js[i * NJ], x = q.x;
+            float2 J[NT > 0 ? NT : 1];
+#pragma unroll
+            for (int p = 0; p < NT; p++) J[p] = js[i * NJ + 1 + p];
+            if constexpr (NT > 0) {
+                J[1] = make_float2(fmaf(q.kappa_e, sv.x, J[1].x), fmaf(q.kappa_e, sv.y, J[1].y));
+                J[2] = make_float2(fmaf(-q.theta_e, sv.y, J[2].x), fmaf(q.theta_e, sv.x, J[2].y));
+            }
+            float *acc = sA + lane;
+            auto add = [&](int k, float val) { acc[k * 32] += val; };
+            add(0, q.R * fmaf(sv.x, sv.x, sv.y * sv.y));
+            add(1, fmaf(sv.x, x.x, sv.y * x.y));
+            add(2, fmaf(sv.x, x.y, -sv.y * x.x));
+            int n = 3;
+#pragma unroll
+            for (int j = 0; j < NT; j++) {
+                add(n++, q.R * fmaf(sv.x, J[j].x, sv.y * J[j].y));
+                add(n++, q.R * fmaf(sv.x, J[j].y, -sv.y * J[j].x));
+                add(n++, fmaf(J[j].x, x.x, J[j].y * x.y));
+                add(n++, fmaf(J[j].x, x.y, -J[j].y * x.x));
+            }
+#pragma unroll
+            for (int j = 0; j < NT; j++)
+#pragma unroll
+                for (int c = j; c < NT; c++) add(n++, q.R * fmaf(J[j].x, J[c].x, J[j].y * J[c].y));
         }
     }
-    if (!lane0 || !active || !(Ss > 0.f)) return;
+    __syncwarp();
+    // inner products: Ss = <s,s>, P = <s,x>, G_j = <s,J_j>, H_jk =
+    // Re<J_j,J_k>, Q_j = <J_j,x>, over the group's lanes
+    auto total = [&](int k) {
+        float t = 0.f;
+        for (int q = 0; q < L; q++) t += sA[k * 32 + g * L + q];
+        return t;
+    };
+    if (!lane0 || !active) return;
+    const float Ss = total(0);
+    const float2 P = make_float2(total(1), total(2));
+    float2 G[NT > 0 ? NT : 1], Q[NT > 0 ? NT : 1];
+    float H[NT > 0 ? NT : 1][NT > 0 ? NT : 1];
+    {
+        int n = 3;
+#pragma unroll
+        for (int j = 0; j < NT; j++) {
+            G[j] = make_float2(total(n), total(n + 1));
+            Q[j] = make_float2(total(n + 2), total(n + 3));
+            n += 4;
+        }
+#pragma unroll
+        for (int j = 0; j < NT; j++)
+#pragma unroll
+            for (int c = j; c < NT; c++) H[j][c] = total(n++);
+    }
+    if (!(Ss > 0.f)) return;
     float *mp = a.maps + v * a.nmaps;
     auto finish = [&](float2 p, float ss) {
         const float ip = sqrtf(p.x * p.x + p.y * p.y);
@@ -449,8 +549,8 @@ __global__ void __launch_bounds__(kThreads) gn_ssfp_kernel(Args a) {
     }
 }
 
-// lanes per voxel and states per lane: the fewest padded states for w, then
-// the most states per lane (S in {2, 4})
+// lanes per atom and states per lane of the adjoint: the fewest padded states
+// for w, then the most states per lane (S in {2, 4})
 static void choose_ls(int w, int *L, int *S) {
     int bl = 32, bs = 4, best = 1 << 30;
     for (int s = 4; s >= 2; s -= 2) {
@@ -467,6 +567,35 @@ static void choose_ls(int w, int *L, int *S) {
     *S = bs;
 }
 
+// Lanes per voxel and states per lane (2 to 5) of the refinement: the layout
+// that fills the warp's lanes with the most useful states, (32 / L) w / (32 S)
+// (w = 50: 10 x 5, 3 voxels per warp, 94 %; 16 x 4, 78 %), unless that leaves
+// schedulers without a warp: then two states per lane (a step is a chain that
+// more lanes shorten).
+static void choose_gn(int w, size_t nvox, int sms, int *L, int *S) {
+    double best = 0;
+    for (int s = 2; s <= 5; s++) {
+        const int l = (w + s - 1) / s;
+        if (l > 32) continue;
+        const double useful = (double)(32 / l) * w / (32.0 * s);
+        if (useful > best + 1e-9) {
+            best = useful;
+            *L = l;
+            *S = s;
+        }
+    }
+    if (w <= 64 && nvox / (32 / *L) < (size_t)sms * 4) {
+        *S = 2;
+        *L = (w + 1) / 2;
+    }
+}
+
+static size_t gn_smem(int L, int NT) {
+    const size_t apc = kThreads / L;
+    return apc * kStepChunk * (sizeof(Step) + (NT + 1) * sizeof(float2)) + gn_sums(NT) * 32 * sizeof(float) +
+           (kStepChunk + 1) * sizeof(float2) + (apc * 6 + 1) * sizeof(float) + 8 + apc * sizeof(long long);
+}
+
 template <int S, int NT>
 static cudaError_t launch(const Args &a, dim3 grid, size_t smem, cudaStream_t st) {
     auto k = gn_ssfp_kernel<S, NT>;
@@ -477,11 +606,18 @@ static cudaError_t launch(const Args &a, dim3 grid, size_t smem, cudaStream_t st
     return cudaGetLastError();
 }
 
-static cudaError_t dispatch(int S, int NT, const Args &a, dim3 grid, size_t smem, cudaStream_t st) {
-    if (S == 2) return NT == 4 ? launch<2, 4>(a, grid, smem, st) : NT == 3 ? launch<2, 3>(a, grid, smem, st)
-                                                                       : launch<2, 0>(a, grid, smem, st);
-    return NT == 4 ? launch<4, 4>(a, grid, smem, st) : NT == 3 ? launch<4, 3>(a, grid, smem, st)
-                                                               : launch<4, 0>(a, grid, smem, st);
+template <int S>
+static cudaError_t dispatch_nt(int NT, const Args &a, dim3 grid, size_t smem, cudaStream_t st) {
+    return NT == 4 ? launch<S, 4>(a, grid, smem, st) : NT == 3 ? launch<S, 3>(a, grid, smem, st)
+                                                               : launch<S, 0>(a, grid, smem, st);
+}
+
+static cudaError_t dispatch(int S, int NT, const Args &a, dim3 grid, cudaStream_t st) {
+    const size_t smem = gn_smem(a.L, NT);
+    return S == 2   ? dispatch_nt<2>(NT, a, grid, smem, st)
+           : S == 3 ? dispatch_nt<3>(NT, a, grid, smem, st)
+           : S == 4 ? dispatch_nt<4>(NT, a, grid, smem, st)
+                    : dispatch_nt<5>(NT, a, grid, smem, st);
 }
 
 }  // namespace ssfpgrad
@@ -522,8 +658,10 @@ int refine_gn_ssfp(float *d_maps, int nmaps, const float *img, size_t img_stride
     a.TI = 40.f;
     a.nvox = (long long)nvoxels;
     a.w = nstates;
-    int L, S;
-    choose_ls(nstates, &L, &S);
+    int L = 32, S = 5, dev = 0, sms = 0;
+    SNAPMRF_CUDA(cudaGetDevice(&dev));
+    SNAPMRF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    choose_gn(nstates, nvoxels, sms, &L, &S);
     a.L = L;
     a.img = reinterpret_cast<const float2 *>(img);
     a.img_stride = (long long)img_stride;
@@ -546,7 +684,6 @@ int refine_gn_ssfp(float *d_maps, int nmaps, const float *img, size_t img_stride
         cnt[1] = cnt[0] + 1;
     }
     const int apc = kThreads / L;
-    const size_t smem = (size_t)apc * kStepChunk * sizeof(Step) + (size_t)apc * (6 * sizeof(float) + sizeof(long long));
     dim3 grid((unsigned)((nvoxels + apc - 1) / apc));
     const bool outputs = nmaps >= 5 || d_m0 || (d_b1map && nmaps >= 4);
     for (int it = 0; it < iterations; it++) {
@@ -561,13 +698,13 @@ int refine_gn_ssfp(float *d_maps, int nmaps, const float *img, size_t img_stride
             if (a.count_out) SNAPMRF_CUDA(cudaMemsetAsync(a.count_out, 0, sizeof(int), st));
         }
         a.finish = outputs && (early || last) ? 1 : 0;
-        SNAPMRF_CUDA(dispatch(S, NT, a, grid, smem, st));
+        SNAPMRF_CUDA(dispatch(S, NT, a, grid, st));
     }
     if (outputs && iterations == 0) {
         a.list_in = a.count_in = nullptr;
         a.list_out = a.count_out = nullptr;
         a.finish = 1;
-        SNAPMRF_CUDA(dispatch(S, 0, a, grid, smem, st));
+        SNAPMRF_CUDA(dispatch(S, 0, a, grid, st));
     }
     return SNAPMRF_OK;
 }
