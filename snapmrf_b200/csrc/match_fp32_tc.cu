@@ -23,11 +23,11 @@
 // atoms; 1.2e-5 imaginary, 4e-6 at T = 200 .. 300), where the bound is 2.1e-4
 // (1.0e-4, 3e-5).
 //
-// 57,600 voxels, 284,458 imaginary atoms in 41 blocks, T = 1000: 36.3 -> 4.9
+// 57,600 voxels, 284,458 imaginary atoms in 41 blocks, T = 1000: 36.4 -> 4.9
 // ms (packing 0.68, scores 2.9 = three BF16 products at 1.68 PFLOP/s, about
-// eight candidates per voxel in FP32 0.88, maps 0.11; the FP32 kernel alone
+// eight candidates per voxel in FP32 0.73, maps 0.11; the FP32 kernel alone
 // runs at 0.61 of the FP32 FMA peak); 4,096 voxels, 837 complex atoms: 0.80 ->
-// 0.23 ms.
+// 0.21 ms.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -237,22 +237,29 @@ __global__ void pack_atoms_kernel(__nv_bfloat16 *B, const float2 *atoms, long lo
 // match_fp32_kernel's order, or the voxel goes to the fall list.  One warp per
 // slot; lane c carries candidate c's chain (kBatch of them at a time) through
 // samples that cp.async stages kDepth steps of kSteps ahead.  The chain is
-// serial by definition: 57,600 voxels of about eight candidates 0.88 ms, their
-// rows 3.7 GB from L2 (waiting for each candidate's load in turn: 2.4 ms).
+// serial by definition: 57,600 voxels of about eight candidates 0.73 ms, their
+// rows 3.7 GB from L2 (8-byte copies and reads 0.88, waiting for each
+// candidate's load in turn 2.4 ms).
 constexpr int kRescoreWarps = 4, kMaxCand = 96, kBatch = 16, kSteps = 16, kDepth = 3;
-struct RescoreSmem {
-    float2 d[kDepth][kBatch][kSteps + 1];  // (rows padded: the lanes' reads differ in bank)
+struct alignas(16) RescoreSmem {
+    float2 d[kDepth][kBatch][kSteps + 2];  // (rows padded: the lanes' reads differ in bank)
     float2 x[kDepth][kSteps];
+    float2 xi[kSteps];                     // (Im x, -Re x): what Im s multiplies d by
     int cand[kMaxCand];
 };
 
-__device__ __forceinline__ void copy8(float2 *dst, const float2 *src, bool in) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-                 "l"(src), "r"(in ? 8 : 0)
-                 : "memory");
+// N samples (1 or 2), of which `have` exist; the rest are filled with zeros.
+template <int N>
+__device__ __forceinline__ void copy_samples(float2 *dst, const float2 *src, int have) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if constexpr (N == 2)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(8 * have) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(8 * have) : "memory");
 }
 
-template <bool IMAG>
+// VEC: every row starts 16-byte aligned, so a lane copies two samples at once.
+template <bool IMAG, bool VEC>
 __global__ void __launch_bounds__(kRescoreWarps * 32)
 rescore_kernel(unsigned long long *keys, tc::Lists lists, const int *list_n, const float *list_best,
                const long long *perm, const float *vnorm2, const long long *tile_start, int nbins,
@@ -317,51 +324,69 @@ rescore_kernel(unsigned long long *keys, tc::Lists lists, const int *list_n, con
     }
     const float2 *x = img + v * img_stride;
     const float2 *d0 = atoms + (long long)bin * bin_natoms * atom_stride;
-    const int steps = (nreps + kSteps - 1) / kSteps, sub = lane % kSteps, which = lane / kSteps;
+    // lanes per row and copy, rows per copy instruction
+    constexpr int N = VEC ? 2 : 1, LPR = kSteps / N, RPI = 32 / LPR;
+    const int steps = (nreps + kSteps - 1) / kSteps, sub = lane % LPR * N, which = lane / LPR;
     float bs = 0.f;
     int bi = -1;
     for (int c0 = 0; c0 < count; c0 += kBatch) {
         const int nb = min(kBatch, count - c0);
-        // (two candidates' samples per copy instruction)
-        const float2 *row[kBatch / 2];
+        const float2 *row[kBatch / RPI];
 #pragma unroll
-        for (int q = 0; q < kBatch / 2; q++)
-            row[q] = d0 + (long long)sm.cand[min(c0 + 2 * q + which, count - 1)] * atom_stride + sub;
+        for (int q = 0; q < kBatch / RPI; q++)
+            row[q] = d0 + (long long)sm.cand[min(c0 + RPI * q + which, count - 1)] * atom_stride;
         auto stage = [&](int s) {
             if (s < steps) {
-                const int t0 = s * kSteps, b = s % kDepth;
-                const bool in = t0 + sub < nreps;
-                if (which == 0) copy8(&sm.x[b][sub], in ? x + t0 + sub : x, in);
+                const int t = s * kSteps + sub, b = s % kDepth;
+                const int have = max(0, min(N, nreps - t)), at = have ? t : 0;
+                if (which == 0) copy_samples<N>(&sm.x[b][sub], x + at, have);
 #pragma unroll
-                for (int q = 0; q < kBatch / 2; q++)
-                    if (2 * q < nb) copy8(&sm.d[b][2 * q + which][sub], in ? row[q] + t0 : row[q] - sub, in);
+                for (int q = 0; q < kBatch / RPI; q++)
+                    if (RPI * q < nb) copy_samples<N>(&sm.d[b][RPI * q + which][sub], row[q] + at, have);
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
         for (int s = 0; s < kDepth - 1; s++) stage(s);
-        float ar = 0.f, ai = 0.f;
+        // IMAG: both sums of candidate c on lane c.  Complex (four FMAs per
+        // sample): Re s on lane c, Im s on lane c + kBatch.
+        static_assert(kBatch == 16 && kSteps == 16, "half a warp each");
+        const bool im = !IMAG && lane >= kBatch;
+        float acc = 0.f, acc2 = 0.f;
         for (int s = 0; s < steps; s++) {
             stage(s + kDepth - 1);
             asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");
             __syncwarp();
-            const float2 *dr = sm.d[s % kDepth][lane % kBatch], *xr = sm.x[s % kDepth];
-            // (samples past nreps are zeros: their products add exact zeros)
+            if (!IMAG) {
+                if (!im) {
+                    const float2 v = sm.x[s % kDepth][lane];
+                    sm.xi[lane] = make_float2(v.y, -v.x);
+                }
+                __syncwarp();
+            }
+            const float4 *dr = reinterpret_cast<const float4 *>(sm.d[s % kDepth][lane % kBatch]);
+            const float4 *xr = reinterpret_cast<const float4 *>(im ? sm.xi : sm.x[s % kDepth]);
+            if ((IMAG ? lane : lane % kBatch) < nb) {
+                // (samples past nreps are zeros: their products add exact zeros)
 #pragma unroll
-            for (int u = 0; u < kSteps; u++) {
-                const float2 d = dr[u], xv = xr[u];
-                if (IMAG) {
-                    ar = fmaf(d.y, xv.y, ar);
-                    ai = fmaf(-d.y, xv.x, ai);
-                } else {
-                    ar = fmaf(d.x, xv.x, ar);
-                    ar = fmaf(d.y, xv.y, ar);
-                    ai = fmaf(d.x, xv.y, ai);
-                    ai = fmaf(-d.y, xv.x, ai);
+                for (int u = 0; u < kSteps / 2; u++) {
+                    const float4 d = dr[u], v = xr[u];
+                    if (IMAG) {
+                        acc = fmaf(d.y, v.y, acc);
+                        acc2 = fmaf(-d.y, v.x, acc2);
+                        acc = fmaf(d.w, v.w, acc);
+                        acc2 = fmaf(-d.w, v.z, acc2);
+                    } else {
+                        acc = fmaf(d.x, v.x, acc);
+                        acc = fmaf(d.y, v.y, acc);
+                        acc = fmaf(d.z, v.z, acc);
+                        acc = fmaf(d.w, v.w, acc);
+                    }
                 }
             }
             __syncwarp();
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
+        const float ar = acc, ai = IMAG ? acc2 : __shfl_down_sync(0xffffffffu, acc, kBatch);
         const float sc = ar * ar + ai * ai;
         if (lane < nb && sc > 0.f && beats(sc, sm.cand[c0 + lane], bs, bi)) {
             bs = sc;
@@ -552,7 +577,8 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
         lists.plan = a.plan;
         lists.cap = cap;
         lists.vt = vt;
-        auto rk = q.imag ? rescore_kernel<true> : rescore_kernel<false>;
+        auto rk = q.imag ? (avec && ivec ? rescore_kernel<true, true> : rescore_kernel<true, false>)
+                         : (avec && ivec ? rescore_kernel<false, true> : rescore_kernel<false, false>);
         rk<<<nblk(cap, kRescoreWarps), kRescoreWarps * 32, 0, st>>>(
             keys, lists, a.list_n, a.list_best, perm, vnorm2, tile_start, nbins, b1 ? vox_bin : nullptr, q.atoms,
             q.atom_stride, img, q.img_stride, (int)q.nreps, bin_natoms, margin_rel, state, fall, fall_counts);
