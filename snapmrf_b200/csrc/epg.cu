@@ -227,7 +227,7 @@ static void plan_fine_tail(const EpgArgs &a, int P, long long nblocks, const voi
     const long long n = a.natoms, B = nblocks;
     *bulk_cpb = (n + apc - 1) / apc;
     *fine_cpb = 0;
-    if (P <= kFineP || a.nstates > 2 * kFineP * kFineL || kRealThreads % 32 || getenv("SNAPMRF_DICT_LAYOUT"))
+    if (P <= kFineP || a.nstates > 2 * kFineP * kFineL || getenv("SNAPMRF_DICT_LAYOUT"))
         return;
     long long bulk;
     if (const char *e = getenv("SNAPMRF_DICT_FINE_ATOMS")) {
@@ -257,7 +257,7 @@ static void plan_fine_tail(const EpgArgs &a, int P, long long nblocks, const voi
 
 template <int ECHO, int S, bool TAIL, bool FOLD>
 static cudaError_t launch_epg_real(EpgArgs a, dim3 grid, cudaStream_t st) {
-    size_t smem = epg_real_smem_bytes(a.L);
+    size_t smem = epg_real_smem_bytes(a.L, FOLD);
     auto k = epg_real_kernel<ECHO, S, TAIL, FOLD>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -273,7 +273,7 @@ static cudaError_t launch_epg_real(EpgArgs a, dim3 grid, cudaStream_t st) {
     // epg_real_fine_kernel)
     a.fine_first = bulk_cpb * (kRealThreads / a.L);
     auto kf = epg_real_fine_kernel<ECHO, FOLD>;
-    const size_t smem_f = epg_real_smem_bytes(kFineL);
+    const size_t smem_f = epg_real_smem_bytes(kFineL, FOLD);
     if ((e = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_f)) != cudaSuccess)
         return e;
     cudaLaunchConfig_t cfg = {};

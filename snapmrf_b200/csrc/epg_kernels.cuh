@@ -373,8 +373,8 @@ __device__ __forceinline__ void rf_real_coeffs2(float alpha, float phi, float2 *
     c[9] = make_float2(0.f, 0.f);
 }
 
-// P pairs of EPG states per lane: slot j = 2i + h of pair i is state
-// k = gl * 2P + j.  Packed two-wide FP32 instructions (__ffma2_rn /
+// P pairs of EPG states per lane: element h of pair i is state
+// k = gl * 2P + h P + i.  Packed two-wide FP32 instructions (__ffma2_rn /
 // __fmul2_rn) perform per element exactly the scalar operations of the
 // complex recursion with its zero terms removed.
 template <int P>
@@ -408,23 +408,25 @@ __device__ __forceinline__ void rl2_rf_k(RealLane2<P> &s, float2 c0, float2 c1, 
 // relaxation keeps them): F-' = (c0 + c1)(F+ + F-) - F+' and
 // Z' = c6 (F+ - F-) + c8 Z, 8 packed operations per pair instead of 9.  It
 // rounds differently from the reference's order (unit-norm C1 atoms move by
-// at most 6e-8) and is used by the folded recursion only.
+// at most 6e-8) and is used by the folded recursion only, whose s.fm holds
+// -F-: no operand of a packed instruction is then negated (a negation is an
+// instruction per element), and no value changes but for the sign of zeros.
 template <int P>
-__device__ __forceinline__ void rl2_rf_k8(RealLane2<P> &s, float2 c0, float2 c1, float2 c2, float2 c6, float2 c8) {
-    const float2 cs = __fadd2_rn(c0, c1);
+__device__ __forceinline__ void rl2_rf_k8(RealLane2<P> &s, float2 c0, float2 nc1, float2 c2, float2 c6, float2 c8) {
+    const float2 minus = make_float2(-1.f, -1.f);
+    const float2 cs = __ffma2_rn(nc1, minus, c0), ncs = __ffma2_rn(c0, minus, nc1);
 #pragma unroll
     for (int i = 0; i < P; i++) {
-        const float2 p = s.fp[i], m = s.fm[i], z = s.zz[i];
+        const float2 p = s.fp[i], n = s.fm[i], z = s.zz[i];
         float2 np = __fmul2_rn(c0, p);
-        np = __ffma2_rn(c1, m, np);
+        np = __ffma2_rn(nc1, n, np);
         np = __ffma2_rn(c2, z, np);
-        const float2 d = __fadd2_rn(p, make_float2(-m.x, -m.y));
-        float2 nz = __fmul2_rn(c6, d);
+        float2 nz = __fmul2_rn(c6, __fadd2_rn(p, n));
         nz = __ffma2_rn(c8, z, nz);
-        float2 nm = __ffma2_rn(cs, m, make_float2(-np.x, -np.y));
-        nm = __ffma2_rn(cs, p, nm);
+        float2 nn = __ffma2_rn(cs, n, np);
+        nn = __ffma2_rn(ncs, p, nn);
         s.fp[i] = np;
-        s.fm[i] = nm;
+        s.fm[i] = nn;
         s.zz[i] = nz;
     }
 }
@@ -449,72 +451,79 @@ __device__ __forceinline__ void rl2_relax(RealLane2<P> &s, float E1, float E2, b
 
 // Gradient shift of the paired real state (see st_shift): F+ up one slot,
 // F- down one slot, f+[0] = -f-[0] (Im of conj), F-[w-1] = 0, slots k >= w
-// zero; with w = 1 the unshifted f-[0] is used.
+// zero; with w = 1 the unshifted f-[0] is used.  A pair holds states P apart,
+// so a pair moves as a whole: only the pair that takes the neighbour's state
+// is put together anew.
 //
 // TAIL: the layout pads at most two slots (w >= 2P L - 2).  Slots k >= w
 // then hold zeros before the shift, so F-[w-1] takes the zero of F-[w] and
-// only F+[w], which receives F+[w-1], must be cleared.  That slot lies in the
-// last pair of the last lane, and tail_keep (0 there, 1 elsewhere) clears it
-// with one multiply instead of a compare per slot; every non-zero value is
-// the same as with the per-slot masks.
-template <int P, bool TAIL = false>
-__device__ __forceinline__ void rl2_shift(RealLane2<P> &s, int gl, int L, int w, float2 tail_keep = {1.f, 1.f}) {
+// only F+[w], which receives F+[w-1], must be cleared.  That slot is the
+// second of the last lane's last pair (or of the one before it), and
+// tail_keep (0 there, 1 elsewhere; .x the pair before the last, .y the last)
+// clears it with a multiply instead of a compare per slot; every non-zero
+// value is the same as with the per-slot masks.
+// NEG: s.fm holds -F-.
+template <int P, bool TAIL, bool NEG>
+__device__ __forceinline__ void rl2_shift(RealLane2<P> &s, int gl, int L, int w, float2 tail_keep) {
     const unsigned full = 0xffffffffu;
     const float up = __shfl_up_sync(full, s.fp[P - 1].y, 1, L);
     const float dn = __shfl_down_sync(full, s.fm[0].x, 1, L);
-    const float old_fm0 = s.fm[0].x;
+    const float old_fm0 = s.fm[0].x, mid_p = s.fp[P - 1].x, mid_m = s.fm[0].y;
 #pragma unroll
-    for (int i = P - 1; i >= 1; i--) s.fp[i] = make_float2(s.fp[i - 1].y, s.fp[i].x);
-    s.fp[0] = make_float2(up, s.fp[0].x);
+    for (int i = P - 1; i >= 1; i--) s.fp[i] = s.fp[i - 1];
+    s.fp[0] = make_float2(up, mid_p);
 #pragma unroll
-    for (int i = 0; i < P - 1; i++) s.fm[i] = make_float2(s.fm[i].y, s.fm[i + 1].x);
-    s.fm[P - 1] = make_float2(s.fm[P - 1].y, (gl == L - 1) ? 0.f : dn);
-    if (gl == 0) s.fp[0].x = -((w == 1) ? old_fm0 : s.fm[0].x);
+    for (int i = 0; i < P - 1; i++) s.fm[i] = s.fm[i + 1];
+    s.fm[P - 1] = make_float2(mid_m, (gl == L - 1) ? 0.f : dn);
+    if (gl == 0) {
+        const float f0 = w == 1 ? old_fm0 : s.fm[0].x;
+        s.fp[0].x = NEG ? f0 : -f0;
+    }
     if (TAIL) {
-        s.fp[P - 1] = __fmul2_rn(s.fp[P - 1], tail_keep);
+        s.fp[P - 1].y *= tail_keep.y;
+        if (P > 1)
+            s.fp[P - 2].y *= tail_keep.x;
+        else
+            s.fp[0].x *= tail_keep.x;
         return;
     }
     const int k0 = gl * 2 * P;
 #pragma unroll
     for (int i = 0; i < P; i++) {
-        if (k0 + 2 * i >= w) s.fp[i].x = 0.f;
-        if (k0 + 2 * i + 1 >= w) s.fp[i].y = 0.f;
-        if (k0 + 2 * i == w - 1) s.fm[i].x = 0.f;
-        if (k0 + 2 * i + 1 == w - 1) s.fm[i].y = 0.f;
+        if (k0 + i >= w) s.fp[i].x = 0.f;
+        if (k0 + P + i >= w) s.fp[i].y = 0.f;
+        if (k0 + i == w - 1) s.fm[i].x = 0.f;
+        if (k0 + P + i == w - 1) s.fm[i].y = 0.f;
     }
 }
 
-// The real-valued kernel stages 32 steps per chunk (half the barriers of 16;
-// its per-step shared data is small).
+// The real-valued kernel: one warp per CTA, so that no CTA barrier makes the
+// warps of a CTA wait for each other at every chunk (C1: 7.82 ms with 128
+// threads, 7.79 with 64, 7.63 with 32; the atoms are bit-identical).  It
+// stages 32 steps per chunk, one per lane.
+constexpr int kRealThreads = 32;
 constexpr int kRealChunk = 32;
-// Threads per CTA of the real-valued kernel: one warp, so that no CTA
-// barrier makes the warps of a CTA wait for each other at every chunk (C1:
-// 7.82 ms with 128 threads, 7.79 with 64, 7.63 with 32; the atoms are
-// bit-identical).
-// SNAPMRF_EPG_REAL_THREADS overrides it for tuning (a multiple of 32).
-#ifndef SNAPMRF_EPG_REAL_THREADS
-#define SNAPMRF_EPG_REAL_THREADS 32
-#endif
-constexpr int kRealThreads = SNAPMRF_EPG_REAL_THREADS;
-static_assert(kRealThreads % 32 == 0, "whole warps");
-constexpr int kRealFS = kRealChunk * 4 + 4;          // floats per atom of relaxation factors
-constexpr int kRealReadoutStride = kRealChunk + 1;  // float2 per group
+// Steps unrolled: the shift only renames registers, and the moves that a
+// loop's end needs come once per four steps (C1's dictionary, 284,458 atoms,
+// T = 1000, w = 50 as 2 lanes x 13 pairs: 6.12 ms with 1, 5.55 with 2, 5.41
+// with 4, 5.36 with 8; 6.60 with pairs of neighbouring states, which every
+// shift puts together anew, and 16-byte pieces of rows written per lane).
+// 166 instead of 224 instructions per warp and step, 104 of them the packed
+// operations: those keep the FP32 pipe 73 % busy, the rest is latency at two
+// to three warps per scheduler (the states take the registers; limits of 128
+// and 144 registers spill and take 6.2-6.5 ms).
+constexpr int kRealUnroll = 4;
+// Resident CTAs per SM asked of the compiler (168 registers at 12).
+constexpr int real_min_ctas(int P) { return P <= 13 ? 12 : 1; }
+constexpr int kRealFS = kRealChunk * 4 + 4;        // floats per atom of relaxation factors
+constexpr int kRealReadoutStride = kRealChunk + 1;  // floats per atom
+__host__ __device__ constexpr int epg_real_nc(bool fold) { return fold ? 6 : 10; }  // RF coefficient pairs per step
 
-inline size_t epg_real_smem_bytes(int L) {
+inline size_t epg_real_smem_bytes(int L, bool fold) {
     int apc = kRealThreads / L;
-    return (size_t)kRealChunk * 10 * sizeof(float2) + (size_t)apc * kRealFS * sizeof(float) +
-           (size_t)apc * kRealReadoutStride * sizeof(float2) + (size_t)apc * 4 * sizeof(float);
+    return (size_t)kRealChunk * epg_real_nc(fold) * sizeof(float2) + (size_t)apc * kRealFS * sizeof(float) +
+           (size_t)apc * kRealReadoutStride * sizeof(float) + (size_t)apc * 4 * sizeof(float);
 }
-
-// (An explicit minimum of 1 block per SM lets ptxas use more registers and
-// costs a resident block per SM; SNAPMRF_EPG_REAL_MIN_BLOCKS is for tuning.)
-#ifdef SNAPMRF_EPG_REAL_MIN_BLOCKS
-#define SNAPMRF_EPG_REAL_BOUNDS __launch_bounds__(kRealThreads, SNAPMRF_EPG_REAL_MIN_BLOCKS)
-#elif defined(SNAPMRF_EPG_REAL_MAXNREG)
-#define SNAPMRF_EPG_REAL_BOUNDS __maxnreg__(SNAPMRF_EPG_REAL_MAXNREG)
-#else
-#define SNAPMRF_EPG_REAL_BOUNDS __launch_bounds__(kRealThreads)
-#endif
 
 // One element of the optional 16-bit copy of Im(atom) (the tensor-core
 // matching operand, one row per atom).
@@ -552,30 +561,31 @@ __device__ __forceinline__ void epg_real_cta(const EpgArgs &a, const int L, cons
     const bool active = ab < a.natoms;
     const long long gatom = blk * a.natoms + ab;
 
-    float2 *sC = reinterpret_cast<float2 *>(smem_raw);        // [kRealChunk][10]
-    float *sF = reinterpret_cast<float *>(sC + kRealChunk * 10);   // [apc][FS]
-    float2 *sR = reinterpret_cast<float2 *>(sF + apc * FS);    // [apc][kRealReadoutStride]
-    float *sP = reinterpret_cast<float *>(sR + apc * kRealReadoutStride);
+    constexpr int NC = epg_real_nc(FOLD);
+    float2 *sC = reinterpret_cast<float2 *>(smem_raw);           // [kRealChunk][NC]
+    float *sF = reinterpret_cast<float *>(sC + kRealChunk * NC);  // [apc][FS]
+    float *sR = sF + apc * FS;                                   // [apc][kRealReadoutStride]
+    float *sP = sR + apc * kRealReadoutStride;                   // [apc][4]
 
-    for (int i = tid; i < apc; i += kRealThreads) {
-        long long at = atom0 + i;
+    if (tid < apc) {
+        const long long at = atom0 + tid;
         float t1 = 1.f, t2 = 1.f;
         if (at < a.natoms) {
             const float *p = a.params + (blk * a.natoms + at) * a.nparams;
             t1 = p[0];
             t2 = p[1];
         }
-        sP[4 * i] = t1;
-        sP[4 * i + 1] = t2;
-        sP[4 * i + 2] = 1.f / t1;
-        sP[4 * i + 3] = 1.f / t2;
+        sP[4 * tid] = t1;
+        sP[4 * tid + 1] = t2;
+        sP[4 * tid + 2] = 1.f / t1;
+        sP[4 * tid + 3] = 1.f / t2;
     }
 
     const float *alpha = a.alpha + blk * nreps;
     const float *phi = a.sched + nreps;
     const float *TR = a.sched + 2 * nreps;
     const float *TE = a.sched + 3 * nreps;
-    __syncthreads();
+    __syncwarp();
     const int w = a.nstates;
     // TAIL layouts: 0 at slot w (cleared after each shift), 1 elsewhere
     float2 tail_keep = make_float2(1.f, 1.f);
@@ -600,107 +610,125 @@ __device__ __forceinline__ void epg_real_cta(const EpgArgs &a, const int L, cons
     }
 
     float nrm = 0.f;
-    float2 *out = a.atoms + gatom * nreps;
-    float *outi = reinterpret_cast<float *>(a.atoms) + gatom * nreps;  // (imaginary rows)
+    const long long row0 = blk * a.natoms + atom0;  // the CTA's first atom
+    const int rows = (int)min((long long)apc, a.natoms - atom0);
+    float *const atoms_i = reinterpret_cast<float *>(a.atoms);  // (imaginary rows)
     for (long long t0 = 0; t0 < nreps; t0 += kRealChunk) {
         const int nch = (int)min((long long)kRealChunk, nreps - t0);
-        __syncthreads();
-        for (int i = tid; i < nch; i += kRealThreads) rf_real_coeffs2(alpha[t0 + i], phi[t0 + i], sC + 10 * i);
-        for (int idx = tid; idx < apc * nch; idx += kRealThreads) {
-            int ga = idx / nch, i = idx - ga * nch;
-            float t1 = sP[4 * ga], t2 = sP[4 * ga + 1];
-            float4 f;
+        __syncwarp();
+        // lane i stages step t0 + i of every atom
+        if (tid < nch) {
+            const long long t = t0 + tid;
+            float2 cf[10];
+            rf_real_coeffs2(alpha[t], phi[t], cf);
             if (FOLD) {
-                // (E1, E2) over the previous step's TR (1 before the first
-                // step), E2 over this step's TE, and Z0's recovery 1 - E1;
-                // rates as reciprocals (|t / T| < 1, so the argument's
-                // rounding moves exp by far less than an ulp)
-                const long long t = t0 + i;
-                const float trp = t > 0 ? TR[t - 1] : 0.f;
-                const float r1 = sP[4 * ga + 2], r2 = sP[4 * ga + 3];
-                const float e1 = t > 0 ? expf(-trp * r1) : 1.f, e2 = t > 0 ? expf(-trp * r2) : 1.f;
-                f = make_float4(e1, e2, expf(-TE[t] * r2), 1.f - e1);
+                float4 *c = reinterpret_cast<float4 *>(sC + NC * tid);
+                c[0] = make_float4(cf[0].x, cf[0].y, -cf[1].x, -cf[1].y);
+                c[1] = make_float4(cf[2].x, cf[2].y, cf[6].x, cf[6].y);
+                c[2] = make_float4(cf[8].x, cf[8].y, 0.f, 0.f);
             } else {
-                float tr = TR[t0 + i], te = TE[t0 + i];
-                float ta = te, tb = tr - te;
-                f = make_float4(expf(-ta / t1), expf(-ta / t2), expf(-tb / t1), expf(-tb / t2));
+#pragma unroll
+                for (int q = 0; q < NC; q++) sC[NC * tid + q] = cf[q];
             }
-            *reinterpret_cast<float4 *>(sF + ga * FS + i * NF) = f;
+            const float tr = TR[t], te = TE[t], tb = tr - te;
+            const float trp = t > 0 ? TR[t - 1] : 0.f;
+            for (int ga = 0; ga < apc; ga++) {
+                const float4 tp = *reinterpret_cast<const float4 *>(sP + 4 * ga);
+                float4 f;
+                if (FOLD) {
+                    // (E1, E2) over the previous step's TR (1 before the first
+                    // step), E2 over this step's TE, and Z0's recovery 1 - E1;
+                    // rates as reciprocals (|t / T| < 1, so the argument's
+                    // rounding moves exp by far less than an ulp)
+                    const float e1 = t > 0 ? expf(-trp * tp.z) : 1.f, e2 = t > 0 ? expf(-trp * tp.w) : 1.f;
+                    f = make_float4(e1, e2, expf(-te * tp.w), 1.f - e1);
+                } else {
+                    f = make_float4(expf(-te / tp.x), expf(-te / tp.y), expf(-tb / tp.x), expf(-tb / tp.y));
+                }
+                *reinterpret_cast<float4 *>(sF + ga * FS + tid * NF) = f;
+            }
         }
-        __syncthreads();
+        __syncwarp();
+#pragma unroll kRealUnroll
         for (int i = 0; i < nch; i++) {
             const float4 f = *reinterpret_cast<const float4 *>(sF + g * FS + i * NF);
             if (FOLD) {
-                const float2 *c = sC + 10 * i;
+                const float4 *c = reinterpret_cast<const float4 *>(sC + NC * i);
+                const float4 c01 = c[0], c26 = c[1];
+                const float2 c8 = *reinterpret_cast<const float2 *>(c + 2);
                 const float2 e1 = make_float2(f.x, f.x), e2 = make_float2(f.y, f.y);
-                rl2_rf_k8<P>(s, __fmul2_rn(c[0], e2), __fmul2_rn(c[1], e2), __fmul2_rn(c[2], e1),
-                             __fmul2_rn(c[6], e2), __fmul2_rn(c[8], e1));
+                rl2_rf_k8<P>(s, __fmul2_rn(make_float2(c01.x, c01.y), e2), __fmul2_rn(make_float2(c01.z, c01.w), e2),
+                             __fmul2_rn(make_float2(c26.x, c26.y), e1), __fmul2_rn(make_float2(c26.z, c26.w), e2),
+                             __fmul2_rn(c8, e1));
                 if (lane0) {
                     // the recovery term (1 - E1) of Z0 through the RF's Z column
-                    s.fp[0].x = fmaf(c[2].x, f.w, s.fp[0].x);
-                    s.fm[0].x = fmaf(c[5].x, f.w, s.fm[0].x);
-                    s.zz[0].x = fmaf(c[8].x, f.w, s.zz[0].x);
+                    s.fp[0].x = fmaf(c26.x, f.w, s.fp[0].x);
+                    s.fm[0].x = fmaf(c26.x, f.w, s.fm[0].x);
+                    s.zz[0].x = fmaf(c8.x, f.w, s.zz[0].x);
                     const float v = f.z * s.fp[0].x;
-                    sR[g * kRealReadoutStride + i] = make_float2(0.f, v);
+                    sR[g * kRealReadoutStride + i] = v;
                     nrm = fmaf(v, v, nrm);
                 }
-                if (ECHO == ECHO_FISP) rl2_shift<P, TAIL>(s, gl, L, w, tail_keep);
+                if (ECHO == ECHO_FISP) rl2_shift<P, TAIL, FOLD>(s, gl, L, w, tail_keep);
             } else {
-                rl2_rf<P>(s, sC + 10 * i);
+                rl2_rf<P>(s, sC + NC * i);
                 rl2_relax<P>(s, f.x, f.y, lane0);
                 if (lane0) {
                     const float v = s.fp[0].x;
-                    sR[g * kRealReadoutStride + i] = make_float2(0.f, v);
+                    sR[g * kRealReadoutStride + i] = v;
                     // the complex path adds round(0*0 + v*v) = round(v*v)
                     nrm = __fadd_rn(nrm, __fmul_rn(v, v));
                 }
-                if (ECHO == ECHO_FISP) rl2_shift<P, TAIL>(s, gl, L, w, tail_keep);
+                if (ECHO == ECHO_FISP) rl2_shift<P, TAIL, FOLD>(s, gl, L, w, tail_keep);
                 rl2_relax<P>(s, f.z, f.w, lane0);
             }
         }
         __syncwarp();
-        if (active)
-            for (int q = gl; q < nch; q += L) {
-                const float2 o = sR[g * kRealReadoutStride + q];
+        // lane i writes sample t0 + i of every atom: 32 samples of a row at once
+        if (tid < nch)
+            for (int r = 0; r < rows; r++) {
+                const long long at = row0 + r, q = t0 + tid;
+                const float v = sR[r * kRealReadoutStride + tid];
                 if (a.imag_rows)
-                    outi[t0 + q] = o.y;
+                    atoms_i[at * nreps + q] = v;
                 else
-                    out[t0 + q] = o;
-                if (a.packed && !a.normalize && !a.pack_normalized) store_packed(a, gatom, t0 + q, o.y);
+                    a.atoms[at * nreps + q] = make_float2(0.f, v);
+                if (a.packed && !a.normalize && !a.pack_normalized) store_packed(a, at, q, v);
             }
     }
-    if (a.normalize || a.norms || a.pack_normalized) {
-        nrm = __shfl_sync(0xffffffffu, nrm, 0, L);
-        if (a.norms && lane0 && active) a.norms[gatom] = sqrtf(nrm);
-        if (a.normalize || (a.pack_normalized && !a.operand_pass)) {
-            __syncwarp();
-            float inv = nrm;
+    if (a.norms && lane0 && active) a.norms[gatom] = sqrtf(nrm);
+    if (a.normalize || (a.pack_normalized && !a.operand_pass)) {
+        for (int r = 0; r < rows; r++) {
+            const long long at = row0 + r;
+            float inv = __shfl_sync(0xffffffffu, nrm, r * L);
             if (inv > 0.f) inv = 1.f / sqrtf(inv);
-            if (active) {
-                if (a.normalize && a.imag_rows) {
-                    // (the same product as the complex row's imaginary part)
-                    for (long long q = gl; q < nreps; q += L) {
-                        const float o = outi[q] * inv;
-                        outi[q] = o;
-                        if (a.packed) store_packed(a, gatom, q, o);
-                    }
-                } else if (a.normalize) {
-                    for (long long q = gl; q < nreps; q += L) {
-                        const float2 o = c_scale(out[q], inv);
-                        out[q] = o;
-                        if (a.packed) store_packed(a, gatom, q, o.y);
-                    }
-                } else {
-                    // the operand of the unit-norm atom (the same product
-                    // as above); the atom itself is not rewritten
-                    for (long long q = gl; q < nreps; q += L)
-                        store_packed(a, gatom, q, a.imag_rows ? outi[q] * inv : c_scale(out[q], inv).y);
+            float2 *out = a.atoms + at * nreps;
+            float *outi = atoms_i + at * nreps;
+            // (a lane reads the samples that it wrote)
+            if (a.normalize && a.imag_rows) {
+                // (the same product as the complex row's imaginary part)
+                for (long long q = tid; q < nreps; q += 32) {
+                    const float o = outi[q] * inv;
+                    outi[q] = o;
+                    if (a.packed) store_packed(a, at, q, o);
                 }
+            } else if (a.normalize) {
+                for (long long q = tid; q < nreps; q += 32) {
+                    const float2 o = c_scale(out[q], inv);
+                    out[q] = o;
+                    if (a.packed) store_packed(a, at, q, o.y);
+                }
+            } else {
+                // the operand of the unit-norm atom (the same product as
+                // above); the atom itself is not rewritten
+                for (long long q = tid; q < nreps; q += 32)
+                    store_packed(a, at, q, a.imag_rows ? outi[q] * inv : c_scale(out[q], inv).y);
             }
         }
     }
-    if (a.packed && active && !a.operand_pass)
-        for (long long q = nreps + gl; q < a.packed_pitch; q += L) store_packed(a, gatom, q, 0.f);
+    if (a.packed && !a.operand_pass)
+        for (int r = 0; r < rows; r++)
+            for (long long q = nreps + tid; q < a.packed_pitch; q += 32) store_packed(a, row0 + r, q, 0.f);
 }
 
 // Fine layout of the real-valued recursion: kFineP pairs of states per lane
@@ -719,7 +747,7 @@ static_assert(kFineP == 1 || kFineP == 2 || kFineP == 4 || kFineP == 8, "fine la
 // below) may start: that grid then starts when every CTA of this one has
 // started, i.e. during its last round.
 template <int ECHO, int P, bool TAIL, bool FOLD>
-__global__ void SNAPMRF_EPG_REAL_BOUNDS epg_real_kernel(EpgArgs a) {
+__global__ void __launch_bounds__(kRealThreads, real_min_ctas(P)) epg_real_kernel(EpgArgs a) {
     asm volatile("griddepcontrol.launch_dependents;");
     epg_real_cta<ECHO, P, TAIL, FOLD>(a, a.L, blockIdx.y, (long long)blockIdx.x * (kRealThreads / a.L));
 }
