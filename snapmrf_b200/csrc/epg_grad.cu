@@ -303,25 +303,6 @@ __device__ __forceinline__ void p_rf_folded(Pair3<P> &x, const FoldedRF &k) {
     }
 }
 
-// The T1 tangent's RF with its relaxation folded in: the product rule adds
-// dE1 z_signal to Z before the RF, i.e. -S dE1 z_signal to F+' and
-// C dE1 z_signal to Z' (F-' follows from the identity; F+ and F- get no
-// source).  sz: the signal's pre-relaxation Z, read before the signal's RF.
-template <int P>
-__device__ __forceinline__ void p_rf_folded_t1(Pair3<P> &x, const FoldedRF &k, const float2 *sz, float2 nSd,
-                                               float2 Cd) {
-#pragma unroll
-    for (int i = 0; i < P; i++) {
-        const float2 p = x.p[i], m = x.m[i], q = x.z[i];
-        const float2 np =
-            __ffma2_rn(nSd, sz[i], __ffma2_rn(k.nS, q, __ffma2_rn(k.s, m, __fmul2_rn(k.c, p))));
-        const float2 d = __fadd2_rn(p, make_float2(-m.x, -m.y));
-        x.z[i] = __ffma2_rn(Cd, sz[i], __ffma2_rn(k.C, q, __fmul2_rn(k.hS, d)));
-        x.m[i] = __ffma2_rn(k.e2, p, __ffma2_rn(k.e2, m, make_float2(-np.x, -np.y)));
-        x.p[i] = np;
-    }
-}
-
 // Shift of one packed stream.  States k >= w hold zeros: F- needs no mask
 // (F-[w-1] takes the zero of F-[w]), F+ takes F+[w-1] into slot w, which
 // keep[] (0 at slot w, 1 elsewhere) clears.
@@ -349,6 +330,53 @@ __device__ __forceinline__ void p_shift(Pair3<P> &x, int gl, int L, int w, const
     }
 }
 
+// The refinement's streams hold states P apart in a pair (element h of pair i
+// is state k = gl * 2P + h P + i), so that the shift moves whole pairs and
+// only renames registers, and m[] holds -F-, so that no operand of a packed
+// instruction is negated (an instruction per element).
+struct GnRF {
+    float2 c, s, nS, hS, C, e2;  // c E2, -s E2, -S E1, hS E2, C E1, E2
+};
+
+// The folded RF on such a stream: 8 packed operations per pair.
+template <int P>
+__device__ __forceinline__ void gn_rf(Pair3<P> &x, const GnRF &k) {
+    const float2 ne2 = make_float2(-k.e2.x, -k.e2.y);
+#pragma unroll
+    for (int i = 0; i < P; i++) {
+        const float2 p = x.p[i], n = x.m[i], q = x.z[i];
+        const float2 np = __ffma2_rn(k.nS, q, __ffma2_rn(k.s, n, __fmul2_rn(k.c, p)));
+        x.z[i] = __ffma2_rn(k.C, q, __fmul2_rn(k.hS, __fadd2_rn(p, n)));
+        x.m[i] = __ffma2_rn(ne2, p, __ffma2_rn(k.e2, n, np));
+        x.p[i] = np;
+    }
+}
+
+// Its shift (see p_shift).
+template <int P, bool PAD>
+__device__ __forceinline__ void gn_shift(Pair3<P> &x, int gl, int L, int w, int src_up, int src_dn) {
+    const unsigned full = 0xffffffffu;
+    const float up = __shfl_sync(full, x.p[P - 1].y, src_up);
+    const float dn = __shfl_sync(full, x.m[0].x, src_dn);
+    const float old_m0 = x.m[0].x, mid_p = x.p[P - 1].x, mid_m = x.m[0].y;
+#pragma unroll
+    for (int i = P - 1; i >= 1; i--) x.p[i] = x.p[i - 1];
+    x.p[0] = make_float2(up, mid_p);
+#pragma unroll
+    for (int i = 0; i < P - 1; i++) x.m[i] = x.m[i + 1];
+    x.m[P - 1] = make_float2(mid_m, (gl == L - 1) ? 0.f : dn);
+    if (gl == 0) x.p[0].x = w == 1 ? old_m0 : x.m[0].x;
+    // (no slot w without padding: the last lane's F- takes a zero instead)
+    if (PAD) {
+        const int j = w - gl * 2 * P;  // slot w in this lane
+#pragma unroll
+        for (int i = 0; i < P; i++) {
+            if (j == i) x.p[i].x = 0.f;
+            if (j == i + P) x.p[i].y = 0.f;
+        }
+    }
+}
+
 // Per-step constants of one voxel, staged in shared memory per chunk.
 // Relaxation is diagonal in the EPG states with one factor for F+ and F-,
 // so it commutes with the dephasing shift: relax(TE), shift, relax(TR-TE)
@@ -357,12 +385,16 @@ __device__ __forceinline__ void p_shift(Pair3<P> &x, int gl, int L, int w, const
 struct GnStep {
     float C, S;            // cos, sin of alpha_t * B1
     float E1, E2;          // relaxation over TR
-    float dE1, dE2;        // dE1/dT1, dE2/dT2
+    float r1, r2;          // d ln E1 / dT1, d ln E2 / dT2
     float Ea, dEa;         // E2 over TE (readout) and dEa/dT2
     float xr, xi;          // voxel sample
 };
 
 constexpr int kGnChunk = 16;
+// Steps unrolled (the shift renames registers; the loop's end moves them):
+// 57,600 voxels, T = 1000, w = 50: 5.69 ms with 1, 5.42 with 2, 5.38 with 4,
+// but 7 pairs per lane take 7.5, 7.0 and 8.4 ms.
+constexpr int kGnUnroll = 2;
 
 // One Gauss-Newton iteration per voxel (TANGENTS) or, without tangents, the
 // final evaluation of PD and M0 at the current parameters.  L lanes per
@@ -425,13 +457,6 @@ __global__ void __launch_bounds__(kGnThreads, P == 5 ? 12 * 32 / kGnThreads : 1)
     const long long v = sI[g];
     const bool active = !idle && sV[4 * g + 3] != 0.f;
     const int T = a.sch.nreps, w = a.w;
-    const int k0 = gl * 2 * P;
-    constexpr bool padded = PAD;
-    float2 keep[P];
-#pragma unroll
-    for (int i = 0; i < P; i++)
-        keep[i] = make_float2(k0 + 2 * i == w ? 0.f : 1.f, k0 + 2 * i + 1 == w ? 0.f : 1.f);
-
     Pair3<P> sv, s1, s2;
     pz<P>(sv);
     if (TANGENTS) {
@@ -453,13 +478,13 @@ __global__ void __launch_bounds__(kGnThreads, P == 5 ? 12 * 32 / kGnThreads : 1)
             GnStep q;
             __sincosf(a.sch.alpha[t] * B1, &q.S, &q.C);
             // the relaxation folded into this step's RF is the previous
-            // interval's (none before the first pulse: E = 1, dE = 0)
+            // interval's (none before the first pulse: E = 1, its derivative 0)
             const float ta = a.sch.TE[t], tr = t > 0 ? a.sch.TR[t - 1] : 0.f;
             const float r1 = 1.f / T1, r2 = 1.f / T2;
             q.E1 = __expf(-tr * r1);
             q.E2 = __expf(-tr * r2);
-            q.dE1 = q.E1 * tr * r1 * r1;
-            q.dE2 = q.E2 * tr * r2 * r2;
+            q.r1 = tr * r1 * r1;
+            q.r2 = tr * r2 * r2;
             q.Ea = __expf(-ta * r2);
             q.dEa = q.Ea * ta * r2 * r2;
             const long long vv = sI[ga];
@@ -471,13 +496,14 @@ __global__ void __launch_bounds__(kGnThreads, P == 5 ? 12 * 32 / kGnThreads : 1)
         }
         __syncthreads();
         const GnStep *qs = step_row(g);
+#pragma unroll kGnUnroll
         for (int i = 0; i < nch; i++) {
             const GnStep q = qs[i];
             const float cc = (1 + q.C) / 2, ss = (1 - q.C) / 2, hS = 0.5f * q.S;
             // RF coefficients with the previous interval's relaxation folded in
-            FoldedRF k;
+            GnRF k;
             k.c = make_float2(cc * q.E2, cc * q.E2);
-            k.s = make_float2(ss * q.E2, ss * q.E2);
+            k.s = make_float2(-ss * q.E2, -ss * q.E2);
             k.nS = make_float2(-q.S * q.E1, -q.S * q.E1);
             k.hS = make_float2(hS * q.E2, hS * q.E2);
             k.C = make_float2(q.C * q.E1, q.C * q.E1);
@@ -485,38 +511,30 @@ __global__ void __launch_bounds__(kGnThreads, P == 5 ? 12 * 32 / kGnThreads : 1)
             // the signal's recovery 1 - E1 on state 0's Z, through the RF's Z column
             const float rec = 1.f - q.E1;
             if (TANGENTS) {
-                // T2 tangent, relaxed first (product rule on the pre-relaxation
-                // signal: F+- += dE2 f+-), then the same folded RF
-                const float2 de2 = make_float2(q.dE2, q.dE2), e2 = make_float2(q.E2, q.E2);
+                // the product rule on the pre-relaxation state, E2 (dF + r2 F)
+                // and E1 (dZ + r1 Z) with r = d ln E / dT: the source is added
+                // before the RF that carries the factor
+                const float2 r1 = make_float2(q.r1, q.r1), r2 = make_float2(q.r2, q.r2);
 #pragma unroll
                 for (int j = 0; j < P; j++) {
-                    s2.p[j] = __ffma2_rn(de2, sv.p[j], __fmul2_rn(e2, s2.p[j]));
-                    s2.m[j] = __ffma2_rn(de2, sv.m[j], __fmul2_rn(e2, s2.m[j]));
+                    s2.p[j] = __ffma2_rn(r2, sv.p[j], s2.p[j]);
+                    s2.m[j] = __ffma2_rn(r2, sv.m[j], s2.m[j]);
+                    s1.z[j] = __ffma2_rn(r1, sv.z[j], s1.z[j]);
                 }
-                // (its Z relaxes by E1 only, and F+- were relaxed above: the
-                // folded RF with E2 = 1 on F+- and E1 on Z)
-                FoldedRF k2;
-                k2.c = make_float2(cc, cc);
-                k2.s = make_float2(ss, ss);
-                k2.nS = k.nS;
-                k2.hS = make_float2(hS, hS);
-                k2.C = k.C;
-                k2.e2 = make_float2(1.f, 1.f);
-                p_rf_folded<P>(s2, k2);
-                // T1 tangent: the source dE1 z_signal and the recovery's
-                // derivative -dE1 on state 0
-                p_rf_folded_t1<P>(s1, k, sv.z, make_float2(-q.S * q.dE1, -q.S * q.dE1),
-                                  make_float2(q.C * q.dE1, q.C * q.dE1));
+                gn_rf<P>(s2, k);
+                gn_rf<P>(s1, k);
                 if (lane0) {
-                    s1.p[0].x = fmaf(q.S, q.dE1, s1.p[0].x);
-                    s1.m[0].x = fmaf(-q.S, q.dE1, s1.m[0].x);
-                    s1.z[0].x = fmaf(-q.C, q.dE1, s1.z[0].x);
+                    // the recovery's derivative -dE1/dT1 on state 0
+                    const float dE1 = q.E1 * q.r1;
+                    s1.p[0].x = fmaf(q.S, dE1, s1.p[0].x);
+                    s1.m[0].x = fmaf(q.S, dE1, s1.m[0].x);
+                    s1.z[0].x = fmaf(-q.C, dE1, s1.z[0].x);
                 }
             }
-            p_rf_folded<P>(sv, k);
+            gn_rf<P>(sv, k);
             if (lane0) {
                 sv.p[0].x = fmaf(-q.S, rec, sv.p[0].x);
-                sv.m[0].x = fmaf(q.S, rec, sv.m[0].x);
+                sv.m[0].x = fmaf(-q.S, rec, sv.m[0].x);
                 sv.z[0].x = fmaf(q.C, rec, sv.z[0].x);
                 // readout s_t = i Ea f+[0] (relaxation over TE)
                 const float f = q.Ea * sv.p[0].x;
@@ -538,10 +556,10 @@ __global__ void __launch_bounds__(kGnThreads, P == 5 ? 12 * 32 / kGnThreads : 1)
                 }
             }
             if (a.shift) {
-                p_shift<P>(sv, gl, L, w, keep, src_up, src_dn, padded);
+                gn_shift<P, PAD>(sv, gl, L, w, src_up, src_dn);
                 if (TANGENTS) {
-                    p_shift<P>(s1, gl, L, w, keep, src_up, src_dn, padded);
-                    p_shift<P>(s2, gl, L, w, keep, src_up, src_dn, padded);
+                    gn_shift<P, PAD>(s1, gl, L, w, src_up, src_dn);
+                    gn_shift<P, PAD>(s2, gl, L, w, src_up, src_dn);
                 }
             }
             // (the relaxation over this step's TR goes into the next RF)
