@@ -818,6 +818,7 @@ __device__ __forceinline__ void roa_init(float t1, float t2, float &m0, float &m
 __global__ void __launch_bounds__(kEpgThreads) roa_kernel(EpgArgs a) {
     __shared__ RoaStep sT[kChunk];
     __shared__ float2 sR[kEpgThreads][kChunk + 1];
+    __shared__ float sN[kEpgThreads];
     const int tid = threadIdx.x;
     const long long blk = blockIdx.y;
     const long long nreps = a.nreps;
@@ -835,6 +836,7 @@ __global__ void __launch_bounds__(kEpgThreads) roa_kernel(EpgArgs a) {
     const float *alpha = a.alpha + blk * nreps;
     const float *phi = a.sched + nreps;
     const float *TR = a.sched + 2 * nreps;
+    const double rate = M_PI * b0 / 1000.0;  // rad / ms over half a TR
     float m0, m1, m2;
     roa_init(t1, t2, m0, m1, m2, a.init_alpha_deg, a.init_phi_deg, a.init_ti);
     float nrm = 0.f;
@@ -856,9 +858,8 @@ __global__ void __launch_bounds__(kEpgThreads) roa_kernel(EpgArgs a) {
             m0 = E2 * n0;
             m1 = E2 * n1;
             m2 = E1 * n2 + (1 - E1);
-            float beta = (float)(M_PI * b0 * tr / 1000.f);
             float sb, cb;
-            __sincosf(beta, &sb, &cb);
+            __sincosf((float)(rate * tr), &sb, &cb);
             float w1 = m0, w2 = m1;
             m0 = cb * w1 + sb * w2;
             m1 = cb * w2 - sb * w1;
@@ -877,13 +878,15 @@ __global__ void __launch_bounds__(kEpgThreads) roa_kernel(EpgArgs a) {
             for (int q = lane; q < nch; q += 32) o[q] = sR[r][q];
         }
     }
-    __syncthreads();
     if (a.norms && active) a.norms[gatom] = sqrtf(nrm);
-    if (a.normalize && active) {
-        float inv = nrm;
-        if (inv > 0.f) inv = 1.f / sqrtf(inv);
-        float2 *out = a.atoms + gatom * nreps;
-        for (long long q = 0; q < nreps; q++) out[q] = c_scale(out[q], inv);
+    if (a.normalize) {
+        sN[tid] = nrm > 0.f ? 1.f / sqrtf(nrm) : nrm;
+        __syncthreads();
+        for (int r = warp; r < kEpgThreads && atom0 + r < a.natoms; r += kEpgThreads / 32) {
+            const float inv = sN[r];
+            float2 *out = a.atoms + (blk * a.natoms + atom0 + r) * nreps;
+            for (long long q = lane; q < nreps; q += 32) out[q] = c_scale(out[q], inv);
+        }
     }
 }
 
@@ -891,21 +894,39 @@ __global__ void __launch_bounds__(kEpgThreads) roa_kernel(EpgArgs a) {
 // divisor of the warp), IPL isochromats per lane; lane r of a group holds
 // isochromats r*IPL .. r*IPL + IPL - 1 (those past n_iso idle), so that G*IPL
 // close above n_iso wastes few slots (n_iso = 100: 8 x 13 = 104, where 32
-// lanes x 4 carried 128).  Isochromat j precesses by an extra pi*j/n_iso per
-// half TR (2*pi*j/n_iso per TR, so the n_iso isochromats dephase uniformly
-// across 2*pi); the readout is the mean of Mx + iMy over isochromats.  The
-// relaxation over TR is folded into the rotation's rows (E2 into the rows of
-// Mx and My, E1 into Mz's, whose recovery 1 - E1 starts the sum; the row's
-// Mx entry is zero), and the step's relaxation factors and B0 phasor are
-// computed once per atom and step by the group's lanes and staged.
+// lanes x 4 carried 128).  Isochromat j precesses by an extra d_j = pi*j/n_iso
+// per half TR (2*pi*j/n_iso per TR, so the n_iso isochromats dephase uniformly
+// across 2*pi); the readout is the mean of Mx + iMy over isochromats.
+//
+// The RF is a rotation about x and one about z (by 2 phi), and all rotations
+// about z commute, so a step is one matrix common to the atom's isochromats
+// (the flip, relaxation over TR and the z-rotation by 2 phi + 2 beta),
+// followed by the isochromat's rotation by 2 d_j:
+//   n = M u,  u' = R(2 d_j) n,  readout = R(-beta) sum_j R(d_j) n_j / n_iso:
+// 16 operations per isochromat and step (3 + 3 + 2 for n, 4 for the sum, 4 for
+// u'), two-wide on pairs of isochromats, instead of 22 scalar ones that added
+// the angles for each.  The atom's constants are computed by the group's lanes,
+// one step each; the lanes' sums meet in shared memory, once per chunk.  No
+// CTA barrier: a warp's groups depend on nothing outside the warp.
+// 55,504 atoms, T = 500, 100 isochromats: 2.92 -> 1.90 ms, of which the 16
+// operations take 1.28 at the measured FP32 peak with the idle slots (1, 2
+// and 4 steps unrolled 1.91, 1.90, 1.92; a limit of 128 registers spills:
+// 1.96); error against 64 bits 2.7e-6 (22 operations: 2.8e-6).
+struct RoaIsoStep {
+    float4 x;  // Mx row: x, y, z; recovery 1 - E1
+    float4 y;  // My row: x, y, z; Mz row: y
+    float4 z;  // Mz row: z; cos, sin of beta (the readout's way back)
+};
+
 template <int IPL>
 __global__ void __launch_bounds__(kEpgThreads) roa_iso_kernel(EpgArgs a, int G) {
     constexpr int MAXA = kEpgThreads / 8;  // atoms per CTA at G = 8
-    __shared__ RoaStep sT[kChunk];
+    constexpr int NP = IPL / 2;            // pairs; an odd isochromat by itself
+    constexpr bool ODD = IPL % 2 != 0;
     // (rows padded by one entry: the groups of a warp read and write
     // different banks)
-    __shared__ float4 sF[MAXA][kChunk + 1];   // per atom and step: E1, E2, sin, cos of beta
-    __shared__ float2 sOut[MAXA][kChunk + 1];  // the readout
+    __shared__ RoaIsoStep sF[MAXA][kChunk + 1];
+    __shared__ float2 sO[kChunk][kEpgThreads + 1];  // each lane's part of the readout
     const int tid = threadIdx.x;
     const int apc = kEpgThreads / G, ga = tid / G, r = tid % G;
     const long long blk = blockIdx.y;
@@ -920,71 +941,105 @@ __global__ void __launch_bounds__(kEpgThreads) roa_iso_kernel(EpgArgs a, int G) 
         t2 = p[1];
         b0 = p[2];
     }
+    const double rate = M_PI * b0 / 1000.0;  // rad / ms over half a TR
     const float *alpha = a.alpha + blk * nreps;
     const float *phi = a.sched + nreps;
     const float *TR = a.sched + 2 * nreps;
     const int n_iso = a.n_iso;
     float i0, i1, i2;
     roa_init(t1, t2, i0, i1, i2, a.init_alpha_deg, a.init_phi_deg, a.init_ti);
-    // (a slot past n_iso gets a zero rotation: its Mx, My stay 0 after the
-    // first step and its readout adds exactly 0)
-    float m0[IPL], m1[IPL], m2[IPL], cd[IPL], sd[IPL];
+    // (a slot past n_iso gets zero rotations: its Mx, My are 0 from the first
+    // step on and its readout adds exactly 0)
+    float mx[IPL], my[IPL], mz[IPL], cd[IPL], sd[IPL], ce[IPL], se[IPL];
 #pragma unroll
     for (int q = 0; q < IPL; q++) {
         const int j = r * IPL + q;
-        m0[q] = i0;
-        m1[q] = i1;
-        m2[q] = i2;
-        double d = M_PI * (double)j / (double)n_iso;
-        cd[q] = j < n_iso ? (float)cos(d) : 0.f;
-        sd[q] = j < n_iso ? (float)sin(d) : 0.f;
+        mx[q] = i0;
+        my[q] = i1;
+        mz[q] = i2;
+        double s1 = 0, c1 = 0;
+        if (j < n_iso) sincospi((double)j / (double)n_iso, &s1, &c1);
+        cd[q] = (float)c1;
+        sd[q] = (float)s1;
+        ce[q] = (float)(c1 * c1 - s1 * s1);
+        se[q] = (float)(2 * c1 * s1);
     }
     const float inv_n = 1.f / (float)n_iso;
     float nrm = 0.f;
     float2 *out = a.atoms + gatom * nreps;
     for (long long t0 = 0; t0 < nreps; t0 += kChunk) {
         const int nch = (int)min((long long)kChunk, nreps - t0);
-        __syncthreads();
-        for (int i = tid; i < nch; i += kEpgThreads) roa_matrix(alpha[t0 + i], phi[t0 + i], sT[i].T);
-        for (int i = r; i < nch; i += G) {
-            const float tr = TR[t0 + i];
-            float sb, cb;
-            const float beta = (float)(M_PI * b0 * tr / 1000.f);
-            __sincosf(beta, &sb, &cb);
-            sF[ga][i] = make_float4(expf(-tr / t1), expf(-tr / t2), sb, cb);
-        }
-        __syncthreads();
-        for (int i = 0; i < nch; i++) {
-            const float *T = sT[i].T;
-            const float4 f = sF[ga][i];
-            const float E1 = f.x, E2 = f.y, sb = f.z, cb = f.w;
-            const float a0 = E2 * T[0], a3 = E2 * T[3], a6 = E2 * T[6];
-            const float a1 = E2 * T[1], a4 = E2 * T[4], a7 = E2 * T[7];
-            const float c5 = E1 * T[5], c8 = E1 * T[8], rec = 1.f - E1;
-            float px = 0.f, py = 0.f;
-#pragma unroll
-            for (int q = 0; q < IPL; q++) {
-                const float x = fmaf(a6, m2[q], fmaf(a3, m1[q], a0 * m0[q]));
-                const float y = fmaf(a7, m2[q], fmaf(a4, m1[q], a1 * m0[q]));
-                m2[q] = fmaf(c8, m2[q], fmaf(c5, m1[q], rec));
-                // rotation by beta then by the isochromat's delta
-                const float cx = cb * cd[q] - sb * sd[q], sx = sb * cd[q] + cb * sd[q];
-                const float w1 = cx * x + sx * y, w2 = cx * y - sx * x;
-                px += w1;
-                py += w2;
-                m0[q] = cx * w1 + sx * w2;
-                m1[q] = cx * w2 - sx * w1;
-            }
-            // the group's sum (a group never straddles a warp)
-            for (int o = G / 2; o; o >>= 1) {
-                px += __shfl_xor_sync(0xffffffffu, px, o);
-                py += __shfl_xor_sync(0xffffffffu, py, o);
-            }
-            if (r == 0) sOut[ga][i] = make_float2(px * inv_n, py * inv_n);
-        }
         __syncwarp();
         for (int i = r; i < nch; i += G) {
-            const float2 v = sOut[ga][i];
+            const float tr = TR[t0 + i];
+            float sb, cb, sa, ca, sp, cp;
+            __sincosf((float)(rate * tr), &sb, &cb);
+            __sincosf(alpha[t0 + i], &sa, &ca);
+            __sincosf(phi[t0 + i], &sp, &cp);
+            const float s2 = 2 * cp * sp, c2 = cp * cp - sp * sp, sb2 = 2 * cb * sb, cb2 = cb * cb - sb * sb;
+            const float E1 = expf(-tr / t1), E2 = expf(-tr / t2);
+            const float ec = E2 * (c2 * cb2 - s2 * sb2), es = E2 * (s2 * cb2 + c2 * sb2);
+            RoaIsoStep k;
+            k.x = make_float4(ec, es * ca, es * sa, 1.f - E1);
+            k.y = make_float4(-es, ec * ca, ec * sa, -E1 * sa);
+            k.z = make_float4(E1 * ca, cb, sb, 0.f);
+            sF[ga][i] = k;
+        }
+        __syncwarp();
+#pragma unroll 2
+        for (int i = 0; i < nch; i++) {
+            const float4 kx = sF[ga][i].x, ky = sF[ga][i].y;
+            const float zz = sF[ga][i].z.x;
+            const float2 x0 = make_float2(kx.x, kx.x), x1 = make_float2(kx.y, kx.y), x2 = make_float2(kx.z, kx.z);
+            const float2 y0 = make_float2(ky.x, ky.x), y1 = make_float2(ky.y, ky.y), y2 = make_float2(ky.z, ky.z);
+            const float2 z1 = make_float2(ky.w, ky.w), z2 = make_float2(zz, zz), rec = make_float2(kx.w, kx.w);
+            float2 px = make_float2(0.f, 0.f), py = px, qy = px;
+#pragma unroll
+            for (int q = 0; q < NP; q++) {
+                const float2 x = make_float2(mx[2 * q], mx[2 * q + 1]), y = make_float2(my[2 * q], my[2 * q + 1]);
+                const float2 z = make_float2(mz[2 * q], mz[2 * q + 1]);
+                const float2 c = make_float2(cd[2 * q], cd[2 * q + 1]), s = make_float2(sd[2 * q], sd[2 * q + 1]);
+                const float2 C = make_float2(ce[2 * q], ce[2 * q + 1]), S = make_float2(se[2 * q], se[2 * q + 1]);
+                const float2 nx = __ffma2_rn(x2, z, __ffma2_rn(x1, y, __fmul2_rn(x0, x)));
+                const float2 ny = __ffma2_rn(y2, z, __ffma2_rn(y1, y, __fmul2_rn(y0, x)));
+                const float2 nz = __ffma2_rn(z2, z, __ffma2_rn(z1, y, rec));
+                px = __ffma2_rn(s, ny, __ffma2_rn(c, nx, px));
+                py = __ffma2_rn(c, ny, py);
+                qy = __ffma2_rn(s, nx, qy);
+                const float2 ux = __ffma2_rn(S, ny, __fmul2_rn(C, nx));
+                    const float2 uy = __ffma2_rn(make_float2(-S.x, -S.y), nx, __fmul2_rn(C, ny));
+                mx[2 * q] = ux.x;
+                mx[2 * q + 1] = ux.y;
+                my[2 * q] = uy.x;
+                my[2 * q + 1] = uy.y;
+                mz[2 * q] = nz.x;
+                mz[2 * q + 1] = nz.y;
+            }
+            float sx = px.x + px.y, sy = (py.x - qy.x) + (py.y - qy.y);
+            if (ODD) {
+                constexpr int q = IPL - 1;
+                const float x = mx[q], y = my[q], z = mz[q];
+                const float nx = fmaf(kx.z, z, fmaf(kx.y, y, kx.x * x));
+                const float ny = fmaf(ky.z, z, fmaf(ky.y, y, ky.x * x));
+                mz[q] = fmaf(zz, z, fmaf(ky.w, y, kx.w));
+                sx = fmaf(sd[q], ny, fmaf(cd[q], nx, sx));
+                sy = fmaf(-sd[q], nx, fmaf(cd[q], ny, sy));
+                mx[q] = fmaf(se[q], ny, ce[q] * nx);
+                my[q] = fmaf(-se[q], nx, ce[q] * ny);
+            }
+            sO[i][tid] = make_float2(sx, sy);
+        }
+        __syncwarp();
+        // the group's sums (a group never straddles a warp)
+        for (int i = r; i < nch; i += G) {
+            float sx = 0.f, sy = 0.f;
+            for (int q = 0; q < G; q++) {
+                const float2 o = sO[i][tid - r + q];
+                sx += o.x;
+                sy += o.y;
+            }
+            const float4 k = sF[ga][i].z;
+            const float2 v = make_float2((k.y * sx - k.z * sy) * inv_n, (k.y * sy + k.z * sx) * inv_n);
             nrm = fmaf(v.x, v.x, fmaf(v.y, v.y, nrm));
             if (active) out[t0 + i] = v;
         }
