@@ -77,15 +77,15 @@ SNR = 40.0
 FLOP_PER_STATE_STEP = 66
 FLOP_PER_STATE_STEP_EXECUTED = 16
 # Gauss-Newton pass (signal + dT1 + dT2 tangents, packed two-wide, the
-# relaxation folded into the RF): per state and step the signal's RF 8, the
-# T1 tangent's RF with its product-rule source 10, the T2 tangent's
-# relaxation 4 and RF 8 = 30 FP32-pipe operations, 60 flop at the pipe's rate
-# (the unfolded form with the shift mask executed 39).
-GN_FLOP_PER_STATE_STEP = 60
+# relaxation folded into the RF): per state and step an RF of 8 each and the
+# product rule's sources, one for the T1 and two for the T2 tangent = 27
+# FP32-pipe operations, 54 flop at the pipe's rate.
+GN_FLOP_PER_STATE_STEP = 54
 # bSSFP (complex recursion with B0 precession), convention: RF 54 + two
-# relaxations 12 + two B0 precessions 24 flop; ROA: 31 flop per isochromat
-# and step.
-SSFP_FLOP_PER_STATE_STEP = 90
+# relaxations 12 + two B0 precessions 24 flop = 90, of which the recursion in
+# the frame of the RF phase executes 48 (24 operations); ROA: 31 flop per
+# isochromat and step.
+SSFP_FLOP_PER_STATE_STEP_EXECUTED = 48
 ROA_FLOP_PER_ISO_STEP = 31
 # DRAM bytes per dictionary atom of the headline dictionary form (T = 1000,
 # w = 50: the imaginary parts of the atoms as FP32 rows with their norms, then
@@ -771,13 +771,15 @@ def run_ours(args) -> None:
         rl_gn = roofline("gn_kernel<5, tangents> (5 lanes x 5 state pairs per voxel) and its tail launch: "
                          "one Gauss-Newton pass over every voxel", "fp32",
                          nvox * T * NSTATES * GN_FLOP_PER_STATE_STEP, gn_pass_ms, fp32_peak, fp32_note,
-                         note="60 flop per state-step at the pipe's rate (signal and two tangents); the "
+                         note="54 flop per state-step at the pipe's rate (signal and two tangents); the "
                               "refinement stage is the sub-grid start "
                               f"({fms[HEAD]['start']:.2f} ms) and up to {args.gn_iters} such passes over the "
                               f"voxels still moving ({gn_ms:.2f} ms in the step)")
         rls = sorted([(gn_ms, rl_gn), (dict_ms, rl_dict), (match_ms, rl_match)], key=lambda x: -x[0])
-        rl_fp32 = roofline("match_fp32_kernel<imag>: FP32 B1-bin match (fp32 form), whole call", "fp32",
-                           nvox * 4.0 * T * natoms, fms["fp32"]["match"], fp32_peak, fp32_note)
+        rl_fp32 = roofline("fp32 B1-bin match screened by bf16 hi/lo tcgen05 scores (three products), exact "
+                           "fp32 chains of the candidates, whole call", "tensor",
+                           nvox * 12.0 * T * natoms, fms["fp32"]["match"], pk["bf16_tflops"],
+                           f"bf16 dense, {pk['source']} (burst)")
 
         oracle_cmp = None
         if args.oracle_sample > 0:
@@ -962,9 +964,10 @@ def run_c4(args) -> None:
     fp32_peak, fp32_note = fp32_fma_peak()
     ssfp_ms, _ = ev_time(lambda: snap.MRF_dict(d_atoms, d_params, h, T4, T4, NATOMS, natoms, 4, w, "epg_ssfp"),
                          args.steps, args.warmup)
-    out["ssfp_dict"] = roofline("epg_ref_kernel<SSFP>: bSSFP dictionary (complex recursion, B0)", "fp32",
-                                NATOMS * T4 * w * SSFP_FLOP_PER_STATE_STEP, ssfp_ms, fp32_peak, fp32_note,
-                                flop_note="90 flop per state-step by convention",
+    out["ssfp_dict"] = roofline("epg_ssfp_kernel: bSSFP dictionary in the frame of the RF phase", "fp32",
+                                NATOMS * T4 * w * SSFP_FLOP_PER_STATE_STEP_EXECUTED, ssfp_ms, fp32_peak, fp32_note,
+                                flop_note="48 flop per state-step executed (24 operations); 90 by the convention "
+                                          "of the complex recursion",
                                 atoms_per_s=round(NATOMS / (ssfp_ms / 1e3), 1))
     d_roa = torch.empty((NATOMS, T4, 2), device=dev)
     roa_ms, _ = ev_time(lambda: snap.MRF_dict(d_roa, d_params, h, T4, T4, NATOMS, natoms, 4, w, "roa_ssfp",
@@ -1022,8 +1025,10 @@ def run_c4(args) -> None:
     ms32, _ = ev_time(lambda: snap.MRF_match(d_maps32, d_img32, d_atoms, d_params, T4, T4, NATOMS, natoms, nv32,
                                              d_index=d_idx32), 1, 1)
     clk.mark_end()
-    out["fp32_match"] = roofline("match_fp32_kernel<complex>: FP32 global match, whole call", "fp32",
-                                 nv32 * 8.0 * T4 * NATOMS, ms32, fp32_peak, fp32_note, voxels=nv32,
+    out["fp32_match"] = roofline("fp32 global match screened by bf16 hi/lo tcgen05 scores (three products), "
+                                 "whole call", "tensor",
+                                 nv32 * 24.0 * T4 * NATOMS, ms32, pk["bf16_tflops"],
+                                 f"bf16 dense, {pk['source']} (burst)", voxels=nv32,
                                  voxels_per_s=round(nv32 / (ms32 / 1e3), 1))
     i32 = d_idx32.cpu().numpy()
     m32 = d_maps32.cpu().numpy()

@@ -459,8 +459,9 @@ int snapmrf_mrf_match_noalloc(float *d_maps, const float *d_img, size_t img_stri
  * entries) summed over atoms;
  * d_grad_alpha_atoms: optional out [natoms][nreps]: the per-atom terms;
  * checkpoint_every: states kept every C steps (0: C = ceil(sqrt(nreps))),
- * so device scratch is natoms * (nreps/C + C) * 3 * nstates floats (rounded
- * up to the kernel's state layout). */
+ * so device scratch is at most natoms * (nreps/C + C) * 3 * nstates floats
+ * (twice that for epg_ssfp; rounded up to the kernel's state layout; epg_fisp
+ * and epg_sr keep a segment's C states on chip and need none for them). */
 int snapmrf_epg_adjoint(const float *d_params, int nparams, const float *h_mrf, size_t nreps,
                         size_t NREPS, size_t natoms, int nstates, const char *echo_type,
                         const float *d_grad_signal, float *d_signal, float *d_grad_params,

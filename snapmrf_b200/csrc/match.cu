@@ -308,8 +308,8 @@ extern "C" int snapmrf_mrf_match(float *d_maps, const float *img, int img_on_hos
     // A host image is streamed to the device in chunks on the library's copy
     // stream (one 2D copy per chunk instead of one copy per voxel,
     // src/functions.cu:1524-1530), into img_device_copy or call scratch; the
-    // FP32 form matches each chunk as it arrives, the tensor-core forms wait
-    // for the whole image.
+    // unscreened FP32 form matches each chunk as it arrives, the tensor-core
+    // forms two ranges of voxels.
     float *img_copy = opts ? opts->img_device_copy : nullptr;
     const bool early = (flags & SNAPMRF_MATCH_UPLOAD_EARLY) != 0;
     if (img_copy && !img_on_host)
