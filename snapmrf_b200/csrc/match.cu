@@ -186,7 +186,12 @@ namespace tc {
 __global__ void publish_error_kernel(const int *err);
 }
 
-// Whether the FP32 form's screen pays for its launches.
+// Whether the FP32 form's screen pays for its launches.  Measured at T = 1000
+// (FP32 kernel / screened, us): 2^26 products (256 voxels x 256 atoms) 249 /
+// 133, 2^28 (4,096 x 64) 248 / 146, 2^30 (1,024 x 1,024) 254 / 144, 2^32
+// (4,096 x 837) 828 / 196; random voxels that leave most of 4,096 atoms within
+// the margin (64 voxels, 2^28) 248 / 242.  Below 2^24 the FP32 kernel's serial
+// chain is all there is to win (240 down to 64 x 64), with few launches.
 static bool screen_pays(long long nvox, long long bin_natoms, long long nreps) {
     return nvox * bin_natoms * nreps >= (1ll << 24);
 }
