@@ -186,14 +186,15 @@ namespace tc {
 __global__ void publish_error_kernel(const int *err);
 }
 
-// Whether the FP32 form's screen pays for its launches.  Measured at T = 1000
-// (FP32 kernel / screened, us): 2^26 products (256 voxels x 256 atoms) 249 /
-// 133, 2^28 (4,096 x 64) 248 / 146, 2^30 (1,024 x 1,024) 254 / 144, 2^32
-// (4,096 x 837) 828 / 196; random voxels that leave most of 4,096 atoms within
-// the margin (64 voxels, 2^28) 248 / 242.  Below 2^24 the FP32 kernel's serial
-// chain is all there is to win (240 down to 64 x 64), with few launches.
+// Whether the FP32 form's screen pays for its launches.  Measured on random
+// rows, T = 1000 (FP32 kernel / screened, us): voxels x atoms 64 x 256 (2^24
+// products) 244 / 134, 256 x 256 249 / 127, 4,096 x 64 248 / 141, 1,024 x 1,024
+// 254 / 135, 4,096 x 837 828 / 196.  A voxel's candidates are rescored by one
+// warp, so few voxels with many atoms gain nothing: 32 x 4,096 248 / 239, 4 x
+// 4,096 244 / 235, 1 x 16,384 249 / 600.  Below 2^24 the FP32 kernel's 240 us
+// take fewer launches and no operands.
 static bool screen_pays(long long nvox, long long bin_natoms, long long nreps) {
-    return nvox * bin_natoms * nreps >= (1ll << 24);
+    return nvox >= 32 && nvox * bin_natoms * nreps >= (1ll << 24);
 }
 
 static inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
