@@ -519,10 +519,29 @@ constexpr int kRealFS = kRealChunk * 4 + 4;        // floats per atom of relaxat
 constexpr int kRealReadoutStride = kRealChunk + 1;  // floats per atom
 __host__ __device__ constexpr int epg_real_nc(bool fold) { return fold ? 6 : 10; }  // RF coefficient pairs per step
 
+// Byte offsets in a CTA's shared memory (apc atoms).  RF coefficients, factors
+// and parameters are read 16 bytes at a time, so each starts on a multiple of
+// 16 for any apc; the readouts, single floats in rows of 33, come last.
+__host__ __device__ constexpr size_t epg_real_off_factors(bool fold) {
+    return (size_t)kRealChunk * epg_real_nc(fold) * sizeof(float2);
+}
+__host__ __device__ constexpr size_t epg_real_off_params(int apc, bool fold) {
+    return epg_real_off_factors(fold) + (size_t)apc * kRealFS * sizeof(float);
+}
+__host__ __device__ constexpr size_t epg_real_off_readouts(int apc, bool fold) {
+    return epg_real_off_params(apc, fold) + (size_t)apc * 4 * sizeof(float);
+}
+constexpr bool epg_real_aligned() {
+    for (int apc = 1; apc <= kRealThreads; apc++)
+        for (int fold = 0; fold < 2; fold++)
+            if (epg_real_off_factors(fold) % 16 || epg_real_off_params(apc, fold) % 16) return false;
+    return epg_real_nc(true) * sizeof(float2) % 16 == 0 && kRealFS % 4 == 0;
+}
+static_assert(epg_real_aligned(), "16-byte reads of coefficients, factors and parameters");
+
 inline size_t epg_real_smem_bytes(int L, bool fold) {
-    int apc = kRealThreads / L;
-    return (size_t)kRealChunk * epg_real_nc(fold) * sizeof(float2) + (size_t)apc * kRealFS * sizeof(float) +
-           (size_t)apc * kRealReadoutStride * sizeof(float) + (size_t)apc * 4 * sizeof(float);
+    const int apc = kRealThreads / L;
+    return epg_real_off_readouts(apc, fold) + (size_t)apc * kRealReadoutStride * sizeof(float);
 }
 
 // One element of the optional 16-bit copy of Im(atom) (the tensor-core
@@ -562,10 +581,10 @@ __device__ __forceinline__ void epg_real_cta(const EpgArgs &a, const int L, cons
     const long long gatom = blk * a.natoms + ab;
 
     constexpr int NC = epg_real_nc(FOLD);
-    float2 *sC = reinterpret_cast<float2 *>(smem_raw);           // [kRealChunk][NC]
-    float *sF = reinterpret_cast<float *>(sC + kRealChunk * NC);  // [apc][FS]
-    float *sR = sF + apc * FS;                                   // [apc][kRealReadoutStride]
-    float *sP = sR + apc * kRealReadoutStride;                   // [apc][4]
+    float2 *sC = reinterpret_cast<float2 *>(smem_raw);                                        // [kRealChunk][NC]
+    float *sF = reinterpret_cast<float *>(smem_raw + epg_real_off_factors(FOLD));             // [apc][FS]
+    float *sP = reinterpret_cast<float *>(smem_raw + epg_real_off_params(apc, FOLD));         // [apc][4]
+    float *sR = reinterpret_cast<float *>(smem_raw + epg_real_off_readouts(apc, FOLD));  // [apc][kRealReadoutStride]
 
     if (tid < apc) {
         const long long at = atom0 + tid;

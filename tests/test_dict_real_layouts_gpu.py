@@ -40,3 +40,28 @@ def test_layouts_match_reference_order(snap, echo, w, T):
     n = np.linalg.norm(got.astype(np.complex128), axis=1, keepdims=True)
     n[n == 0] = 1.0  # (a schedule that starts with a zero flip angle: zero atoms stay zero)
     np.testing.assert_allclose(unit.imag, (got / n).imag, rtol=0, atol=(T + 4) * np.finfo(np.float32).eps)
+
+
+@pytest.mark.parametrize("echo", ["epg_fisp", "epg_sr"])
+@pytest.mark.parametrize("w", [257, 400, 512, 513, 800, 1024])
+def test_wide_layouts(snap, oracle, echo, w):
+    """More than 256 states: two atoms and one atom per warp.  A state k is
+    reached after k steps, so in 120 steps the atoms are those of 256 states,
+    the most that the reference order takes: bit for bit with the relaxations
+    apart, to the roundings of 120 folded steps (see above) otherwise.  Steps
+    enough to reach the last states: against the CPU oracle, whose sines and
+    exponentials are the host's (2e-5 of the peak is the bar at 120 steps
+    elsewhere; the roundings add up with the steps)."""
+    T, n = 120, 37
+    h, p = mrf_schedule(T, seed=3), _params(n, 5)
+    ref = run_dict(snap, echo, p, h, T, natoms=n, nstates=256, flags=snap.DICT_REFERENCE_ORDER)
+    apart = run_dict(snap, echo, p, h, T, natoms=n, nstates=w, flags=snap.DICT_SEPARATE_RELAX)
+    np.testing.assert_array_equal(apart, ref)
+    got = run_dict(snap, echo, p, h, T, natoms=n, nstates=w)
+    assert np.abs(got - ref).max() <= 4 * T * np.finfo(np.float32).eps * np.abs(ref).max()
+    T, n = w + 30, 5
+    h, p = mrf_schedule(T, seed=4), _params(n, 6)
+    ref = oracle.dict_atoms(echo, p, h, T, natoms=n, nstates=w)
+    for flags in (0, snap.DICT_SEPARATE_RELAX):
+        got = run_dict(snap, echo, p, h, T, natoms=n, nstates=w, flags=flags)
+        assert (np.abs(got - ref).max(1) <= 2e-5 * T / 120 * np.abs(ref).max(1)).all()
