@@ -14,14 +14,27 @@
 // chosen atom is the one that the FP32 kernel alone chooses: maps and indices
 // are the same bit for bit (tests/test_match_screen_gpu.py).
 //
-// The bound, relative to ||d|| ||x|| (the voxels are scaled to unit norm, the
-// largest ||d|| of the dictionary stands for all), of the difference between
-// the two scores: the FP32 chain's n FMAs, 2^-24 each of a partial sum that
-// Cauchy and Schwarz keep below ||d|| ||x||; the BF16 pairs, 3 2^-18; the
-// tensor core's accumulation, 1.25 2^-23 (a truncated last bit and a quarter)
-// per MMA.  Measured, the scores differ by at most 1.6e-5 at T = 1000 (complex
-// atoms; 1.2e-5 imaginary, 4e-6 at T = 200 .. 300), where the bound is 2.1e-4
-// (1.0e-4, 3e-5).
+// The bound of the difference between an atom's two scores (as complex
+// numbers, for a voxel of unit norm).  With v = hi + lo + rest:
+//  - the products left out, lo lo', rest v' and (hi + lo) rest', are inner
+//    products: at most ||lo_d|| ||lo_x|| + ||rest_d|| + ||d|| ||rest_x||
+//    (Cauchy and Schwarz), the norms summed while packing;
+//  - both sides round a running sum whose k-th value is at most
+//    ||d_1..k|| ||x_1..k||.  FP32: 2^-24 of it at each of the 32 elements of a
+//    chunk.  Tensor core: an MMA adds 16 products to the sum with every addend
+//    cut at 2^-25 of the largest and the result cut to 24 bits, so
+//    (16 / 4 + 1) 2^-23 of it at each of a chunk's six MMAs (measured on the
+//    device with addends of 2^-22 .. 2^-29 beside a sum of 1, each sign: cut
+//    exactly there, never rounded up; NVIDIA documents no bound).  Summed over
+//    the chunks c, by Cauchy and Schwarz again: 92 2^-24 sqrt(sum_c
+//    ||d_1..c||^2) sqrt(sum_c ||x_1..c||^2), the weighted norms of both;
+//  - what is left (the voxel's scaling, the squares and roots of the
+//    comparison) is 2^-22 of ||d||; 2^-20 is allowed, and 0.1 % on everything
+//    for what the bounds above neglect of second order.
+// The largest values of any atom of the dictionary stand for each.  On the
+// configurations' dictionaries the bound is 1.3e-4 (T = 1000, imaginary atoms;
+// 2.6e-4 complex; 3.8e-5 and 6.7e-5 at T = 200), where the scores were seen to
+// differ by 1.6e-5 at most.
 //
 // 57,600 voxels, 284,458 imaginary atoms in 41 blocks, T = 1000: 36.4 -> 4.9
 // ms (packing 0.68, scores 2.9 = three BF16 products at 1.68 PFLOP/s, about
@@ -59,7 +72,8 @@ namespace screen {
 
 constexpr int KB = 32;               // elements of K per 64-element row chunk (hi, then lo)
 constexpr float kMaxAbs = 1e15f;     // larger samples (or not finite) are left to the FP32 kernel
-constexpr float kMinNorm2 = 1e-30f;  // smaller norms too (of either side or their product): squares would lose bits
+constexpr float kMinNorm2 = 1e-30f;  // smaller norms of a voxel and squared scores too: squares would lose bits
+constexpr float kMinAtom2 = 1e-18f;  // (and of all atoms: the squares of their lo and rest parts would)
 constexpr float kMaxNorm2 = 1e30f;
 // Operand memory of one pass: larger dictionaries are screened in chunks of
 // atoms, larger images in ranges of voxels.
@@ -68,8 +82,8 @@ constexpr size_t kAtomBytes = 2ull << 30, kVoxelBytes = 1ull << 30;
 struct State {
     int err;                 // error word of the scoring kernel, or 7
     int bad_atoms;           // an atom is not finite or out of range: the FP32 kernel takes every voxel
-    unsigned norm2_bits;     // largest squared atom norm
     int nfall;               // voxels left to the FP32 kernel
+    tc::AtomStats atoms;
 };
 
 __global__ void init_kernel(unsigned long long *keys, long long nkeys, long long *perm, long long nperm, int *counts,
@@ -78,29 +92,46 @@ __global__ void init_kernel(unsigned long long *keys, long long nkeys, long long
     if (i < nkeys) keys[i] = 0ull;
     if (i < nperm) perm[i] = -1;
     if (i < nbins) counts[i] = fall_counts[i] = 0;
-    if (i == 0) *st = State{0, 0, 0u, 0};
+    if (i == 0) *st = State{0, 0, 0, {0u, 0u, 0u, 0u}};
 }
 
-// hi and lo of two neighbouring elements, packed.
-__device__ __forceinline__ void split2(float a, float b, uint32_t *hi, uint32_t *lo) {
+// Running sums of a row (see tc::AtomStats).
+struct RowSums {
+    float norm2 = 0.f, weighted2 = 0.f, lo2 = 0.f, rest2 = 0.f;
+};
+
+// hi and lo of two neighbouring elements, packed; the squares of lo and of
+// what both leave (exact differences).
+__device__ __forceinline__ void split2(float a, float b, uint32_t *hi, uint32_t *lo, RowSums &r) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     const float2 f = __bfloat1622float2(h);
-    const __nv_bfloat162 l = __floats2bfloat162_rn(a - f.x, b - f.y);
+    const float da = a - f.x, db = b - f.y;
+    const __nv_bfloat162 l = __floats2bfloat162_rn(da, db);
+    const float2 g = __bfloat1622float2(l);
+    r.lo2 = fmaf(g.x, g.x, fmaf(g.y, g.y, r.lo2));
+    const float ra = da - g.x, rb = db - g.y;
+    r.rest2 = fmaf(ra, ra, fmaf(rb, rb, r.rest2));
     *hi = *reinterpret_cast<const uint32_t *>(&h);
     *lo = *reinterpret_cast<const uint32_t *>(&l);
 }
 
 // Eight elements k0 .. k0 + 7 of a row (k0 a multiple of 8): 16 bytes of hi
 // and, 64 bytes further, 16 bytes of lo.
-__device__ __forceinline__ void store8(__nv_bfloat16 *row, long long k0, const float *v) {
+__device__ __forceinline__ void store8(__nv_bfloat16 *row, long long k0, const float *v, RowSums &r) {
     uint4 h, l;
-    split2(v[0], v[1], &h.x, &l.x);
-    split2(v[2], v[3], &h.y, &l.y);
-    split2(v[4], v[5], &h.z, &l.z);
-    split2(v[6], v[7], &h.w, &l.w);
+    split2(v[0], v[1], &h.x, &l.x, r);
+    split2(v[2], v[3], &h.y, &l.y, r);
+    split2(v[4], v[5], &h.z, &l.z, r);
+    split2(v[6], v[7], &h.w, &l.w, r);
     __nv_bfloat16 *p = row + (k0 / KB) * (2 * KB) + k0 % KB;
     *reinterpret_cast<uint4 *>(p) = h;
     *reinterpret_cast<uint4 *>(p + KB) = l;
+}
+
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
 // N samples from t of a row, zeros past nreps (VEC: 16-byte loads).
@@ -120,11 +151,9 @@ __device__ __forceinline__ void load_samples(const float2 *x, long long t, long 
 }
 
 // A rows: the slot's voxel at unit norm, two rows (Re, Im) for purely
-// imaginary atoms, else one interleaved row.  vnorm2[slot]: its squared norm, 0
-// when every sample is 0 (no atom scores above 0), -1 when the FP32 kernel has
-// to take it.  One warp per slot.
+// imaginary atoms, else one interleaved row; its VoxelStats.  One warp per slot.
 template <bool IMAG, bool VEC>
-__global__ void pack_voxels_kernel(__nv_bfloat16 *A, float *vnorm2, const float2 *img, long long img_stride,
+__global__ void pack_voxels_kernel(__nv_bfloat16 *A, tc::VoxelStats *stats, const float2 *img, long long img_stride,
                                    const long long *perm, long long nslots, long long nreps, long long Kp) {
     const long long slot = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x % 32;
@@ -149,9 +178,9 @@ __global__ void pack_voxels_kernel(__nv_bfloat16 *A, float *vnorm2, const float2
     }
     const bool fit = n >= kMinNorm2 && mx <= kMaxAbs && n <= kMaxNorm2;  // (false for NaN)
     const float inv = fit ? rsqrtf(n) : 0.f;
-    if (lane == 0) vnorm2[slot] = fit ? n : (n == 0.f && mx == 0.f) ? 0.f : -1.f;
     const long long K = IMAG ? Kp / 2 : Kp / 4;  // samples, padded
     __nv_bfloat16 *row = A + (IMAG ? 2 * slot : slot) * Kp;
+    RowSums sums;
     for (long long t = (IMAG ? 8 : 4) * lane; t < K; t += (IMAG ? 256 : 128)) {
         float2 s[IMAG ? 8 : 4];
         if (inv > 0.f) {
@@ -160,33 +189,40 @@ __global__ void pack_voxels_kernel(__nv_bfloat16 *A, float *vnorm2, const float2
 #pragma unroll
             for (int u = 0; u < (IMAG ? 8 : 4); u++) s[u] = make_float2(0.f, 0.f);
         }
-        float a[8], b[8];
+        float a[8], b[8], e = 0.f;
 #pragma unroll
         for (int u = 0; u < 8; u++) {
             if (IMAG) {
                 a[u] = s[u].x * inv;
                 b[u] = s[u].y * inv;
+                e = fmaf(b[u], b[u], e);
             } else {
                 a[u] = (u & 1 ? s[u / 2].y : s[u / 2].x) * inv;
             }
+            e = fmaf(a[u], a[u], e);
         }
-        store8(row, IMAG ? t : 2 * t, a);
-        if (IMAG) store8(row + Kp, t, b);
+        const long long k0 = IMAG ? t : 2 * t;
+        sums.weighted2 = fmaf((float)(Kp / (2 * KB) - k0 / KB), e, sums.weighted2);
+        store8(row, k0, a, sums);
+        if (IMAG) store8(row + Kp, t, b, sums);
     }
+    const float w2 = warp_sum(sums.weighted2), l2 = warp_sum(sums.lo2), r2 = warp_sum(sums.rest2);
+    if (lane == 0)
+        stats[slot] = {fit ? n : (n == 0.f && mx == 0.f) ? 0.f : -1.f, sqrtf(w2), sqrtf(l2), sqrtf(r2)};
 }
 
 // B rows of atoms [a0, a0 + n) (row r of the operand: atom a0 + r): one row
 // (Im d) for purely imaginary atoms (a real part sets the error word to 7),
-// else two, (Re d, Im d) and (-Im d, Re d); the largest squared norm and
-// whether every sample is finite and in range.  One warp per atom.  Bound by
+// else two, (Re d, Im d) and (-Im d, Re d); the AtomStats and whether every
+// sample is finite and in range.  One warp per atom.  Bound by
 // its traffic: C1's 284,458 atoms (2.28 GB read, 1.17 GB written) 0.6 ms.
 template <bool IMAG, bool VEC>
 __global__ void pack_atoms_kernel(__nv_bfloat16 *B, const float2 *atoms, long long atom_stride, long long n,
                                   long long nreps, long long Kp, State *st) {
     const long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-    __shared__ float smax[8];
-    float n2 = 0.f, mx = 0.f;
+    __shared__ RowSums srow[8];
+    RowSums sums;
     bool real_part = false, bad = false;
     if (r < n) {
         const float2 *src = atoms + r * atom_stride;
@@ -195,10 +231,10 @@ __global__ void pack_atoms_kernel(__nv_bfloat16 *B, const float2 *atoms, long lo
         for (long long t = (IMAG ? 8 : 4) * lane; t < K; t += (IMAG ? 256 : 128)) {
             float2 s[IMAG ? 8 : 4];
             load_samples<IMAG ? 8 : 4, VEC>(src, t, nreps, s);
-            float a[8], b[8];
+            float a[8], b[8], e = 0.f;
 #pragma unroll
             for (int u = 0; u < (IMAG ? 8 : 4); u++) {
-                n2 += s[u].x * s[u].x + s[u].y * s[u].y;
+                e += s[u].x * s[u].x + s[u].y * s[u].y;
                 bad |= !(fabsf(s[u].x) <= kMaxAbs && fabsf(s[u].y) <= kMaxAbs);
             }
 #pragma unroll
@@ -211,25 +247,33 @@ __global__ void pack_atoms_kernel(__nv_bfloat16 *B, const float2 *atoms, long lo
                     b[u] = u & 1 ? s[u / 2].x : -s[u / 2].y;
                 }
             }
-            store8(row, IMAG ? t : 2 * t, a);
-            if (!IMAG) store8(row + Kp, 2 * t, b);
+            const long long k0 = IMAG ? t : 2 * t;
+            sums.norm2 += e;
+            sums.weighted2 = fmaf((float)(Kp / (2 * KB) - k0 / KB), e, sums.weighted2);
+            store8(row, k0, a, sums);
+            if (!IMAG) {
+                RowSums same;  // (the same elements, other signs)
+                store8(row + Kp, k0, b, same);
+            }
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
-    bad |= !(n2 <= kMaxNorm2);
+    sums = {warp_sum(sums.norm2), warp_sum(sums.weighted2), warp_sum(sums.lo2), warp_sum(sums.rest2)};
+    bad |= !(sums.norm2 <= kMaxNorm2);
     if (IMAG && __any_sync(0xffffffffu, real_part) && lane == 0) atomicCAS(&st->err, 0, 7);
     if (__any_sync(0xffffffffu, bad)) {
-        n2 = 0.f;
+        sums = RowSums();
         if (lane == 0) atomicExch(&st->bad_atoms, 1);
     }
-    if (lane == 0) smax[warp] = n2;
+    if (lane == 0) srow[warp] = sums;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 0; w < (int)blockDim.x / 32; w++) mx = fmaxf(mx, smax[w]);
-        // (one atomic per CTA, and only while it raises the value)
+    if (threadIdx.x < 4) {
+        // one value per thread: one atomic per CTA, and only while it raises the value
+        const int q = threadIdx.x;
+        float mx = 0.f;
+        for (int w = 0; w < (int)blockDim.x / 32; w++) mx = fmaxf(mx, reinterpret_cast<const float *>(&srow[w])[q]);
         const unsigned bits = __float_as_uint(mx);
-        if (bits > *reinterpret_cast<volatile unsigned *>(&st->norm2_bits)) atomicMax(&st->norm2_bits, bits);
+        unsigned *top = reinterpret_cast<unsigned *>(&st->atoms) + q;
+        if (bits > *reinterpret_cast<volatile unsigned *>(top)) atomicMax(top, bits);
     }
 }
 
@@ -262,9 +306,9 @@ __device__ __forceinline__ void copy_samples(float2 *dst, const float2 *src, int
 template <bool IMAG, bool VEC>
 __global__ void __launch_bounds__(kRescoreWarps * 32)
 rescore_kernel(unsigned long long *keys, tc::Lists lists, const int *list_n, const float *list_best,
-               const long long *perm, const float *vnorm2, const long long *tile_start, int nbins,
+               const long long *perm, const tc::VoxelStats *vstats, const long long *tile_start, int nbins,
                const int *vox_bin, const float2 *atoms, long long atom_stride, const float2 *img,
-               long long img_stride, int nreps, long long bin_natoms, float margin_rel, State *st, int *fall,
+               long long img_stride, int nreps, long long bin_natoms, float chain, State *st, int *fall,
                int *fall_counts) {
     __shared__ RescoreSmem smem[kRescoreWarps];
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -272,8 +316,8 @@ rescore_kernel(unsigned long long *keys, tc::Lists lists, const int *list_n, con
     const long long slot = blockIdx.x * (long long)kRescoreWarps + warp;
     if (slot >= tile_start[nbins] * lists.vt) return;
     const long long v = perm[slot];
-    const float xn2 = vnorm2[slot];
-    if (v < 0 || xn2 == 0.f) return;
+    const tc::VoxelStats vs = vstats[slot];
+    if (v < 0 || vs.norm2 == 0.f) return;
     const int bin = vox_bin ? vox_bin[v] : 0;
     auto leave = [&]() {
         if (lane == 0) {
@@ -281,9 +325,9 @@ rescore_kernel(unsigned long long *keys, tc::Lists lists, const int *list_n, con
             atomicAdd(&fall_counts[bin], 1);
         }
     };
-    const float norm2 = __uint_as_float(st->norm2_bits);
-    if (xn2 < 0.f || st->bad_atoms || norm2 < kMinNorm2 || norm2 * xn2 < kMinNorm2 || norm2 * xn2 > kMaxNorm2)
-        return leave();
+    const tc::AtomStats as = st->atoms;
+    const float norm2 = __uint_as_float(as.norm2);
+    if (vs.norm2 < 0.f || st->bad_atoms || norm2 < kMinAtom2 || norm2 * vs.norm2 > kMaxNorm2) return leave();
     // the slot's lists: counts and best scores, one list per lane
     constexpr int LISTS = tc::split_lists(IMAG), CAPL = tc::LIST_CAP / LISTS;
     const tc::ListSlots at = tc::list_slots(lists, slot);
@@ -300,8 +344,8 @@ rescore_kernel(unsigned long long *keys, tc::Lists lists, const int *list_n, con
     const bool over = n > CAPL;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
-    const float low = sqrtf(best) - margin_rel * sqrtf(norm2);
-    if (__any_sync(0xffffffffu, over) || !(low > 0.f)) return leave();
+    const float low = sqrtf(best) - tc::screen_margin(as, vs, chain);
+    if (__any_sync(0xffffffffu, over) || !(low > 0.f) || best * vs.norm2 < kMinNorm2) return leave();
     const float thr = low * low * (1.f - 0x1p-20f);
     int count = 0;
     for (int l = 0; l < nl; l++) {
@@ -471,7 +515,7 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
     const size_t oTs = take(lb), oTi = take(lb), oLn = take(hb), oLb = take(hb), oPlan = take(sizeof(tc::TailPlan));
     const size_t oKey = take((size_t)nv_max * 8);
     const size_t oPerm = take((size_t)cap * 8), oFperm = take((size_t)nv_max * 8), oFall = take((size_t)nv_max * 4);
-    const size_t oVb = take((size_t)nv_max * 4), oKind = take((size_t)cap * 4);
+    const size_t oVb = take((size_t)nv_max * 4), oVs = take((size_t)cap * sizeof(tc::VoxelStats));
     const size_t oBin = take(5 * (size_t)(nbins + 1) * 8), oCnt = take(2 * (size_t)nbins * 4), oSt = take(sizeof(State));
     DeviceScratch s;
     const cudaError_t ae = s.alloc(bytes, st);
@@ -486,16 +530,14 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
     unsigned long long *keys = reinterpret_cast<unsigned long long *>(b + oKey);
     long long *perm = reinterpret_cast<long long *>(b + oPerm), *fperm = reinterpret_cast<long long *>(b + oFperm);
     int *fall = reinterpret_cast<int *>(b + oFall), *vox_bin = reinterpret_cast<int *>(b + oVb);
-    float *vnorm2 = reinterpret_cast<float *>(b + oKind);
+    tc::VoxelStats *vstats = reinterpret_cast<tc::VoxelStats *>(b + oVs);
     long long *tile_start = reinterpret_cast<long long *>(b + oBin), *cursor = tile_start + nbins + 1;
     long long *fslot = cursor + nbins + 1, *ftile = fslot + nbins + 1, *fcursor = ftile + nbins + 1;
     int *counts = reinterpret_cast<int *>(b + oCnt), *fall_counts = counts + nbins;
     State *state = reinterpret_cast<State *>(b + oSt);
     *done = true;
 
-    const float eps = 0x1p-24f, n = (float)K;
-    const float delta = n * eps + 3.f * 0x1p-18f + 1.25f * 6.f * (float)nk * 0x1p-23f + 0x1p-20f;
-    const float margin_rel = 2.f * delta * (1.f + 0x1p-16f);
+    const float chain = 92.f * 0x1p-24f * (1.f + (float)K * 0x1p-22f);
     auto aligned = [](const void *p, long long stride) {
         return stride % 2 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0;
     };
@@ -523,7 +565,7 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
         const bool ivec = aligned(img, q.img_stride);
         auto pv = q.imag ? (ivec ? pack_voxels_kernel<true, true> : pack_voxels_kernel<true, false>)
                          : (ivec ? pack_voxels_kernel<false, true> : pack_voxels_kernel<false, false>);
-        pv<<<nblk(cap * 32, 256), 256, 0, st>>>(A, vnorm2, img, q.img_stride, perm, cap, q.nreps, Kp);
+        pv<<<nblk(cap * 32, 256), 256, 0, st>>>(A, vstats, img, q.img_stride, perm, cap, q.nreps, Kp);
         SNAPMRF_LAUNCH_CHECK();
 
         tc::ScoreLaunch sl;
@@ -545,8 +587,9 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
         a.top_s = reinterpret_cast<float *>(b + oTs);
         a.top_i = reinterpret_cast<int *>(b + oTi);
         a.plan = reinterpret_cast<tc::TailPlan *>(b + oPlan);
-        a.margin_rel = margin_rel;
-        a.norm2_bits = &state->norm2_bits;
+        a.chain = chain;
+        a.atom_stats = &state->atoms;
+        a.vox_stats = vstats;
         a.list_n = reinterpret_cast<int *>(b + oLn);
         a.list_best = reinterpret_cast<float *>(b + oLb);
         a.err = &state->err;
@@ -580,8 +623,8 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
         auto rk = q.imag ? (avec && ivec ? rescore_kernel<true, true> : rescore_kernel<true, false>)
                          : (avec && ivec ? rescore_kernel<false, true> : rescore_kernel<false, false>);
         rk<<<nblk(cap, kRescoreWarps), kRescoreWarps * 32, 0, st>>>(
-            keys, lists, a.list_n, a.list_best, perm, vnorm2, tile_start, nbins, b1 ? vox_bin : nullptr, q.atoms,
-            q.atom_stride, img, q.img_stride, (int)q.nreps, bin_natoms, margin_rel, state, fall, fall_counts);
+            keys, lists, a.list_n, a.list_best, perm, vstats, tile_start, nbins, b1 ? vox_bin : nullptr, q.atoms,
+            q.atom_stride, img, q.img_stride, (int)q.nreps, bin_natoms, chain, state, fall, fall_counts);
         SNAPMRF_LAUNCH_CHECK();
         fall_bins_kernel<<<1, 1024, 0, st>>>(state, fall, fall_counts, b1 ? vox_bin : nullptr, fslot, ftile, fcursor,
                                              fperm, nbins);

@@ -330,7 +330,8 @@ match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             int ln = 0;
             float best = 0.f, keep = 0.f, margin = 0.f;
             if constexpr (SPLIT) {
-                margin = p.margin_rel * sqrtf(__uint_as_float(*p.norm2_bits));
+                margin = screen_margin(*p.atom_stats,
+                                       p.vox_stats[(item0 + u.item) * VPT + (IMAG ? row / 2 : row)], p.chain);
                 if (p.resume) {
                     ln = p.list_n[lid];
                     best = p.list_best[lid];

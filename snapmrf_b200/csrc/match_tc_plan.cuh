@@ -35,6 +35,25 @@ constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + HOLD_BYTES + 1024;
 static_assert(SMEM_BYTES + 2 * BM * 8 + 512 <= 227 * 1024, "shared memory of one CTA");
 constexpr uint32_t TMEM_COLS = 512;
 
+// What the FP32 form's screen knows of its operands.  v = hi + lo + rest, hi
+// and lo its BF16 parts; weighted: sum of (nk - k / 32) v_k^2, nk chunks of 32
+// elements.  Atoms: the largest value of any (the bits of floats >= 0 order as
+// integers); voxels: of the slot's voxel at unit norm.
+struct AtomStats {
+    unsigned norm2, weighted2, lo2, rest2;
+};
+struct VoxelStats {
+    float norm2;                // 0: nothing scores above 0; < 0: left to the FP32 kernel
+    float weighted, lo, rest;   // square roots
+};
+// Twice a bound of |approximate score - FP32 score| (the argument: match_fp32_tc.cu).
+__device__ __forceinline__ float screen_margin(const AtomStats &a, const VoxelStats &v, float chain) {
+    auto root = [](unsigned bits) { return sqrtf(__uint_as_float(bits)); };
+    const float first = chain * root(a.weighted2) * v.weighted;
+    const float second = root(a.lo2) * v.lo + root(a.rest2) + root(a.norm2) * (v.rest + 0x1p-20f);
+    return 2.002f * (first + second);
+}
+
 struct Args {
     const long long *tile_start;  // [nbins + 1], in work items
     int nbins;
@@ -52,10 +71,11 @@ struct Args {
     float *top_s;                 // [slots][NLISTS][TOPK_MAX]; SPLIT: [slots][LIST_CAP]
     int *top_i;
     int *err;
-    // SPLIT: candidates within `margin_rel` x the largest atom norm of the
-    // best score, LIST_CAP per slot shared by its split_lists lists
-    float margin_rel;
-    const unsigned *norm2_bits;   // largest squared atom norm so far (float bits)
+    // SPLIT: candidates within screen_margin of the best score, LIST_CAP per
+    // slot shared by its split_lists lists
+    float chain;                  // see screen_margin
+    const AtomStats *atom_stats;  // of the atoms packed so far
+    const VoxelStats *vox_stats;  // [slots]
     int *list_n;                  // [slots][lists] entries, more than the list holds: overflow
     float *list_best;             // [slots][lists] the best score the list's thread has seen
     int resume;                   // the lists continue those of an earlier launch (atom0 > 0)

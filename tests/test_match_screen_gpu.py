@@ -115,3 +115,58 @@ def test_more_near_ties_than_a_list_holds(snap, imag):
     a, b = _both(snap, img, atoms, params, 120, 20000, None, imag)
     np.testing.assert_array_equal(a[1], b[1])
     np.testing.assert_array_equal(a[0], b[0])
+
+
+@pytest.mark.parametrize("imag", [True, False])
+@pytest.mark.parametrize("T", [8, 9, 16, 17, 31, 33, 48])
+def test_short_rows(snap, imag, T):
+    """Few samples: the split of the operands, not the sums' rounding, decides
+    the screen's bound."""
+    atoms, img, params = _inputs(2100, 1300, T, 1, imag, seed=T)
+    a, b = _both(snap, img, atoms, params, T, 1300, None, imag)
+    np.testing.assert_array_equal(a[1], b[1])
+    np.testing.assert_array_equal(a[0], b[0])
+
+
+@pytest.mark.parametrize("imag", [True, False])
+def test_parts_left_out_by_the_split(snap, imag):
+    """Rows made for the split's largest error: 15 of 16 samples just below
+    and just above 1 + 2^-8 round to neighbouring BF16 values, the products of
+    the low parts that the screen leaves out have opposite signs, and the atom
+    that scores higher in FP32 (by 2k ulp) looks worse to the screen by 2^-15."""
+    T, n = 16, 1100
+    f = np.float32
+    x = np.zeros((1100, T), f)
+    # (scaled to unit norm by a factor a few ulp off 1: m keeps them above the tie)
+    x[:, :15] = f(1 + 2.0 ** -8) / 4 + (1 + np.arange(1100) % 64)[:, None].astype(f) * f(2.0 ** -25)
+    x[:, 15] = np.sqrt(1 - 15 * x[:, 0].astype(np.float64) ** 2)
+    img = np.where((np.arange(1100) % 2 == 0)[:, None], x * 1j, x + 0j).astype(np.complex64)
+    params = np.random.default_rng(2).uniform(1, 100, (n, 4)).astype(f)
+    for k in (1, 2, 3, 8):
+        d = np.zeros((n, T), f)     # (the other atoms score 0: nothing else is listed)
+        d[20, :15] = f(1 + 2.0 ** -8) - f(k * 2.0 ** -23)
+        d[320, :15] = f(1 + 2.0 ** -8) + f(k * 2.0 ** -23)
+        a, b = _both(snap, img, (1j * d if imag else d + 0j).astype(np.complex64), params, T, n, None, imag)
+        np.testing.assert_array_equal(a[1], b[1])
+        np.testing.assert_array_equal(a[0], b[0])
+        assert (b[1] == 320).all()
+
+
+@pytest.mark.parametrize("imag", [True, False])
+def test_sums_that_the_tensor_core_cuts(snap, imag):
+    """A large first product, then small ones that an FP32 sum and the tensor
+    core's round differently (1.25 2^-24 beside 1: up to 2^-23 and down to
+    2^-24), against the same products in the other order."""
+    T, n = 1000, 300
+    rng = np.random.default_rng(11)
+    d = np.full((n, T), np.sqrt(1.25 * 2.0 ** -24))
+    d[:, 0] = 1.0
+    d[n // 2:] = d[n // 2:, ::-1]
+    d *= 1 + 4e-5 * rng.uniform(-1, 1, (n, 1))
+    x = np.full((120, T), np.sqrt(1.25 * 2.0 ** -24)) * (1 + 1e-3 * rng.standard_normal((120, T)))
+    x[:, 0] = x[:, -1] = 1.0
+    x = (x * np.exp(1j * np.pi / 2 * rng.integers(0, 4, (120, 1)))).astype(np.complex64)
+    params = rng.uniform(1, 100, (n, 4)).astype(np.float32)
+    a, b = _both(snap, x, (1j * d if imag else d + 0j).astype(np.complex64), params, T, n, None, imag)
+    np.testing.assert_array_equal(a[1], b[1])
+    np.testing.assert_array_equal(a[0], b[0])
