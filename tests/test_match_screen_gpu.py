@@ -170,3 +170,22 @@ def test_sums_that_the_tensor_core_cuts(snap, imag):
     a, b = _both(snap, x, (1j * d if imag else d + 0j).astype(np.complex64), params, T, n, None, imag)
     np.testing.assert_array_equal(a[1], b[1])
     np.testing.assert_array_equal(a[0], b[0])
+
+
+@pytest.mark.parametrize("imag", [True, False])
+def test_blocks_without_voxels_are_not_looked_at(snap, imag):
+    """A B1 block that no voxel falls into: whatever its atoms hold (a real
+    part, NaN, another scale) changes nothing."""
+    nb, natoms = 4, 700
+    atoms, img, params = _inputs(600, natoms, 90, nb, imag, seed=21)
+    b1map = np.random.default_rng(1).choice(np.float32([0.8, 1.0]), 600)      # blocks 0 and 2
+    want = _both(snap, img, atoms, params, 90, natoms, b1map, imag)
+    other = atoms.copy()
+    other[natoms:2 * natoms] *= 1e12
+    other[natoms + 3, 5] = 0.25 + 1j
+    other[3 * natoms + 1, 2] = np.nan
+    other[3 * natoms + 2, 2] = 1e30
+    a, b = _both(snap, img, other, params, 90, natoms, b1map, imag)
+    for got in (a, b, want[0]):
+        np.testing.assert_array_equal(got[1], want[1][1])
+        np.testing.assert_array_equal(got[0], want[1][0])
