@@ -281,7 +281,7 @@ __global__ void pack_atoms_kernel(__nv_bfloat16 *B, const float2 *atoms, long lo
     }
 }
 
-// The voxels' winners: FP32 scores of every listed atom within the bound, in
+// The winners of the voxels of bins [bin_lo, bin_hi): FP32 scores of every listed atom within the bound, in
 // match_fp32_kernel's order, or the voxel goes to the fall list.  One warp per
 // slot; lane c carries candidate c's chain (kBatch of them at a time) through
 // samples that cp.async stages kDepth steps of kSteps ahead.  The chain is
@@ -310,15 +310,15 @@ __device__ __forceinline__ void copy_samples(float2 *dst, const float2 *src, int
 template <bool IMAG, bool VEC>
 __global__ void __launch_bounds__(kRescoreWarps * 32)
 rescore_kernel(unsigned long long *keys, tc::Lists lists, const int *list_n, const float *list_best,
-               const long long *perm, const tc::VoxelStats *vstats, const long long *tile_start, int nbins,
+               const long long *perm, const tc::VoxelStats *vstats, const long long *tile_start, int bin_lo, int bin_hi,
                const int *vox_bin, const float2 *atoms, long long atom_stride, const float2 *img,
                long long img_stride, int nreps, long long bin_natoms, float chain, State *st, int *fall,
                int *fall_counts) {
     __shared__ RescoreSmem smem[kRescoreWarps];
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     RescoreSmem &sm = smem[warp];
-    const long long slot = blockIdx.x * (long long)kRescoreWarps + warp;
-    if (slot >= tile_start[nbins] * lists.vt) return;
+    const long long slot = tile_start[bin_lo] * lists.vt + blockIdx.x * (long long)kRescoreWarps + warp;
+    if (slot >= tile_start[bin_hi] * lists.vt) return;
     const long long v = perm[slot];
     const tc::VoxelStats vs = vstats[slot];
     if (v < 0 || vs.norm2 == 0.f) return;
@@ -504,9 +504,7 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
     int num_sms = 0, dev = 0;
     SNAPMRF_CUDA(cudaGetDevice(&dev));
     SNAPMRF_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
-    // (items are split only when one launch covers the whole dictionary)
-    const bool one = bins_per == nbins && chunk == bin_natoms;
-    const long long lslots = cap + (one ? tc::split_slots(cap / vt, num_sms) * vt : 0);
+    const long long lslots = cap + tc::split_slots(cap / vt, num_sms) * vt;
 
     size_t bytes = 0;
     auto take = [&](size_t n) {
@@ -585,7 +583,7 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
         a.tile_start = tile_start;
         a.nbins = nbins;
         a.bin_natoms = bin_natoms;
-        a.max_parts = one ? tc::MAX_PARTS : 1;
+        a.plan_tiles = (int)((chunk + apt - 1) / apt);
         a.ascale2 = nullptr;
         a.cap = cap;
         a.top_s = reinterpret_cast<float *>(b + oTs);
@@ -599,6 +597,14 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
         a.err = &state->err;
         auto pa = q.imag ? (avec ? pack_atoms_kernel<true, true> : pack_atoms_kernel<true, false>)
                          : (avec ? pack_atoms_kernel<false, true> : pack_atoms_kernel<false, false>);
+        tc::Lists lists;
+        lists.top_s = a.top_s;
+        lists.top_i = a.top_i;
+        lists.plan = a.plan;
+        lists.cap = cap;
+        lists.vt = vt;
+        auto rk = q.imag ? (avec && ivec ? rescore_kernel<true, true> : rescore_kernel<true, false>)
+                         : (avec && ivec ? rescore_kernel<false, true> : rescore_kernel<false, false>);
         for (int b0 = 0; b0 < nbins; b0 += bins_per) {
             const int nb = std::min(bins_per, nbins - b0);
             for (long long a0 = 0; a0 < bin_natoms; a0 += chunk) {
@@ -617,19 +623,12 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
                 int rc = tc::launch_scores(sl, num_sms, st);
                 if (rc) return rc;
             }
+            // (the next bins' launch uses the split items' lists again)
+            rk<<<nblk(cap, kRescoreWarps), kRescoreWarps * 32, 0, st>>>(
+                keys, lists, a.list_n, a.list_best, perm, vstats, tile_start, b0, b0 + nb, b1 ? vox_bin : nullptr,
+                q.atoms, q.atom_stride, img, q.img_stride, (int)q.nreps, bin_natoms, chain, state, fall, fall_counts);
+            SNAPMRF_LAUNCH_CHECK();
         }
-        tc::Lists lists;
-        lists.top_s = a.top_s;
-        lists.top_i = a.top_i;
-        lists.plan = a.plan;
-        lists.cap = cap;
-        lists.vt = vt;
-        auto rk = q.imag ? (avec && ivec ? rescore_kernel<true, true> : rescore_kernel<true, false>)
-                         : (avec && ivec ? rescore_kernel<false, true> : rescore_kernel<false, false>);
-        rk<<<nblk(cap, kRescoreWarps), kRescoreWarps * 32, 0, st>>>(
-            keys, lists, a.list_n, a.list_best, perm, vstats, tile_start, nbins, b1 ? vox_bin : nullptr, q.atoms,
-            q.atom_stride, img, q.img_stride, (int)q.nreps, bin_natoms, chain, state, fall, fall_counts);
-        SNAPMRF_LAUNCH_CHECK();
         fall_bins_kernel<<<1, 1024, 0, st>>>(state, fall, fall_counts, b1 ? vox_bin : nullptr, fslot, ftile, fcursor,
                                              fperm, nbins);
         SNAPMRF_LAUNCH_CHECK();

@@ -121,7 +121,7 @@ match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     constexpr bool HELD = TOPK > 4;         // (four slots insert at once)
     const int natiles = (p.chunk_natoms + APT - 1) / APT;
     const long long item0 = p.tile_start[p.bin_lo];
-    const TailPlan plan = tail_plan(p.tile_start[p.bin_hi] - item0, gridDim.x, natiles, p.max_parts);
+    const TailPlan plan = tail_plan(item0, p.tile_start[p.bin_hi] - item0, gridDim.x, p.plan_tiles);
     if (blockIdx.x == 0 && threadIdx.x == 0) *p.plan = plan;
 
     if (threadIdx.x == 0) {
@@ -1298,7 +1298,7 @@ int match_bf16(const TcMatchRequest &q, cudaStream_t st) {
     a.bin_natoms = bin_natoms;
     a.atom0 = 0;
     a.chunk_natoms = (int)bin_natoms;
-    a.max_parts = MAX_PARTS;
+    a.plan_tiles = (int)((bin_natoms + (imag ? BN : BA) - 1) / (imag ? BN : BA));
     a.plan = reinterpret_cast<TailPlan *>(b + oPlan);
     a.ascale2 = fp8 ? ascale2 : nullptr;
     a.cap = cap;

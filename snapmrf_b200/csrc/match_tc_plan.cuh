@@ -61,7 +61,7 @@ struct Args {
     long long bin_natoms;         // atoms per bin
     int atom0;                    // atoms [atom0, atom0 + chunk_natoms) of each bin are in the operand
     int chunk_natoms;
-    int max_parts;                // see tail_plan
+    int plan_tiles;               // atom tiles that tail_plan splits: of the first chunk
     struct TailPlan *plan;        // out: the launch's plan, for the rescoring
     int nk;                       // K chunks of BK
     int tile_stride;              // atom tiles visited in the order (at * tile_stride) % natiles
@@ -88,23 +88,27 @@ __host__ __device__ constexpr int split_lists(bool imag) { return imag ? 4 : 2; 
 // item; the `rem` items past the last whole round would leave most CTAs idle for a full item's time, so each is split into `parts` by its
 // atom tiles (part p takes every parts-th tile from p on), each part with
 // lists of its own that the rescoring joins.  parts: the fewest (up to
-// max_parts and the tiles there are) whose last rounds take the least time, if
+// MAX_PARTS and the tiles there are) whose last rounds take the least time, if
 // that is at most 3/4 of the unsplit item's.  240 x 240 voxels over 41 B1
 // blocks, BF16 top-16 (921 items on 148 CTAs): 6.33 rounds instead of 7.
 // 16,384 voxels against 111,008 complex atoms (128 items, 0.875 of an item's
 // time in 8 parts) measured slower split, 6.22 against 6.01 ms: the chip is
 // at its power limit either way, and the rescoring joins 16 lists.
+// (A bin larger than the operand is scored in chunks whose launches go on with
+// the same lists, so they share the plan of the first chunk.)
 struct TailPlan {
+    long long item0;       // the launch's first item; the numbers below count from it
     long long bulk, work;  // items before the split ones; CTA work units
     int parts;
 };
-__device__ __forceinline__ TailPlan tail_plan(long long items, int grid, int natiles, int max_parts) {
+__device__ __forceinline__ TailPlan tail_plan(long long item0, long long items, int grid, int natiles) {
     TailPlan t;
+    t.item0 = item0;
     t.bulk = items / grid * grid;
     const int rem = (int)(items - t.bulk);
     t.parts = 1;
     int best = rem ? natiles : 0;  // tile times of the last rounds
-    for (int s = 2; rem && s <= min(max_parts, natiles); s++) {
+    for (int s = 2; rem && s <= min(MAX_PARTS, natiles); s++) {
         const int c = ((rem * s + grid - 1) / grid) * ((natiles + s - 1) / s);
         if (c < best && 4 * c <= 3 * natiles) {
             best = c;
@@ -164,7 +168,7 @@ struct ListSlots {
 };
 __device__ __forceinline__ ListSlots list_slots(const Lists &l, long long slot) {
     const TailPlan t = *l.plan;
-    const long long item = slot / l.vt;
+    const long long item = slot / l.vt - t.item0;
     if (item < t.bulk || t.parts == 1) return {slot, 1};
     return {l.cap + (item - t.bulk) * t.parts * l.vt + slot % l.vt, t.parts};
 }
