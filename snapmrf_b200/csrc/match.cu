@@ -186,15 +186,20 @@ namespace tc {
 __global__ void publish_error_kernel(const int *err);
 }
 
-// Whether the FP32 form's screen pays for its launches.  Measured on random
-// rows, T = 1000 (FP32 kernel / screened, us): voxels x atoms 64 x 256 (2^24
-// products) 244 / 134, 256 x 256 249 / 127, 4,096 x 64 248 / 141, 1,024 x 1,024
-// 254 / 135, 4,096 x 837 828 / 196.  A voxel's candidates are rescored by one
-// warp, so few voxels with many atoms gain nothing: 32 x 4,096 248 / 239, 4 x
-// 4,096 244 / 235, 1 x 16,384 249 / 600.  Below 2^24 the FP32 kernel's 240 us
-// take fewer launches and no operands.
-static bool screen_pays(long long nvox, long long bin_natoms, long long nreps) {
-    return nvox >= 32 && nvox * bin_natoms * nreps >= (1ll << 24);
+// Whether the FP32 form's screen pays for its launches.  Measured, T = 1000
+// (FP32 kernel / screened, us).  One block, random rows: voxels x atoms 64 x
+// 256 (2^24 products) 244 / 134, 256 x 256 249 / 127, 4,096 x 64 248 / 141,
+// 1,024 x 1,024 254 / 135, 4,096 x 837 828 / 200.  Below 2^24 the FP32
+// kernel's 240 us take fewer launches and no operands; below 32 voxels the
+// candidates' chains take as long: 32 x 4,096 248 / 239, 4 x 4,096 244 / 235.
+// Several blocks: how the voxels fall on them is not known here, and the FP32
+// kernel reads only blocks with voxels.  All in one of 41 blocks of 6,938
+// atoms, imaginary: 32 voxels 191 / 293, 100 288 / 297, 1,000 731 / 318;
+// complex (twice the operand, in three passes): 32 280 / 530, 320 466 / 534,
+// 1,000 1,269 / 550.  Over all 41: 100 voxels 1,716 / 946 and 3,196 / 2,924.
+// The lines lie where the first of these cost nothing.
+static bool screen_pays(long long nvox, long long bin_natoms, long long nreps, bool blocks, bool imag) {
+    return nvox >= (!blocks ? 32 : imag ? 96 : 384) && nvox * bin_natoms * nreps >= (1ll << 24);
 }
 
 static inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -572,7 +577,9 @@ extern "C" int snapmrf_mrf_match(float *d_maps, const float *img, int img_on_hos
     // Screened on the tensor cores where that applies (see match_fp32_tc.cu):
     // not for compressed scores, blocks with several B1 values, or calls too
     // small to pay for its launches.
-    const bool screen = !comp && !general && screen_pays(nvox, (long long)(d_b1 ? natoms : NATOMS), (long long)nreps);
+    const bool screen = !comp && !general &&
+                        screen_pays(nvox, (long long)(d_b1 ? natoms : NATOMS), (long long)nreps, d_b1 && nblocks > 1,
+                                    (flags & SNAPMRF_MATCH_IMAG_ATOMS) != 0);
     auto range = [&](long long v0, long long n) -> int {
         float *maps = d_maps + 5 * v0;
         int64_t *index = d_index ? d_index + v0 : nullptr;
