@@ -78,6 +78,7 @@ constexpr float kMaxNorm2 = 1e30f;
 // Operand memory of one pass: larger dictionaries are screened in chunks of
 // atoms, larger images in ranges of voxels.
 constexpr size_t kAtomBytes = 2ull << 30, kVoxelBytes = 1ull << 30;
+constexpr size_t kListBytes = 1ull << 30;  // and of the candidates' lists
 
 struct State {
     int err;                 // error word of the scoring kernel, or 7
@@ -281,13 +282,14 @@ __global__ void pack_atoms_kernel(__nv_bfloat16 *B, const float2 *atoms, long lo
     }
 }
 
-// The winners of the voxels of bins [bin_lo, bin_hi): FP32 scores of every listed atom within the bound, in
-// match_fp32_kernel's order, or the voxel goes to the fall list.  One warp per
-// slot; lane c carries candidate c's chain (kBatch of them at a time) through
-// samples that cp.async stages kDepth steps of kSteps ahead.  The chain is
-// serial by definition: 57,600 voxels of about eight candidates 0.73 ms, their
-// rows 3.7 GB from L2 (8-byte copies and reads 0.88, waiting for each
-// candidate's load in turn 2.4 ms).
+// The winners of the voxels of bins [bin_lo, bin_hi): FP32 scores of every
+// listed atom within the bound, in match_fp32_kernel's order, or the voxel goes
+// to the fall list.  One warp per slot (WIDE: one CTA, whose warps take the
+// batches in turn); lane c carries candidate c's chain (kBatch of them at a
+// time) through samples that cp.async stages kDepth steps of kSteps ahead.
+// The chain is serial by definition: 57,600 voxels of about ten candidates
+// 0.80 ms, their rows 4.6 GB from L2 (8-byte copies and reads 0.88, waiting
+// for each candidate's load in turn 2.4 ms).
 constexpr int kRescoreWarps = 4, kMaxCand = 96, kBatch = 16, kSteps = 16, kDepth = 3;
 struct alignas(16) RescoreSmem {
     float2 d[kDepth][kBatch][kSteps + 2];  // (rows padded: the lanes' reads differ in bank)
@@ -307,24 +309,29 @@ __device__ __forceinline__ void copy_samples(float2 *dst, const float2 *src, int
 }
 
 // VEC: every row starts 16-byte aligned, so a lane copies two samples at once.
-template <bool IMAG, bool VEC>
-__global__ void __launch_bounds__(kRescoreWarps * 32)
-rescore_kernel(unsigned long long *keys, tc::Lists lists, const int *list_n, const float *list_best,
+// (7 CTAs per SM, as shared memory allows: 4,096 voxels in one wave)
+template <bool IMAG, bool VEC, bool WIDE>
+__global__ void __launch_bounds__(kRescoreWarps * 32, 7)
+rescore_kernel(unsigned long long *keys, tc::Lists lists, int list_cap, const int *list_n, const float *list_best,
                const long long *perm, const tc::VoxelStats *vstats, const long long *tile_start, int bin_lo, int bin_hi,
                const int *vox_bin, const float2 *atoms, long long atom_stride, const float2 *img,
                long long img_stride, int nreps, long long bin_natoms, float chain, State *st, int *fall,
                int *fall_counts) {
     __shared__ RescoreSmem smem[kRescoreWarps];
+    __shared__ float wide_s[kRescoreWarps];
+    __shared__ int wide_i[kRescoreWarps];
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     RescoreSmem &sm = smem[warp];
-    const long long slot = tile_start[bin_lo] * lists.vt + blockIdx.x * (long long)kRescoreWarps + warp;
+    const long long slot = tile_start[bin_lo] * lists.vt +
+                           (WIDE ? blockIdx.x : blockIdx.x * (long long)kRescoreWarps + warp);
+    const bool first_warp = !WIDE || warp == 0;
     if (slot >= tile_start[bin_hi] * lists.vt) return;
     const long long v = perm[slot];
     const tc::VoxelStats vs = vstats[slot];
     if (v < 0 || vs.norm2 == 0.f) return;
     const int bin = vox_bin ? vox_bin[v] : 0;
     auto leave = [&]() {
-        if (lane == 0) {
+        if (first_warp && lane == 0) {
             fall[atomicAdd(&st->nfall, 1)] = (int)v;
             atomicAdd(&fall_counts[bin], 1);
         }
@@ -333,114 +340,124 @@ rescore_kernel(unsigned long long *keys, tc::Lists lists, const int *list_n, con
     const float norm2 = __uint_as_float(as.norm2);
     if (vs.norm2 < 0.f || st->bad_atoms || norm2 < kMinAtom2 || norm2 * vs.norm2 > kMaxNorm2) return leave();
     // the slot's lists: counts and best scores, one list per lane
-    constexpr int LISTS = tc::split_lists(IMAG), CAPL = tc::LIST_CAP / LISTS;
+    constexpr int LISTS = tc::split_lists(IMAG);
     const tc::ListSlots at = tc::list_slots(lists, slot);
     const int nl = at.n * LISTS;
     static_assert(tc::MAX_PARTS * 4 <= 32, "a lane per list");
-    long long lid = 0;
+    long long lbase = 0;
     int n = 0;
     float best = 0.f;
     if (lane < nl) {
-        lid = (at.first + (long long)(lane / LISTS) * lists.vt) * LISTS + lane % LISTS;
+        const long long lid = (at.first + (long long)(lane / LISTS) * lists.vt) * LISTS + lane % LISTS;
+        lbase = tc::list_offset(lid, lists.cap * LISTS, list_cap, at.n);
         n = list_n[lid];
         best = list_best[lid];
     }
-    const bool over = n > CAPL;
+    const bool over = n == tc::LIST_OVER;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
     const float low = sqrtf(best) - tc::screen_margin(as, vs, chain);
     if (__any_sync(0xffffffffu, over) || !(low > 0.f) || best * vs.norm2 < kMinNorm2) return leave();
     const float thr = low * low * (1.f - 0x1p-20f);
-    int count = 0;
-    for (int l = 0; l < nl; l++) {
-        const long long base = __shfl_sync(0xffffffffu, lid, l) * CAPL;
-        const int nn = __shfl_sync(0xffffffffu, n, l);
-        for (int e0 = 0; e0 < nn; e0 += 32) {
-            const bool in = e0 + lane < nn && lists.top_s[base + e0 + lane] >= thr;
-            const unsigned m = __ballot_sync(0xffffffffu, in);
-            const int pos = count + __popc(m & ((1u << lane) - 1));
-            if (in && pos < kMaxCand) sm.cand[pos] = lists.top_i[base + e0 + lane];
-            count += __popc(m);
-        }
-    }
-    if (count > kMaxCand) return leave();
-    __syncwarp();
-    if (count == 1) {
-        // no other atom can win (|s| > 0: it is above the bound)
-        if (lane == 0) keys[v] = pack_key(best, (unsigned)sm.cand[0]);
-        return;
-    }
     const float2 *x = img + v * img_stride;
     const float2 *d0 = atoms + (long long)bin * bin_natoms * atom_stride;
     // lanes per row and copy, rows per copy instruction
     constexpr int N = VEC ? 2 : 1, LPR = kSteps / N, RPI = 32 / LPR;
     const int steps = (nreps + kSteps - 1) / kSteps, sub = lane % LPR * N, which = lane / LPR;
     float bs = 0.f;
-    int bi = -1;
-    for (int c0 = 0; c0 < count; c0 += kBatch) {
-        const int nb = min(kBatch, count - c0);
-        const float2 *row[kBatch / RPI];
-#pragma unroll
-        for (int q = 0; q < kBatch / RPI; q++)
-            row[q] = d0 + (long long)sm.cand[min(c0 + RPI * q + which, count - 1)] * atom_stride;
-        auto stage = [&](int s) {
-            if (s < steps) {
-                const int t = s * kSteps + sub, b = s % kDepth;
-                const int have = max(0, min(N, nreps - t)), at = have ? t : 0;
-                if (which == 0) copy_samples<N>(&sm.x[b][sub], x + at, have);
-#pragma unroll
-                for (int q = 0; q < kBatch / RPI; q++)
-                    if (RPI * q < nb) copy_samples<N>(&sm.d[b][RPI * q + which][sub], row[q] + at, have);
+    int bi = -1, seen = 0, l = 0, e0 = 0;
+    do {
+        // the next candidates (WIDE: this warp's), until the buffer has no room for 32 more
+        int count = 0;
+        while (l < nl && count <= kMaxCand - 32) {
+            const long long base = __shfl_sync(0xffffffffu, lbase, l) + e0;
+            const int left = __shfl_sync(0xffffffffu, n, l) - e0;
+            const bool in = lane < left && lists.top_s[base + lane] >= thr;
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            const int rank = seen + __popc(m & ((1u << lane) - 1));
+            const bool mine = in && (!WIDE || rank / kBatch % kRescoreWarps == warp);
+            const unsigned mm = __ballot_sync(0xffffffffu, mine);
+            if (mine) sm.cand[count + __popc(mm & ((1u << lane) - 1))] = lists.top_i[base + lane];
+            seen += __popc(m);
+            count += __popc(mm);
+            e0 += 32;
+            if (left <= 32) {
+                l++;
+                e0 = 0;
             }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        };
-        for (int s = 0; s < kDepth - 1; s++) stage(s);
-        // IMAG: both sums of candidate c on lane c.  Complex (four FMAs per
-        // sample): Re s on lane c, Im s on lane c + kBatch.
-        static_assert(kBatch == 16 && kSteps == 16, "half a warp each");
-        const bool im = !IMAG && lane >= kBatch;
-        float acc = 0.f, acc2 = 0.f;
-        for (int s = 0; s < steps; s++) {
-            stage(s + kDepth - 1);
-            asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");
-            __syncwarp();
-            if (!IMAG) {
-                if (!im) {
-                    const float2 v = sm.x[s % kDepth][lane];
-                    sm.xi[lane] = make_float2(v.y, -v.x);
+        }
+        __syncwarp();
+        if (seen == 1 && l == nl) {
+            // no other atom can win (|s| > 0: it is above the bound)
+            if (first_warp && lane == 0) keys[v] = pack_key(best, (unsigned)sm.cand[0]);
+            return;
+        }
+        for (int c0 = 0; c0 < count; c0 += kBatch) {
+            const int nb = min(kBatch, count - c0);
+            const float2 *row[kBatch / RPI];
+#pragma unroll
+            for (int q = 0; q < kBatch / RPI; q++)
+                row[q] = d0 + (long long)sm.cand[min(c0 + RPI * q + which, count - 1)] * atom_stride;
+            auto stage = [&](int s) {
+                if (s < steps) {
+                    const int t = s * kSteps + sub, b = s % kDepth;
+                    const int have = max(0, min(N, nreps - t)), at = have ? t : 0;
+                    if (which == 0) copy_samples<N>(&sm.x[b][sub], x + at, have);
+#pragma unroll
+                    for (int q = 0; q < kBatch / RPI; q++)
+                        if (RPI * q < nb) copy_samples<N>(&sm.d[b][RPI * q + which][sub], row[q] + at, have);
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            };
+            for (int s = 0; s < kDepth - 1; s++) stage(s);
+            // IMAG: both sums of candidate c on lane c.  Complex (four FMAs per
+            // sample): Re s on lane c, Im s on lane c + kBatch.
+            static_assert(kBatch == 16 && kSteps == 16, "half a warp each");
+            const bool im = !IMAG && lane >= kBatch;
+            float acc = 0.f, acc2 = 0.f;
+            for (int s = 0; s < steps; s++) {
+                stage(s + kDepth - 1);
+                asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");
+                __syncwarp();
+                if (!IMAG) {
+                    if (!im) {
+                        const float2 v = sm.x[s % kDepth][lane];
+                        sm.xi[lane] = make_float2(v.y, -v.x);
+                    }
+                    __syncwarp();
+                }
+                const float4 *dr = reinterpret_cast<const float4 *>(sm.d[s % kDepth][lane % kBatch]);
+                const float4 *xr = reinterpret_cast<const float4 *>(im ? sm.xi : sm.x[s % kDepth]);
+                if ((IMAG ? lane : lane % kBatch) < nb) {
+                    // (samples past nreps are zeros: their products add exact zeros)
+#pragma unroll
+                    for (int u = 0; u < kSteps / 2; u++) {
+                        const float4 d = dr[u], v = xr[u];
+                        if (IMAG) {
+                            acc = fmaf(d.y, v.y, acc);
+                            acc2 = fmaf(-d.y, v.x, acc2);
+                            acc = fmaf(d.w, v.w, acc);
+                            acc2 = fmaf(-d.w, v.z, acc2);
+                        } else {
+                            acc = fmaf(d.x, v.x, acc);
+                            acc = fmaf(d.y, v.y, acc);
+                            acc = fmaf(d.z, v.z, acc);
+                            acc = fmaf(d.w, v.w, acc);
+                        }
+                    }
                 }
                 __syncwarp();
             }
-            const float4 *dr = reinterpret_cast<const float4 *>(sm.d[s % kDepth][lane % kBatch]);
-            const float4 *xr = reinterpret_cast<const float4 *>(im ? sm.xi : sm.x[s % kDepth]);
-            if ((IMAG ? lane : lane % kBatch) < nb) {
-                // (samples past nreps are zeros: their products add exact zeros)
-#pragma unroll
-                for (int u = 0; u < kSteps / 2; u++) {
-                    const float4 d = dr[u], v = xr[u];
-                    if (IMAG) {
-                        acc = fmaf(d.y, v.y, acc);
-                        acc2 = fmaf(-d.y, v.x, acc2);
-                        acc = fmaf(d.w, v.w, acc);
-                        acc2 = fmaf(-d.w, v.z, acc2);
-                    } else {
-                        acc = fmaf(d.x, v.x, acc);
-                        acc = fmaf(d.y, v.y, acc);
-                        acc = fmaf(d.z, v.z, acc);
-                        acc = fmaf(d.w, v.w, acc);
-                    }
-                }
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            const float ar = acc, ai = IMAG ? acc2 : __shfl_down_sync(0xffffffffu, acc, kBatch);
+            const float sc = ar * ar + ai * ai;
+            if (lane < nb && sc > 0.f && beats(sc, sm.cand[c0 + lane], bs, bi)) {
+                bs = sc;
+                bi = sm.cand[c0 + lane];
             }
-            __syncwarp();
         }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        const float ar = acc, ai = IMAG ? acc2 : __shfl_down_sync(0xffffffffu, acc, kBatch);
-        const float sc = ar * ar + ai * ai;
-        if (lane < nb && sc > 0.f && beats(sc, sm.cand[c0 + lane], bs, bi)) {
-            bs = sc;
-            bi = sm.cand[c0 + lane];
-        }
-    }
+        __syncwarp();
+    } while (l < nl);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float os = __shfl_xor_sync(0xffffffffu, bs, o);
@@ -449,6 +466,19 @@ rescore_kernel(unsigned long long *keys, tc::Lists lists, const int *list_n, con
             bs = os;
             bi = oi;
         }
+    }
+    if (WIDE) {
+        if (lane == 0) {
+            wide_s[warp] = bs;
+            wide_i[warp] = bi;
+        }
+        __syncthreads();
+        if (threadIdx.x != 0) return;
+        for (int w = 1; w < kRescoreWarps; w++)
+            if (beats(wide_s[w], wide_i[w], bs, bi)) {
+                bs = wide_s[w];
+                bi = wide_i[w];
+            }
     }
     if (lane == 0 && bi >= 0) keys[v] = pack_key(bs, (unsigned)bi);
 }
@@ -495,15 +525,30 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
     const long long row_bytes = rows * Kp * 2, fit = std::max<long long>(apt, (long long)kAtomBytes / row_bytes);
     const int bins_per = (int)std::min<long long>(nbins, std::max(1ll, fit / bin_natoms));
     const long long chunk = bin_natoms <= fit ? bin_natoms : fit / apt * apt;
-    // voxels per pass
-    const long long nv_fit = std::max<long long>(vt, (long long)kVoxelBytes / ((q.imag ? 2 : 1) * Kp * 2));
+    // Entries per list: the atoms within the bound grow in number with the
+    // grid's density (T = 1000, imaginary / complex, mean and most of 512
+    // voxels: 6,938 atoms 9, 27 / 17, 49; 41,588 51, 153 / 99, 294; 164,551
+    // 201, 599 / 390, 1,169; 334,125 408, 1,214 / 793, 2,364), over four / two
+    // lists.  Full lists send the voxel to the FP32 kernel after the screen:
+    // 4,096 voxels, 164,551 atoms 58.2 / 111 ms by that kernel alone, 63.4 /
+    // 121 with lists for 64 entries, 5.9 / 11.5 with these.
+    const int nlists = tc::split_lists(q.imag);
+    int list_cap = 64;
+    while (list_cap < 2048 && list_cap * 256ll < bin_natoms) list_cap *= 2;
+    const long long split_list = tc::split_entries(list_cap) * nlists * 8;  // bytes of a split slot's lists
+    int num_sms = 0, dev = 0;
+    SNAPMRF_CUDA(cudaGetDevice(&dev));
+    SNAPMRF_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
+    // voxels per pass (at most num_sms - 1 items of vt voxels are split)
+    const long long own_list = (long long)nlists * list_cap * 8, list_room = (long long)kListBytes;
+    const long long nv_lists = std::max(list_room / (own_list + split_list),
+                                        (list_room - (num_sms - 1) * vt * split_list) / own_list);
+    const long long nv_fit =
+        std::max<long long>(vt, std::min((long long)kVoxelBytes / ((q.imag ? 2 : 1) * Kp * 2), nv_lists));
     const long long nv_max = std::min(q.nvox, nv_fit);
     const long long cap = ((nv_max + vt - 1) / vt + nbins) * vt;
     const long long arows = (q.imag ? 2 : 1) * cap, brows = rows * chunk * bins_per;
     if (arows > 0x7fffffffll || brows > 0x7fffffffll) return SNAPMRF_OK;
-    int num_sms = 0, dev = 0;
-    SNAPMRF_CUDA(cudaGetDevice(&dev));
-    SNAPMRF_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
     const long long lslots = cap + tc::split_slots(cap / vt, num_sms) * vt;
 
     size_t bytes = 0;
@@ -513,7 +558,9 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
         return off;
     };
     const size_t oA = take((size_t)arows * Kp * 2), oB = take((size_t)brows * Kp * 2);
-    const size_t lb = (size_t)lslots * tc::LIST_CAP * 4, hb = (size_t)lslots * tc::split_lists(q.imag) * 4;
+    const size_t lb = (size_t)cap * nlists * list_cap * 4 +
+                      (size_t)std::min<long long>(cap / vt, num_sms - 1) * vt * split_list / 2;
+    const size_t hb = (size_t)lslots * nlists * 4;
     const size_t oTs = take(lb), oTi = take(lb), oLn = take(hb), oLb = take(hb), oPlan = take(sizeof(tc::TailPlan));
     const size_t oKey = take((size_t)nv_max * 8);
     const size_t oPerm = take((size_t)cap * 8), oFperm = take((size_t)nv_max * 8), oFall = take((size_t)nv_max * 4);
@@ -589,6 +636,7 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
         a.top_s = reinterpret_cast<float *>(b + oTs);
         a.top_i = reinterpret_cast<int *>(b + oTi);
         a.plan = reinterpret_cast<tc::TailPlan *>(b + oPlan);
+        a.list_cap = list_cap;
         a.chain = chain;
         a.atom_stats = &state->atoms;
         a.vox_stats = vstats;
@@ -603,8 +651,15 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
         lists.plan = a.plan;
         lists.cap = cap;
         lists.vt = vt;
-        auto rk = q.imag ? (avec && ivec ? rescore_kernel<true, true> : rescore_kernel<true, false>)
-                         : (avec && ivec ? rescore_kernel<false, true> : rescore_kernel<false, false>);
+        // (long lists are of fine grids: batch after batch per voxel)
+        const bool wide = list_cap > 64;
+        auto pick = [&](auto vec_wide, auto vec, auto wd, auto plain) {
+            return avec && ivec ? (wide ? vec_wide : vec) : (wide ? wd : plain);
+        };
+        auto rk = q.imag ? pick(rescore_kernel<true, true, true>, rescore_kernel<true, true, false>,
+                                rescore_kernel<true, false, true>, rescore_kernel<true, false, false>)
+                         : pick(rescore_kernel<false, true, true>, rescore_kernel<false, true, false>,
+                                rescore_kernel<false, false, true>, rescore_kernel<false, false, false>);
         for (int b0 = 0; b0 < nbins; b0 += bins_per) {
             const int nb = std::min(bins_per, nbins - b0);
             for (long long a0 = 0; a0 < bin_natoms; a0 += chunk) {
@@ -624,8 +679,8 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
                 if (rc) return rc;
             }
             // (the next bins' launch uses the split items' lists again)
-            rk<<<nblk(cap, kRescoreWarps), kRescoreWarps * 32, 0, st>>>(
-                keys, lists, a.list_n, a.list_best, perm, vstats, tile_start, b0, b0 + nb, b1 ? vox_bin : nullptr,
+            rk<<<nblk(cap, wide ? 1 : kRescoreWarps), kRescoreWarps * 32, 0, st>>>(
+                keys, lists, list_cap, a.list_n, a.list_best, perm, vstats, tile_start, b0, b0 + nb, b1 ? vox_bin : nullptr,
                 q.atoms, q.atom_stride, img, q.img_stride, (int)q.nreps, bin_natoms, chain, state, fall, fall_counts);
             SNAPMRF_LAUNCH_CHECK();
         }

@@ -325,11 +325,15 @@ match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             // atom within the margin of the best score seen so far (by the
             // lane pair of a voxel in the IMAG form).  An atom left out is
             // certain to lose to the one that set that best.
-            constexpr int LISTS = split_lists(IMAG), CAPL = LIST_CAP / LISTS;
+            constexpr int LISTS = split_lists(IMAG);
             const long long lid = slot * LISTS + (IMAG ? 2 * half + (lane & 1) : half);
-            int ln = 0;
+            long long lbase = 0;
+            int ln = 0, lcap = 0;
             float best = 0.f, keep = 0.f, margin = 0.f;
             if constexpr (SPLIT) {
+                const int parts = u.step;
+                lbase = list_offset(lid, p.cap * LISTS, p.list_cap, parts);
+                lcap = part_cap(p.list_cap, parts);
                 margin = screen_margin(*p.atom_stats,
                                        p.vox_stats[(item0 + u.item) * VPT + (IMAG ? row / 2 : row)], p.chain);
                 if (p.resume) {
@@ -412,28 +416,43 @@ match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                             const float low = sqrtf(best) - margin;
                             keep = low > 0.f ? low * low * (1.f - 0x1p-20f) : 0.f;
                         }
-                        if (mx >= keep && mx > 0.f) {
-                            float *ls = p.top_s + lid * CAPL;
-                            int *li = p.top_i + lid * CAPL;
+                        const bool some = mx >= keep && mx > 0.f;
+                        if (!__any_sync(0xffffffffu, some)) continue;
+                        // A list without room for 16 more: the warp drops the
+                        // entries that its best has left behind; fewer than a
+                        // quarter, and the voxel has too many (the next such
+                        // pass would come too soon).
+                        __syncwarp();
+                        for (unsigned full = __ballot_sync(0xffffffffu, some && ln <= lcap && ln + 16 > lcap); full;
+                             full &= full - 1) {
+                            const int src = __ffs(full) - 1;
+                            const long long base = __shfl_sync(0xffffffffu, lbase, src);
+                            const int n = __shfl_sync(0xffffffffu, ln, src);
+                            const float least = __shfl_sync(0xffffffffu, keep, src);
+                            int k = 0;
+                            for (int e0 = 0; e0 < n; e0 += 32) {
+                                const bool in = e0 + lane < n;
+                                const float s = in ? p.top_s[base + e0 + lane] : 0.f;
+                                const int i = in ? p.top_i[base + e0 + lane] : 0;
+                                const bool stays = in && s >= least;
+                                const unsigned m = __ballot_sync(0xffffffffu, stays);
+                                __syncwarp();
+                                if (stays) {
+                                    const int at = k + __popc(m & ((1u << lane) - 1));
+                                    p.top_s[base + at] = s;
+                                    p.top_i[base + at] = i;
+                                }
+                                k += __popc(m);
+                                __syncwarp();
+                            }
+                            if (lane == src) ln = 4 * k <= 3 * lcap ? k : LIST_OVER;
+                        }
+                        if (some && ln <= lcap) {
 #pragma unroll
                             for (int j = 0; j < 16; j++) {
-                                if (!(sc[j] >= keep && sc[j] > 0.f) || ln > CAPL) continue;
-                                if (ln == CAPL) {
-                                    // full: entries that the best has left
-                                    // behind go; none left to go: overflow
-                                    int k = 0;
-                                    for (int e = 0; e < CAPL; e++) {
-                                        const float s = ls[e];
-                                        if (s >= keep) {
-                                            ls[k] = s;
-                                            li[k++] = li[e];
-                                        }
-                                    }
-                                    ln = k < CAPL ? k : CAPL + 1;
-                                    if (ln > CAPL) continue;
-                                }
-                                ls[ln] = sc[j];
-                                li[ln++] = a0 + j;
+                                if (!(sc[j] >= keep && sc[j] > 0.f)) continue;
+                                p.top_s[lbase + ln] = sc[j];
+                                p.top_i[lbase + ln++] = a0 + j;
                             }
                         }
                         continue;

@@ -68,19 +68,19 @@ struct Args {
     uint32_t idesc;               // tcgen05 instruction descriptor
     const float *ascale2;         // E4M3: [NATOMS] 1 / (atom scale)^2
     long long cap;                // voxel slots; the split items' lists start there
-    float *top_s;                 // [slots][NLISTS][TOPK_MAX]; SPLIT: [slots][LIST_CAP]
+    float *top_s;                 // [slots][NLISTS][TOPK_MAX]; SPLIT: lists at list_offset
     int *top_i;
     int *err;
-    // SPLIT: candidates within screen_margin of the best score, LIST_CAP per
-    // slot shared by its split_lists lists
+    // SPLIT: candidates within screen_margin of the best score
+    int list_cap;                 // entries per list
     float chain;                  // see screen_margin
     const AtomStats *atom_stats;  // of the atoms packed so far
     const VoxelStats *vox_stats;  // [slots]
-    int *list_n;                  // [slots][lists] entries, more than the list holds: overflow
+    int *list_n;                  // [slots][lists] entries, LIST_OVER: more than the list holds
     float *list_best;             // [slots][lists] the best score the list's thread has seen
     int resume;                   // the lists continue those of an earlier launch (atom0 > 0)
 };
-constexpr int LIST_CAP = 128;     // SPLIT: candidates per voxel slot
+constexpr int LIST_OVER = 1 << 30;
 // SPLIT: lists per voxel slot (one per epilogue thread of the voxel)
 __host__ __device__ constexpr int split_lists(bool imag) { return imag ? 4 : 2; }
 
@@ -171,6 +171,26 @@ __device__ __forceinline__ ListSlots list_slots(const Lists &l, long long slot) 
     const long long item = slot / l.vt - t.item0;
     if (item < t.bulk || t.parts == 1) return {slot, 1};
     return {l.cap + (item - t.bulk) * t.parts * l.vt + slot % l.vt, t.parts};
+}
+
+// SPLIT: entries of a list of an item in `parts` parts.  A part sees every
+// parts-th tile; near atoms share tiles, so its share may be twice the average.
+__host__ __device__ inline int part_cap(int cap, int parts) {
+    if (parts == 1) return cap;
+    const int share = (2 * cap / parts + 31) / 32 * 32;
+    return share > 64 ? share : 64;
+}
+// Where list `lid` (list slot x lists + list) begins: the slots' own lists
+// first (`own` of them), then those of the split items.
+__device__ __forceinline__ long long list_offset(long long lid, long long own, int cap, int parts) {
+    return lid < own ? lid * cap : own * cap + (lid - own) * part_cap(cap, parts);
+}
+// Entries of one of a split voxel slot's lists over its parts, at most.
+inline long long split_entries(int cap) {
+    long long most = 0;
+    for (int parts = 2; parts <= MAX_PARTS; parts++)
+        most = std::max(most, (long long)parts * part_cap(cap, parts));
+    return most;
 }
 
 inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }

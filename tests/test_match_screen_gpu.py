@@ -189,3 +189,20 @@ def test_blocks_without_voxels_are_not_looked_at(snap, imag):
     for got in (a, b, want[0]):
         np.testing.assert_array_equal(got[1], want[1][1])
         np.testing.assert_array_equal(got[0], want[1][0])
+
+
+@pytest.mark.parametrize("imag", [True, False])
+@pytest.mark.parametrize("nvox,natoms,smooth", [(300, 40000, 4000.0), (70, 70000, 20000.0), (2000, 17000, 600.0),
+                                                (100, 17000, 0.0)])
+def test_long_lists(snap, imag, nvox, natoms, smooth):
+    """Lists that grow with the dictionary, are compacted or overflow, and are
+    rescored by several warps per voxel (0: all atoms the same, the first wins)."""
+    if smooth:
+        atoms, img, params = _inputs(nvox, natoms, 110, 1, imag, seed=natoms, smooth=smooth)
+    else:
+        atoms, img, params = _inputs(nvox, 50, 110, 1, imag, seed=9)
+        atoms = np.repeat(atoms[7:8], natoms, 0)
+        params = np.random.default_rng(1).uniform(1, 100, (natoms, 4)).astype(np.float32)
+    a, b = _both(snap, img, atoms, params, 110, natoms, None, imag)
+    np.testing.assert_array_equal(a[1], b[1])
+    np.testing.assert_array_equal(a[0], b[0])
