@@ -46,6 +46,8 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdio>
+#include <cstdlib>
 
 #include "common.h"
 #define SNAPMRF_MATCH_KERNEL_DECLARATION_ONLY
@@ -77,11 +79,10 @@ constexpr float kMinAtom2 = 1e-18f;  // (and of all atoms: the squares of their 
 constexpr float kMaxNorm2 = 1e30f;
 // Operand memory of one pass: larger dictionaries are screened in chunks of
 // atoms, larger images in ranges of voxels.
-constexpr size_t kAtomBytes = 2ull << 30, kVoxelBytes = 1ull << 30;
-constexpr size_t kListBytes = 1ull << 30;  // and of the candidates' lists
+constexpr long long kAtomBytes = 2ll << 30, kVoxelBytes = 1ll << 30;
+constexpr long long kListBytes = 1ll << 30;  // and of the candidates' lists
 
 struct State {
-    int err;                 // error word of the scoring kernel, or 7
     int bad_atoms;           // an atom is not finite or out of range: the FP32 kernel takes every voxel
     int nfall;               // voxels left to the FP32 kernel
     tc::AtomStats atoms;
@@ -93,7 +94,7 @@ __global__ void init_kernel(unsigned long long *keys, long long nkeys, long long
     if (i < nkeys) keys[i] = 0ull;
     if (i < nperm) perm[i] = -1;
     if (i < nbins) counts[i] = fall_counts[i] = 0;
-    if (i == 0) *st = State{0, 0, 0, {0u, 0u, 0u, 0u}};
+    if (i == 0) *st = State{0, 0, {0u, 0u, 0u, 0u}};
 }
 
 // Running sums of a row (see tc::AtomStats).
@@ -221,7 +222,7 @@ __global__ void pack_voxels_kernel(__nv_bfloat16 *A, tc::VoxelStats *stats, cons
 template <bool IMAG, bool VEC>
 __global__ void pack_atoms_kernel(__nv_bfloat16 *B, const float2 *atoms, long long atom_stride, long long n,
                                   long long nreps, long long Kp, const long long *tile_start, int bin_lo,
-                                  long long per_bin, State *st) {
+                                  long long per_bin, State *st, int *err) {
     const long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
     const int bin = bin_lo + (int)(min(r, n - 1) / per_bin);
@@ -264,7 +265,7 @@ __global__ void pack_atoms_kernel(__nv_bfloat16 *B, const float2 *atoms, long lo
     }
     sums = {warp_sum(sums.norm2), warp_sum(sums.weighted2), warp_sum(sums.lo2), warp_sum(sums.rest2)};
     bad |= !(sums.norm2 <= kMaxNorm2);
-    if (IMAG && __any_sync(0xffffffffu, real_part) && lane == 0) atomicCAS(&st->err, 0, 7);
+    if (IMAG && __any_sync(0xffffffffu, real_part) && lane == 0) atomicCAS(err, 0, 7);
     if (__any_sync(0xffffffffu, bad)) {
         sums = RowSums();
         if (lane == 0) atomicExch(&st->bad_atoms, 1);
@@ -521,8 +522,19 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
     const int vt = q.imag ? tc::BM / 2 : tc::BM, apt = q.imag ? tc::BN : tc::BA, rows = q.imag ? 1 : 2;
     const long long K = (q.imag ? 1 : 2) * q.nreps, nk = (K + KB - 1) / KB, Kp = nk * 2 * KB;
     if (Kp > 0x7fffffffll / 4) return SNAPMRF_OK;
+    // SNAPMRF_SCREEN_PASS="atoms,voxels,lists" (bytes) overrides the pass
+    // sizes, so that tests reach several passes with small inputs
+    long long atom_bytes = kAtomBytes, voxel_bytes = kVoxelBytes, list_room = kListBytes;
+    if (const char *e = getenv("SNAPMRF_SCREEN_PASS")) {
+        long long pa = 0, pv = 0, pl = 0;
+        if (sscanf(e, "%lld,%lld,%lld", &pa, &pv, &pl) == 3 && pa > 0 && pv > 0 && pl > 0) {
+            atom_bytes = pa;
+            voxel_bytes = pv;
+            list_room = pl;
+        }
+    }
     // atoms per pass: whole bins, or a chunk of one bin's tiles
-    const long long row_bytes = rows * Kp * 2, fit = std::max<long long>(apt, (long long)kAtomBytes / row_bytes);
+    const long long row_bytes = rows * Kp * 2, fit = std::max<long long>(apt, atom_bytes / row_bytes);
     const int bins_per = (int)std::min<long long>(nbins, std::max(1ll, fit / bin_natoms));
     const long long chunk = bin_natoms <= fit ? bin_natoms : fit / apt * apt;
     // Entries per list: the atoms within the bound grow in number with the
@@ -540,11 +552,11 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
     SNAPMRF_CUDA(cudaGetDevice(&dev));
     SNAPMRF_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
     // voxels per pass (at most num_sms - 1 items of vt voxels are split)
-    const long long own_list = (long long)nlists * list_cap * 8, list_room = (long long)kListBytes;
+    const long long own_list = (long long)nlists * list_cap * 8;
     const long long nv_lists = std::max(list_room / (own_list + split_list),
                                         (list_room - (num_sms - 1) * vt * split_list) / own_list);
     const long long nv_fit =
-        std::max<long long>(vt, std::min((long long)kVoxelBytes / ((q.imag ? 2 : 1) * Kp * 2), nv_lists));
+        std::max<long long>(vt, std::min(voxel_bytes / ((q.imag ? 2 : 1) * Kp * 2), nv_lists));
     const long long nv_max = std::min(q.nvox, nv_fit);
     const long long cap = ((nv_max + vt - 1) / vt + nbins) * vt;
     const long long arows = (q.imag ? 2 : 1) * cap, brows = rows * chunk * bins_per;
@@ -565,7 +577,7 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
     const size_t oKey = take((size_t)nv_max * 8);
     const size_t oPerm = take((size_t)cap * 8), oFperm = take((size_t)nv_max * 8), oFall = take((size_t)nv_max * 4);
     const size_t oVb = take((size_t)nv_max * 4), oVs = take((size_t)cap * sizeof(tc::VoxelStats));
-    const size_t oBin = take(5 * (size_t)(nbins + 1) * 8), oCnt = take(2 * (size_t)nbins * 4), oSt = take(sizeof(State));
+    const size_t oBin = take(5 * (size_t)(nbins + 1) * 8), oCnt = take(2 * (size_t)nbins * 4), oSt = take(sizeof(State)), oErr = take(4);
     DeviceScratch s;
     const cudaError_t ae = s.alloc(bytes, st);
     if (ae == cudaErrorMemoryAllocation) {
@@ -584,7 +596,9 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
     long long *fslot = cursor + nbins + 1, *ftile = fslot + nbins + 1, *fcursor = ftile + nbins + 1;
     int *counts = reinterpret_cast<int *>(b + oCnt), *fall_counts = counts + nbins;
     State *state = reinterpret_cast<State *>(b + oSt);
+    int *err = reinterpret_cast<int *>(b + oErr);  // of the whole call: a wait that ran out, or 7
     *done = true;
+    SNAPMRF_CUDA(cudaMemsetAsync(err, 0, 4, st));
 
     const float chain = 92.f * 0x1p-24f * (1.f + (float)K * 0x1p-22f);
     auto aligned = [](const void *p, long long stride) {
@@ -642,7 +656,7 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
         a.vox_stats = vstats;
         a.list_n = reinterpret_cast<int *>(b + oLn);
         a.list_best = reinterpret_cast<float *>(b + oLb);
-        a.err = &state->err;
+        a.err = err;
         auto pa = q.imag ? (avec ? pack_atoms_kernel<true, true> : pack_atoms_kernel<true, false>)
                          : (avec ? pack_atoms_kernel<false, true> : pack_atoms_kernel<false, false>);
         tc::Lists lists;
@@ -667,7 +681,7 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
                 const long long ca = std::min(chunk, bin_natoms - a0);
                 const long long na = nb * ca;
                 pa<<<nblk(na * 32, 256), 256, 0, st>>>(B, q.atoms + (b0 * bin_natoms + a0) * q.atom_stride,
-                                                       q.atom_stride, na, q.nreps, Kp, tile_start, b0, ca, state);
+                                                       q.atom_stride, na, q.nreps, Kp, tile_start, b0, ca, state, err);
                 SNAPMRF_LAUNCH_CHECK();
                 sl.brows = rows * na;
                 a.bin_lo = b0;
@@ -705,18 +719,16 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
         m.perm_mod = 0;
         m.atiles_per_split = 0;
         SNAPMRF_CUDA(launch_match_fp32(m, dim3(2 * num_sms), q.imag, st));
-        float *maps = q.maps + v0 * 5;
-        long long *index = q.index_out ? q.index_out + v0 : nullptr;
         finalize_maps_kernel<<<nblk(nv * 32, 256), 256, 0, st>>>(
-            maps, index, keys, nullptr, b1 ? vox_bin : nullptr, q.atoms, q.atom_stride, img, q.img_stride, q.nreps,
-            q.params, q.nparams, bin_natoms, nv);
-        SNAPMRF_LAUNCH_CHECK();
-        // a timed-out wait or an atom with a real part: NaN maps, indices -1
-        poison_maps_kernel<<<nblk(nv, 256), 256, 0, st>>>(maps, index, nv, &state->err);
-        SNAPMRF_LAUNCH_CHECK();
-        tc::publish_error_kernel<<<1, 1, 0, st>>>(&state->err);
+            q.maps + v0 * 5, q.index_out ? q.index_out + v0 : nullptr, keys, nullptr, b1 ? vox_bin : nullptr, q.atoms,
+            q.atom_stride, img, q.img_stride, q.nreps, q.params, q.nparams, bin_natoms, nv);
         SNAPMRF_LAUNCH_CHECK();
     }
+    // a timed-out wait or an atom with a real part: NaN maps, indices -1
+    poison_maps_kernel<<<nblk(q.nvox, 256), 256, 0, st>>>(q.maps, q.index_out, q.nvox, err);
+    SNAPMRF_LAUNCH_CHECK();
+    tc::publish_error_kernel<<<1, 1, 0, st>>>(err);
+    SNAPMRF_LAUNCH_CHECK();
     return SNAPMRF_OK;
 }
 

@@ -206,3 +206,78 @@ def test_long_lists(snap, imag, nvox, natoms, smooth):
     a, b = _both(snap, img, atoms, params, 110, natoms, None, imag)
     np.testing.assert_array_equal(a[1], b[1])
     np.testing.assert_array_equal(a[0], b[0])
+
+
+def _row_bytes(T, imag):
+    """Operand bytes of an atom and of a voxel: 32 elements in 128 bytes."""
+    chunks = ((1 if imag else 2) * T + 31) // 32
+    return (1 if imag else 2) * chunks * 128, (2 if imag else 1) * chunks * 128
+
+
+@pytest.mark.parametrize("imag", [True, False])
+@pytest.mark.parametrize("nb,natoms,per_atoms,per_voxels,lists", [
+    (5, 700, 1500, 1 << 20, 1 << 30),     # two blocks per pass, the last alone
+    (3, 700, 300, 1 << 20, 1 << 30),      # a block in chunks of 256, the last short
+    (1, 3000, 600, 500, 1 << 30),         # chunks, and five ranges of voxels
+    (4, 700, 100000, 500, 1 << 30),       # ranges of voxels alone
+    (1, 3000, 600, 100000, 1 << 23)])     # ranges from the lists' room
+def test_passes(snap, monkeypatch, imag, nb, natoms, per_atoms, per_voxels, lists):
+    """Dictionaries, images and lists larger than one pass: atom norms that
+    rise and fall from chunk to chunk, blocks with and without voxels."""
+    T, nvox = 130, 2100
+    atoms, img, params = _inputs(nvox, natoms, T, nb, imag, seed=natoms + nb)
+    atoms = (atoms * np.float32(10.0) ** np.linspace(-1, 1, len(atoms), dtype=np.float32)[:, None]).astype(np.complex64)
+    atoms[len(atoms) // 2:] = atoms[:len(atoms) // 2 - 1:-1].copy()
+    b1map = None
+    if nb > 1:
+        b1map = np.random.default_rng(3).choice(np.float32(0.8 + 0.1 * np.arange(1, nb)), nvox)
+    rb = _row_bytes(T, imag)
+    monkeypatch.setenv("SNAPMRF_SCREEN_PASS", f"{per_atoms * rb[0]},{per_voxels * rb[1]},{lists}")
+    a, b = _both(snap, img, atoms, params, T, natoms, b1map, imag)
+    np.testing.assert_array_equal(a[1], b[1])
+    np.testing.assert_array_equal(a[0], b[0])
+
+
+@pytest.mark.parametrize("imag", [True, False])
+@pytest.mark.parametrize("smooth", [20000.0, 2000.0])
+def test_lists_across_chunks(snap, monkeypatch, imag, smooth):
+    """Near ties in every chunk of a block: lists that go on from launch to
+    launch, fill up and overflow."""
+    T = 120
+    atoms, img, params = _inputs(300, 20000, T, 1, imag, seed=8, smooth=smooth)
+    monkeypatch.setenv("SNAPMRF_SCREEN_PASS", f"{3000 * _row_bytes(T, imag)[0]},{1 << 30},{1 << 30}")
+    a, b = _both(snap, img, atoms, params, T, 20000, None, imag)
+    np.testing.assert_array_equal(a[1], b[1])
+    np.testing.assert_array_equal(a[0], b[0])
+
+
+def test_a_real_part_in_any_range_fails_the_whole_call(snap, monkeypatch):
+    """One error for the call, wherever the voxels of the offending block lie."""
+    torch = torch_cuda()
+    T, natoms, nvox = 100, 700, 1500
+    atoms, img, params = _inputs(nvox, natoms, T, 2, True, seed=4)
+    atoms[natoms + 9, 3] += 0.5
+    b1map = np.where(np.arange(nvox) < 1490, 0.8, 0.9).astype(np.float32)
+    monkeypatch.setenv("SNAPMRF_SCREEN_PASS", f"{1 << 30},{400 * _row_bytes(T, True)[1]},{1 << 30}")
+    maps = torch.full((nvox, 5), -3.0, device="cuda")
+    idx = torch.full((nvox,), -9, dtype=torch.int64, device="cuda")
+    snap.MRF_match(maps, torch.from_numpy(img.view(np.float32)).cuda(), torch.from_numpy(atoms.view(np.float32)).cuda(),
+                   torch.from_numpy(params).cuda(), T, T, 2 * natoms, natoms, nvox,
+                   in_b1map=torch.from_numpy(b1map).cuda(), d_index=idx, img_stride=T, flags=snap.MATCH_IMAG_ATOMS)
+    torch.cuda.synchronize()
+    assert snap.device_error(reset=True) == 7
+    assert torch.isnan(maps).all() and (idx == -1).all()
+
+
+@pytest.mark.parametrize("use_map", [True, False])
+def test_host_image_in_two_ranges(snap, use_map):
+    """A host image of five copies: all but the last two chunks' voxels are
+    matched first, as the same image on the device is in one range."""
+    from gpu_util import run_match
+    T, nb, natoms, nvox = 1000, 2, 300, 10500
+    atoms, img, params = _inputs(nvox, natoms, T, nb, True, seed=6)
+    b1map = np.random.default_rng(3).choice(np.float32([0.8, 0.9]), nvox) if use_map else None
+    out = [run_match(snap, img, atoms, params, natoms=natoms, b1map=b1map, device_img=dev, flags=snap.MATCH_IMAG_ATOMS)
+           for dev in (False, True)]
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+    np.testing.assert_array_equal(out[0][0], out[1][0])
