@@ -309,16 +309,23 @@ typedef struct snapmrf_match_opts {
 /* d_maps: out, device [nvoxels][nmaps] (nmaps == 5, nparams == 4)
  * img: [nvoxels][img_stride] complex, host memory when img_on_host != 0.
  * A host image is copied in up to 8 chunks of at least 16 MB on a copy
- * stream of the library (one per host thread and device); the FP32 form
- * matches each chunk as soon as it has arrived, while the next ones are in
- * flight, and the tensor-core forms start once the whole image is there.
+ * stream of the library (one per host thread and device); matching runs in
+ * two ranges of voxels, all but the last two chunks first (small FP32 calls:
+ * chunk by chunk), while later chunks are in flight.
  * Page-locked host memory makes the copies asynchronous: the call then
  * returns before they finish, so keep the host image unchanged until the
  * call's work on `stream` has completed;
  * nreps time points are matched.  Per B1 block the first atom with the
  * largest |<atom, voxel>| wins; blocks are merged by nearest B1 when a B1
  * map is given (ties to the lower block, differences >= 10 to block 0),
- * otherwise by the largest PD (ties to the lower block). */
+ * otherwise by the largest PD (ties to the lower block).
+ * Scratch: the tensor-core forms pack both operands.  FP32 matching does from
+ * 2^24 products on (32 voxels; 96 or 384 against several B1 blocks): nreps
+ * floats per purely imaginary atom, 4 nreps per complex atom, 2 nreps per
+ * voxel, at most 2 GB and 1 GB in a pass, and up to 1 GB of candidate lists.
+ * It comes from the library's pool, which keeps it for the next call
+ * (snapmrf_release_scratch gives it back).  An FP32 call that cannot have it,
+ * or whose tensor-core kernel gives up a wait, is matched without (a few MB). */
 int snapmrf_mrf_match(float *d_maps, const float *img, int img_on_host,
                       const float *d_atoms, const float *d_params, size_t nreps,
                       size_t NATOMS, size_t natoms, size_t nvoxels, int nparams, int nmaps,

@@ -83,18 +83,19 @@ constexpr long long kAtomBytes = 2ll << 30, kVoxelBytes = 1ll << 30;
 constexpr long long kListBytes = 1ll << 30;  // and of the candidates' lists
 
 struct State {
+    int wait_err;            // a bounded wait of the scoring kernel ran out: the FP32 kernel takes every voxel
     int bad_atoms;           // an atom is not finite or out of range: the FP32 kernel takes every voxel
     int nfall;               // voxels left to the FP32 kernel
     tc::AtomStats atoms;
 };
 
 __global__ void init_kernel(unsigned long long *keys, long long nkeys, long long *perm, long long nperm, int *counts,
-                            int *fall_counts, int nbins, State *st) {
+                            int *fall_counts, int nbins, int wait_err, State *st) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i < nkeys) keys[i] = 0ull;
     if (i < nperm) perm[i] = -1;
     if (i < nbins) counts[i] = fall_counts[i] = 0;
-    if (i == 0) *st = State{0, 0, {0u, 0u, 0u, 0u}};
+    if (i == 0) *st = State{wait_err, 0, 0, {0u, 0u, 0u, 0u}};
 }
 
 // Running sums of a row (see tc::AtomStats).
@@ -339,7 +340,7 @@ rescore_kernel(unsigned long long *keys, tc::Lists lists, int list_cap, const in
     };
     const tc::AtomStats as = st->atoms;
     const float norm2 = __uint_as_float(as.norm2);
-    if (vs.norm2 < 0.f || st->bad_atoms || norm2 < kMinAtom2 || norm2 * vs.norm2 > kMaxNorm2) return leave();
+    if (st->wait_err || vs.norm2 < 0.f || st->bad_atoms || norm2 < kMinAtom2 || norm2 * vs.norm2 > kMaxNorm2) return leave();
     // the slot's lists: counts and best scores, one list per lane
     constexpr int LISTS = tc::split_lists(IMAG);
     const tc::ListSlots at = tc::list_slots(lists, slot);
@@ -596,9 +597,11 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
     long long *fslot = cursor + nbins + 1, *ftile = fslot + nbins + 1, *fcursor = ftile + nbins + 1;
     int *counts = reinterpret_cast<int *>(b + oCnt), *fall_counts = counts + nbins;
     State *state = reinterpret_cast<State *>(b + oSt);
-    int *err = reinterpret_cast<int *>(b + oErr);  // of the whole call: a wait that ran out, or 7
+    int *err = reinterpret_cast<int *>(b + oErr);  // 7: an atom with a real part, for the whole call
     *done = true;
     SNAPMRF_CUDA(cudaMemsetAsync(err, 0, 4, st));
+    // (tests: as if a wait of every scoring launch had run out)
+    const int wait_err = getenv("SNAPMRF_SCREEN_WAIT_ERROR") ? 1 : 0;
 
     const float chain = 92.f * 0x1p-24f * (1.f + (float)K * 0x1p-22f);
     auto aligned = [](const void *p, long long stride) {
@@ -612,7 +615,7 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
         const float *b1 = q.b1map ? q.b1map + v0 : nullptr;
         const long long ninit = std::max<long long>(std::max(nv, q.b1map ? cap : 0), nbins);
         init_kernel<<<nblk(ninit, 256), 256, 0, st>>>(keys, nv, perm, q.b1map ? cap : 0, counts, fall_counts, nbins,
-                                                      state);
+                                                      wait_err, state);
         SNAPMRF_LAUNCH_CHECK();
         if (b1) {
             assign_bins_kernel<<<nblk(nv, 256), 256, 0, st>>>(vox_bin, counts, b1, q.params, q.nparams, q.natoms,
@@ -656,7 +659,7 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
         a.vox_stats = vstats;
         a.list_n = reinterpret_cast<int *>(b + oLn);
         a.list_best = reinterpret_cast<float *>(b + oLb);
-        a.err = err;
+        a.err = &state->wait_err;
         auto pa = q.imag ? (avec ? pack_atoms_kernel<true, true> : pack_atoms_kernel<true, false>)
                          : (avec ? pack_atoms_kernel<false, true> : pack_atoms_kernel<false, false>);
         tc::Lists lists;
@@ -724,11 +727,13 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
             q.atom_stride, img, q.img_stride, q.nreps, q.params, q.nparams, bin_natoms, nv);
         SNAPMRF_LAUNCH_CHECK();
     }
-    // a timed-out wait or an atom with a real part: NaN maps, indices -1
-    poison_maps_kernel<<<nblk(q.nvox, 256), 256, 0, st>>>(q.maps, q.index_out, q.nvox, err);
-    SNAPMRF_LAUNCH_CHECK();
-    tc::publish_error_kernel<<<1, 1, 0, st>>>(err);
-    SNAPMRF_LAUNCH_CHECK();
+    if (q.imag) {
+        // an atom with a real part: NaN maps, indices -1, error word 7
+        poison_maps_kernel<<<nblk(q.nvox, 256), 256, 0, st>>>(q.maps, q.index_out, q.nvox, err);
+        SNAPMRF_LAUNCH_CHECK();
+        tc::publish_error_kernel<<<1, 1, 0, st>>>(err);
+        SNAPMRF_LAUNCH_CHECK();
+    }
     return SNAPMRF_OK;
 }
 

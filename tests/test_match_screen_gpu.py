@@ -269,6 +269,15 @@ def test_a_real_part_in_any_range_fails_the_whole_call(snap, monkeypatch):
     assert torch.isnan(maps).all() and (idx == -1).all()
 
 
+@pytest.mark.parametrize("imag", [True, False])
+def test_a_wait_that_runs_out_leaves_the_call_to_the_fp32_kernel(snap, monkeypatch, imag):
+    atoms, img, params = _inputs(700, 1500, 150, 1, imag, seed=3)
+    monkeypatch.setenv("SNAPMRF_SCREEN_WAIT_ERROR", "1")
+    a, b = _both(snap, img, atoms, params, 150, 1500, None, imag)
+    np.testing.assert_array_equal(a[1], b[1])
+    np.testing.assert_array_equal(a[0], b[0])
+
+
 @pytest.mark.parametrize("use_map", [True, False])
 def test_host_image_in_two_ranges(snap, use_map):
     """A host image of five copies: all but the last two chunks' voxels are
