@@ -872,7 +872,9 @@ __global__ void __launch_bounds__(32) adjoint_kernel(AdjArgs a) {
     // reverse sweep, one segment at a time
     Pair3<P> nu;
     pz<P>(nu);
-    float gT1 = 0.f, gT2 = 0.f, gB1 = 0.f;
+    // (each sum takes its steps from the last to the first, and a lane the
+    // steps t = its number mod L, so that no result depends on C)
+    float gT1 = 0.f, gT2 = 0.f, gEa = 0.f, gB1 = 0.f;
     auto back = [&](const Pair3<P> &s, int i) {
         const AdjConst k = sk[i];
         if (a.shift) p_shift_adj<P>(nu, gl, L, w, keep, src_up, src_dn);
@@ -931,8 +933,8 @@ __global__ void __launch_bounds__(32) adjoint_kernel(AdjArgs a) {
                 put_pairs<P>(d + lanes * P, x.m);
                 put_pairs<P>(d + 2 * lanes * P, x.z);
             }
-            const float wr = sk[i].w.z, y = forward(x, sk[i]);
-            if (lane0) gT2 = fmaf(wr, y, gT2);
+            const float y = forward(x, sk[i]);
+            if (lane0) sf[i] = y;
         }
         for (int i = (n - 1) & ~1; i >= 0; i -= 2) {
             Pair3<P> s;
@@ -952,16 +954,17 @@ __global__ void __launch_bounds__(32) adjoint_kernel(AdjArgs a) {
         }
         __syncwarp();
         // the lanes' terms of each step, one step per lane
-        for (int i = gl; i < n; i += L) {
+        for (int i = n - 1 - ((t0 + n - 1 - gl) & (L - 1)); i >= 0; i -= L) {
             float ga = 0.f;
 #pragma unroll
             for (int q = 0; q < L; q++) ga += sga[i * 33 + g * L + q];
             if (active) a.galpha_atoms[at * T + t0 + i] = ga * B1;
             gB1 = fmaf(ga, a.sch.alpha[t0 + i], gB1);
+            gEa = fmaf(sk[i].w.z, sf[i], gEa);
         }
     }
     gT1 = group_sum(gT1, L);
-    gT2 = group_sum(gT2, L);
+    gT2 = group_sum(gT2 + gEa, L);
     gB1 = group_sum(gB1, L);
     if (lane0 && active) {
         a.gparams[at * 3 + 0] = gT1;

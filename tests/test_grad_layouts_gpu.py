@@ -87,3 +87,27 @@ def test_crb_layouts_and_segments(snap, w):
     np.testing.assert_array_equal(loss[:3].cpu().numpy(), ref[0].cpu().numpy())
     if torch.isfinite(ref[1]).all():
         assert (ga / 300 - ref[1]).abs().max() <= 1e-5 * ref[1].abs().max()
+
+
+@pytest.mark.parametrize("n", [3, 2500])
+@pytest.mark.parametrize("w", [7, 20, 50])
+def test_adjoint_does_not_depend_on_the_segments(snap, n, w):
+    """A schedule long enough that the checkpoint interval changes the sweep's
+    segments (16 steps, or more where that would keep too many checkpoints):
+    the same bits from each."""
+    torch = torch_cuda()
+    long = 4000 if n == 3 else 1600
+    h = mrf_schedule(long, seed=w)
+    p = torch.from_numpy(_params(n, w)).cuda()
+    g = torch.randn((n, long, 2), device="cuda", generator=torch.Generator("cuda").manual_seed(w))
+    out = []
+    for every in (0, 1, 40, long):
+        gp, ga = torch.empty((n, 3), device="cuda"), torch.empty(long, device="cuda")
+        sig, per = torch.empty((n, long, 2), device="cuda"), torch.empty((n, long), device="cuda")
+        snap.epg_adjoint(p, h, long, long, n, g, gp, 4, w, "epg_fisp", d_signal=sig, d_grad_alpha=ga,
+                         d_grad_alpha_atoms=per, checkpoint_every=every)
+        out.append((gp, ga, sig, per))
+    assert torch.isfinite(out[0][0]).all()
+    for other in out[1:]:
+        for x, y in zip(out[0], other):
+            assert torch.equal(x, y)
