@@ -483,8 +483,9 @@ __global__ void __launch_bounds__(kGnThreads, P == 5 ? 12 * 32 / kGnThreads : 1)
             const float r1 = 1.f / T1, r2 = 1.f / T2;
             q.E1 = __expf(-tr * r1);
             q.E2 = __expf(-tr * r2);
-            q.r1 = tr * r1 * r1;
-            q.r2 = tr * r2 * r2;
+            // (finite where E has long been 0: 0 times it has to stay 0)
+            q.r1 = fminf(tr * r1 * r1, 1e15f);
+            q.r2 = fminf(tr * r2 * r2, 1e15f);
             q.Ea = __expf(-ta * r2);
             q.dEa = q.Ea * ta * r2 * r2;
             const long long vv = sI[ga];

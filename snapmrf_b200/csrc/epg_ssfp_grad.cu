@@ -345,9 +345,10 @@ __global__ void __launch_bounds__(kThreads) gn_ssfp_kernel(Args a) {
             const float2 ea = b0_phasor(b0, ta), eb = b0_phasor(b0, tb);
             const float2 z = sZ[i], zn = sZ[i + 1];
             q.w = c_scale(c_mul_fma(c_mul_fma(ea, eb), c_mul_conj(zn, z)), E2);
-            q.kappa = tr / (t2 * t2);
+            // (finite where E2 has long been 0: 0 times it has to stay 0)
+            q.kappa = fminf(tr / (t2 * t2), 1e15f);
             q.theta = (float)(2 * M_PI * tr / 1000.0);
-            q.kappa_e = ta / (t2 * t2);
+            q.kappa_e = fminf(ta / (t2 * t2), 1e15f);
             q.theta_e = (float)(2 * M_PI * ta / 1000.0);
             const float2 r = c_scale(c_mul_fma(ea, z), E2a);
             q.R = fmaf(r.x, r.x, r.y * r.y);

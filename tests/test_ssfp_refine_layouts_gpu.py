@@ -52,3 +52,22 @@ def test_layouts_refine_alike(snap, w, use_map):
     truth = np.concatenate([p, np.ones((few, 1), np.float32)], 1)
     assert np.median(np.abs(a[:, :2] / truth[:, :2] - 1)) < 5e-3
     assert np.median(np.abs(a[:, 2] - truth[:, 2])) < 0.2
+
+
+@pytest.mark.parametrize("echo", ["epg_fisp", "epg_ssfp"])
+def test_vanished_t2(snap, echo):
+    """T2 so short that 1 / T2^2 leaves FP32's range, sampled at TE = 0 (there
+    is a signal): its derivative is as 0 as at a T2 of 1e-10 ms."""
+    torch = torch_cuda()
+    T, w = 60, 10
+    r = np.random.default_rng(2)
+    h = np.stack([r.uniform(0.2, 0.9, T), np.zeros(T), np.full(T, 12.0), np.zeros(T)]).astype(np.float32)
+    if echo == "epg_ssfp":
+        h[2:] -= np.float32([[16.0], [3.5]])
+    img = torch.randn((2, T, 2), device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    img[1] = img[0]
+    maps = torch.tensor([[800, 1e-10, 0, 1, 1], [800, 1e-20, 0, 1, 1]], device="cuda")
+    snap.refine_gn(maps, img, h, T, T, 2, w, echo, iterations=1, tol=0.0)
+    maps = maps.cpu().numpy()
+    assert np.isfinite(maps).all()
+    np.testing.assert_array_equal(maps[0], maps[1])
