@@ -815,8 +815,9 @@ __global__ void __launch_bounds__(32) adjoint_kernel(AdjArgs a) {
             if (reverse) {
                 const float ge = active ? Ea * a.gsig[at * T + t].y : 0.f;
                 k.rev2.w = ge;
-                k.w.x = trp / (T1 * T1);
-                k.w.y = trp / (T2 * T2);
+                // (finite where E has long been 0: 0 times it has to stay 0)
+                k.w.x = fminf(trp / (T1 * T1), 1e15f);
+                k.w.y = fminf(trp / (T2 * T2), 1e15f);
                 k.w.z = ge * te / (T2 * T2);
             }
             sk[i] = k;

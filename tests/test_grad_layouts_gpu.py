@@ -111,3 +111,19 @@ def test_adjoint_does_not_depend_on_the_segments(snap, n, w):
     for other in out[1:]:
         for x, y in zip(out[0], other):
             assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("n", [2, 2500])
+def test_adjoint_of_a_vanished_t2(snap, n):
+    """T2 so short that 1 / T2^2 leaves FP32's range: the gradients of a T2 of
+    1e-10 ms, whose decay is as complete."""
+    torch = torch_cuda()
+    h = mrf_schedule(T, seed=1)
+    p = torch.from_numpy(_params(n, 1)).cuda()
+    g = torch.randn((1, T, 2), device="cuda", generator=torch.Generator("cuda").manual_seed(1)).repeat(n, 1, 1)
+    out = []
+    for t2 in (1e-10, 1e-20):
+        p[:, 1] = t2
+        out.append(_adjoint(snap, torch, p, g.contiguous(), h, 20, "epg_fisp"))
+    for x, y in zip(*out):
+        assert torch.isfinite(x).all() and torch.equal(x, y)
