@@ -468,7 +468,11 @@ int snapmrf_mrf_match_noalloc(float *d_maps, const float *d_img, size_t img_stri
  * checkpoint_every: states kept every C steps (0: C = ceil(sqrt(nreps))),
  * so device scratch is at most natoms * (nreps/C + C) * 3 * nstates floats
  * (twice that for epg_ssfp; rounded up to the kernel's state layout; epg_fisp
- * and epg_sr keep a segment's C states on chip and need none for them). */
+ * and epg_sr keep a segment's C states on chip and need none for them).
+ * Results do not depend on checkpoint_every; for epg_fisp and epg_sr (and
+ * snapmrf_crb_gradient's gradient) the number of atoms in a call chooses the
+ * lanes per atom, and sums over states follow them, so an atom's gradients may
+ * differ in their last bits between small and large calls. */
 int snapmrf_epg_adjoint(const float *d_params, int nparams, const float *h_mrf, size_t nreps,
                         size_t NREPS, size_t natoms, int nstates, const char *echo_type,
                         const float *d_grad_signal, float *d_signal, float *d_grad_params,

@@ -32,7 +32,6 @@
 namespace snapmrf {
 namespace grad {
 
-constexpr int kThreads = 128;
 // Threads per CTA of gn_kernel: one warp, so that no CTA barrier makes the
 // warps of a CTA wait for each other at every chunk (C1, three iterations:
 // 14.42 ms against 14.63 with 128 threads; identical maps).
@@ -263,23 +262,6 @@ __device__ __forceinline__ void pz(Pair3<P> &x) {
     for (int i = 0; i < P; i++) x.p[i] = x.m[i] = x.z[i] = make_float2(0.f, 0.f);
 }
 
-// RF pulse on one packed stream: F+' = c F+ + s F- - S Z, F-' = s F+ + c F-
-// + S Z, Z' = hS (F+ - F-) + C Z (hS = S / 2 with its sign), computed as
-// F-' = (c + s)(F+ + F-) - F+': 8 packed operations per pair instead of 9.
-template <int P>
-__device__ __forceinline__ void p_rf(Pair3<P> &x, float2 c, float2 s, float2 nS, float2 hS, float2 C) {
-    const float2 cs = __fadd2_rn(c, s);
-#pragma unroll
-    for (int i = 0; i < P; i++) {
-        const float2 p = x.p[i], m = x.m[i], q = x.z[i];
-        const float2 np = __ffma2_rn(nS, q, __ffma2_rn(s, m, __fmul2_rn(c, p)));
-        const float2 d = __fadd2_rn(p, make_float2(-m.x, -m.y));
-        x.z[i] = __ffma2_rn(C, q, __fmul2_rn(hS, d));
-        x.m[i] = __ffma2_rn(cs, p, __ffma2_rn(cs, m, make_float2(-np.x, -np.y)));
-        x.p[i] = np;
-    }
-}
-
 // The RF with the previous interval's relaxation folded in (the shift
 // commutes with relaxation, so relax(TR), shift, RF = shift, relax(TR), RF):
 // on the pre-relaxation state (p, m, z), F+' = c' p + s' m + nS' z,
@@ -311,7 +293,7 @@ __device__ __forceinline__ void p_rf_folded(Pair3<P> &x, const FoldedRF &k) {
 // width; a group's ends replace what they receive.
 template <int P>
 __device__ __forceinline__ void p_shift(Pair3<P> &x, int gl, int L, int w, const float2 *keep, int src_up,
-                                        int src_dn, bool padded) {
+                                        int src_dn) {
     const unsigned full = 0xffffffffu;
     const float up = __shfl_sync(full, x.p[P - 1].y, src_up);
     const float dn = __shfl_sync(full, x.m[0].x, src_dn);
@@ -323,11 +305,8 @@ __device__ __forceinline__ void p_shift(Pair3<P> &x, int gl, int L, int w, const
     for (int i = 0; i < P - 1; i++) x.m[i] = make_float2(x.m[i].y, x.m[i + 1].x);
     x.m[P - 1] = make_float2(x.m[P - 1].y, (gl == L - 1) ? 0.f : dn);
     if (gl == 0) x.p[0].x = -((w == 1) ? old_m0 : x.m[0].x);
-    // (no slot w without padding: the last lane's F- takes a zero instead)
-    if (padded) {
 #pragma unroll
-        for (int i = 0; i < P; i++) x.p[i] = __fmul2_rn(x.p[i], keep[i]);
-    }
+    for (int i = 0; i < P; i++) x.p[i] = __fmul2_rn(x.p[i], keep[i]);
 }
 
 // The refinement's streams hold states P apart in a pair (element h of pair i
@@ -839,7 +818,7 @@ __global__ void __launch_bounds__(32) adjoint_kernel(AdjArgs a) {
             x.z[0].x += k.fwd2.w;
         }
         const float y = x.p[0].x;
-        if (a.shift) p_shift<P>(x, gl, L, w, keep, src_up, src_dn, true);
+        if (a.shift) p_shift<P>(x, gl, L, w, keep, src_up, src_dn);
         return y;
     };
 
@@ -977,7 +956,9 @@ __global__ void __launch_bounds__(32) adjoint_kernel(AdjArgs a) {
 
 // Lanes and pairs per lane of the adjoint: two or four atoms per warp (fewer
 // shuffles per state) when that still gives every scheduler two warps, else
-// one atom per warp (a chain per step, which more lanes shorten).
+// one atom per warp (a chain per step, which more lanes shorten).  The sums
+// over an atom's states follow the lanes, so a gradient may differ in its last
+// bits between a call of few atoms and one of many; the signal does not.
 static void choose_adjoint(int w, size_t n, int *L, int *P) {
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -1395,7 +1376,8 @@ __global__ void __launch_bounds__(kCrbThreads) crb_adjoint_kernel(CrbArgs a) {
 // Lanes and states per lane of the CRB sweeps: one tissue per warp, the fewest
 // states per lane, while that leaves no scheduler more than one warp (each
 // step is a chain, and more lanes shorten it); more tissues than that share
-// warps in the adjoint's layout.
+// warps in the adjoint's layout.  The gradient's sums follow the lanes (last
+// bits); signals and losses do not.
 static void choose(int w, int *L, int *S);
 static void choose_crb(int w, size_t n, int *L, int *S) {
     int dev = 0, sms = 148;

@@ -513,7 +513,12 @@ constexpr int kRealChunk = 32;
 // to three warps per scheduler (the states take the registers; limits of 128
 // and 144 registers spill and take 6.2-6.5 ms).
 constexpr int kRealUnroll = 4;
-// Resident CTAs per SM asked of the compiler (168 registers at 12).
+// Resident CTAs per SM asked of the compiler (168 registers at 12).  With more
+// pairs a lane takes 208 to 254 registers, and still gains: 138,760 atoms, T =
+// 500, ms with pairs of neighbours (148 to 180 registers) and now: w = 50 (13
+// pairs) 1.70 / 1.40, 53 (14, padded) 2.50 / 2.13, 56 (14) 1.75 / 1.46, 57 (15,
+// padded) 2.86 / 2.27, 64 (16) 1.95 / 1.58; 45 and 49 (spilling 12-36 bytes)
+// 2.22 / 2.13 and 2.58 / 2.23.
 constexpr int real_min_ctas(int P) { return P <= 13 ? 12 : 1; }
 constexpr int kRealFS = kRealChunk * 4 + 4;        // floats per atom of relaxation factors
 constexpr int kRealReadoutStride = kRealChunk + 1;  // floats per atom
@@ -1026,7 +1031,7 @@ __global__ void __launch_bounds__(kEpgThreads) roa_iso_kernel(EpgArgs a, int G) 
                 py = __ffma2_rn(c, ny, py);
                 qy = __ffma2_rn(s, nx, qy);
                 const float2 ux = __ffma2_rn(S, ny, __fmul2_rn(C, nx));
-                    const float2 uy = __ffma2_rn(make_float2(-S.x, -S.y), nx, __fmul2_rn(C, ny));
+                const float2 uy = __ffma2_rn(make_float2(-S.x, -S.y), nx, __fmul2_rn(C, ny));
                 mx[2 * q] = ux.x;
                 mx[2 * q + 1] = ux.y;
                 my[2 * q] = uy.x;
