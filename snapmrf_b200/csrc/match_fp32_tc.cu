@@ -25,9 +25,10 @@
 //    cut at 2^-25 of the largest and the result cut to 24 bits, so
 //    (16 / 4 + 1) 2^-23 of it at each of a chunk's six MMAs (measured on the
 //    device with addends of 2^-22 .. 2^-29 beside a sum of 1, each sign: cut
-//    exactly there, never rounded up; NVIDIA documents no bound).  Summed over
-//    the chunks c, by Cauchy and Schwarz again: 92 2^-24 sqrt(sum_c
-//    ||d_1..c||^2) sqrt(sum_c ||x_1..c||^2), the weighted norms of both;
+//    exactly there, never rounded up; NVIDIA documents no bound), 60 2^-24 a
+//    chunk, 61 since hi may be 2^-8 longer than v.  Summed over the chunks c,
+//    by Cauchy and Schwarz again: 93 2^-24 sqrt(sum_c ||d_1..c||^2) sqrt(sum_c
+//    ||x_1..c||^2), the weighted norms of both;
 //  - what is left (the voxel's scaling, the squares and roots of the
 //    comparison) is 2^-22 of ||d||; 2^-20 is allowed, and 0.1 % on everything
 //    for what the bounds above neglect of second order.
@@ -36,11 +37,11 @@
 // 2.6e-4 complex; 3.8e-5 and 6.7e-5 at T = 200), where the scores were seen to
 // differ by 1.6e-5 at most.
 //
-// 57,600 voxels, 284,458 imaginary atoms in 41 blocks, T = 1000: 36.4 -> 4.9
+// 57,600 voxels, 284,458 imaginary atoms in 41 blocks, T = 1000: 36.4 -> 4.8
 // ms (packing 0.68, scores 2.9 = three BF16 products at 1.68 PFLOP/s, about
-// eight candidates per voxel in FP32 0.73, maps 0.11; the FP32 kernel alone
+// nine candidates per voxel in FP32 0.8, maps 0.11; the FP32 kernel alone
 // runs at 0.61 of the FP32 FMA peak); 4,096 voxels, 837 complex atoms: 0.80 ->
-// 0.21 ms.
+// 0.21 ms; fine grids: see list_cap.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -603,7 +604,7 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
     // (tests: as if a wait of every scoring launch had run out)
     const int wait_err = getenv("SNAPMRF_SCREEN_WAIT_ERROR") ? 1 : 0;
 
-    const float chain = 92.f * 0x1p-24f * (1.f + (float)K * 0x1p-22f);
+    const float chain = 93.f * 0x1p-24f * (1.f + (float)K * 0x1p-22f);
     auto aligned = [](const void *p, long long stride) {
         return stride % 2 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0;
     };
