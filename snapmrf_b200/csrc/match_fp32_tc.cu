@@ -563,6 +563,9 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
     const long long cap = ((nv_max + vt - 1) / vt + nbins) * vt;
     const long long arows = (q.imag ? 2 : 1) * cap, brows = rows * chunk * bins_per;
     if (arows > 0x7fffffffll || brows > 0x7fffffffll) return SNAPMRF_OK;
+    // (every block's voxels are padded to vt: thousands of blocks with few
+    // voxels each would take many times a pass's room)
+    if (cap * ((q.imag ? 2 : 1) * Kp * 2 + own_list) > 2 * (voxel_bytes + list_room)) return SNAPMRF_OK;
     const long long lslots = cap + tc::split_slots(cap / vt, num_sms) * vt;
 
     size_t bytes = 0;

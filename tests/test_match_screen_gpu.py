@@ -220,7 +220,8 @@ def _row_bytes(T, imag):
     (3, 700, 300, 1 << 20, 1 << 30),      # a block in chunks of 256, the last short
     (1, 3000, 600, 500, 1 << 30),         # chunks, and five ranges of voxels
     (4, 700, 100000, 500, 1 << 30),       # ranges of voxels alone
-    (1, 3000, 600, 100000, 1 << 23)])     # ranges from the lists' room
+    (1, 3000, 600, 100000, 1 << 23),      # ranges from the lists' room
+    (5, 700, 1500, 50, 1 << 16)])         # more padded slots than room: the FP32 kernel
 def test_passes(snap, monkeypatch, imag, nb, natoms, per_atoms, per_voxels, lists):
     """Dictionaries, images and lists larger than one pass: atom norms that
     rise and fall from chunk to chunk, blocks with and without voxels."""
