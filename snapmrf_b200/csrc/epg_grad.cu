@@ -907,15 +907,16 @@ __global__ void __launch_bounds__(32) adjoint_kernel(AdjArgs a) {
             }
         }
         __syncwarp();
-        for (int i = 0; i < n; i++) {
-            if (!(i & 1) && holds) {
+        for (int i = 0; i < n; i += 2) {
+            if (holds) {
                 float2 *d = mine + (size_t)(i / 2) * 3 * lanes * P;
                 put_pairs<P>(d, x.p);
                 put_pairs<P>(d + lanes * P, x.m);
                 put_pairs<P>(d + 2 * lanes * P, x.z);
             }
-            const float y = forward(x, sk[i]);
-            if (lane0) sf[i] = y;
+            float2 y = make_float2(forward(x, sk[i]), 0.f);
+            if (i + 1 < n) y.y = forward(x, sk[i + 1]);
+            if (lane0) *reinterpret_cast<float2 *>(sf + i) = y;  // (C is even)
         }
         for (int i = (n - 1) & ~1; i >= 0; i -= 2) {
             Pair3<P> s;
