@@ -19,27 +19,30 @@
 //  - the products left out, lo lo', rest v' and (hi + lo) rest', are inner
 //    products: at most ||lo_d|| ||lo_x|| + ||rest_d|| + ||d|| ||rest_x||
 //    (Cauchy and Schwarz), the norms summed while packing;
-//  - both sides round a running sum whose k-th value is at most
-//    ||d_1..k|| ||x_1..k||.  FP32: 2^-24 of it at each of the 32 elements of a
-//    chunk.  Tensor core: an MMA adds 16 products to the sum with every addend
-//    cut at 2^-25 of the largest and the result cut to 24 bits, so
-//    (16 / 4 + 1) 2^-23 of it at each of a chunk's six MMAs (measured on the
-//    device with addends of 2^-22 .. 2^-29 beside a sum of 1, each sign: cut
-//    exactly there, never rounded up; NVIDIA documents no bound), 60 2^-24 a
-//    chunk, 61 since hi may be 2^-8 longer than v.  Summed over the chunks c,
-//    by Cauchy and Schwarz again: 93 2^-24 sqrt(sum_c ||d_1..c||^2) sqrt(sum_c
-//    ||x_1..c||^2), the weighted norms of both;
+//  - both sides round a running sum, at most ||d|| ||x|| over the elements
+//    that it holds.  FP32: 2^-24 of it at each of the 32 elements of a chunk.
+//    Tensor core: an MMA adds 16 products to the sum with every addend cut at
+//    2^-25 of the largest and the result cut to 24 bits, so (16 / 4 + 1) 2^-23
+//    of it at each of a chunk's six MMAs (measured on the device with addends
+//    of 2^-22 .. 2^-29 beside a sum of 1, each sign: cut exactly there, never
+//    rounded up; NVIDIA documents no bound), 60 2^-24 a chunk, 61 since hi may
+//    be 2^-8 longer than v.  Summed over the chunks, by Cauchy and Schwarz
+//    again: sqrt(sum_c ||d_1..c||^2) sqrt(sum_c ||x_1..c||^2), the forward norms
+//    of both.  The tensor core takes the chunks from the last to the first,
+//    so its sum has the backward norms: atoms whose signal is over early
+//    (short T1 and T2) set the largest forward norm and have small backward
+//    ones, and both sums in one order would bound them a quarter higher;
 //  - what is left (the voxel's scaling, the squares and roots of the
 //    comparison) is 2^-22 of ||d||; 2^-20 is allowed, and 0.1 % on everything
 //    for what the bounds above neglect of second order.
 // The largest values of any atom of the dictionary stand for each.  On the
-// configurations' dictionaries the bound is 1.3e-4 (T = 1000, imaginary atoms;
-// 2.6e-4 complex; 3.8e-5 and 6.7e-5 at T = 200), where the scores were seen to
+// configurations' dictionaries the bound is 1.1e-4 (T = 1000, imaginary atoms;
+// 2.2e-4 complex; 2.8e-5 and 4.9e-5 at T = 200), where the scores were seen to
 // differ by 1.6e-5 at most.
 //
 // 57,600 voxels, 284,458 imaginary atoms in 41 blocks, T = 1000: 36.4 -> 4.8
 // ms (packing 0.68, scores 2.9 = three BF16 products at 1.68 PFLOP/s, about
-// nine candidates per voxel in FP32 0.8, maps 0.11; the FP32 kernel alone
+// eight candidates per voxel in FP32 0.8, maps 0.11; the FP32 kernel alone
 // runs at 0.61 of the FP32 FMA peak); 4,096 voxels, 837 complex atoms: 0.80 ->
 // 0.21 ms; fine grids: see list_cap.
 #include <cuda_bf16.h>
@@ -96,12 +99,12 @@ __global__ void init_kernel(unsigned long long *keys, long long nkeys, long long
     if (i < nkeys) keys[i] = 0ull;
     if (i < nperm) perm[i] = -1;
     if (i < nbins) counts[i] = fall_counts[i] = 0;
-    if (i == 0) *st = State{wait_err, 0, 0, {0u, 0u, 0u, 0u}};
+    if (i == 0) *st = State{wait_err, 0, 0, {0u, 0u, 0u, 0u, 0u}};
 }
 
 // Running sums of a row (see tc::AtomStats).
 struct RowSums {
-    float norm2 = 0.f, weighted2 = 0.f, lo2 = 0.f, rest2 = 0.f;
+    float norm2 = 0.f, forward2 = 0.f, backward2 = 0.f, lo2 = 0.f, rest2 = 0.f;
 };
 
 // hi and lo of two neighbouring elements, packed; the squares of lo and of
@@ -206,13 +209,15 @@ __global__ void pack_voxels_kernel(__nv_bfloat16 *A, tc::VoxelStats *stats, cons
             e = fmaf(a[u], a[u], e);
         }
         const long long k0 = IMAG ? t : 2 * t;
-        sums.weighted2 = fmaf((float)(Kp / (2 * KB) - k0 / KB), e, sums.weighted2);
+        sums.forward2 = fmaf((float)(Kp / (2 * KB) - k0 / KB), e, sums.forward2);
+        sums.backward2 = fmaf((float)(k0 / KB + 1), e, sums.backward2);
         store8(row, k0, a, sums);
         if (IMAG) store8(row + Kp, t, b, sums);
     }
-    const float w2 = warp_sum(sums.weighted2), l2 = warp_sum(sums.lo2), r2 = warp_sum(sums.rest2);
+    const float f2 = warp_sum(sums.forward2), b2 = warp_sum(sums.backward2);
+    const float l2 = warp_sum(sums.lo2), r2 = warp_sum(sums.rest2);
     if (lane == 0)
-        stats[slot] = {fit ? n : (n == 0.f && mx == 0.f) ? 0.f : -1.f, sqrtf(w2), sqrtf(l2), sqrtf(r2)};
+        stats[slot] = {fit ? n : (n == 0.f && mx == 0.f) ? 0.f : -1.f, sqrtf(f2), sqrtf(b2), sqrtf(l2), sqrtf(r2)};
 }
 
 // B rows of atoms [a0, a0 + n) (row r of the operand: atom a0 + r): one row
@@ -257,7 +262,8 @@ __global__ void pack_atoms_kernel(__nv_bfloat16 *B, const float2 *atoms, long lo
             }
             const long long k0 = IMAG ? t : 2 * t;
             sums.norm2 += e;
-            sums.weighted2 = fmaf((float)(Kp / (2 * KB) - k0 / KB), e, sums.weighted2);
+            sums.forward2 = fmaf((float)(Kp / (2 * KB) - k0 / KB), e, sums.forward2);
+            sums.backward2 = fmaf((float)(k0 / KB + 1), e, sums.backward2);
             store8(row, k0, a, sums);
             if (!IMAG) {
                 RowSums same;  // (the same elements, other signs)
@@ -265,7 +271,8 @@ __global__ void pack_atoms_kernel(__nv_bfloat16 *B, const float2 *atoms, long lo
             }
         }
     }
-    sums = {warp_sum(sums.norm2), warp_sum(sums.weighted2), warp_sum(sums.lo2), warp_sum(sums.rest2)};
+    sums = {warp_sum(sums.norm2), warp_sum(sums.forward2), warp_sum(sums.backward2), warp_sum(sums.lo2),
+            warp_sum(sums.rest2)};
     bad |= !(sums.norm2 <= kMaxNorm2);
     if (IMAG && __any_sync(0xffffffffu, real_part) && lane == 0) atomicCAS(err, 0, 7);
     if (__any_sync(0xffffffffu, bad)) {
@@ -274,7 +281,7 @@ __global__ void pack_atoms_kernel(__nv_bfloat16 *B, const float2 *atoms, long lo
     }
     if (lane == 0) srow[warp] = sums;
     __syncthreads();
-    if (threadIdx.x < 4) {
+    if (threadIdx.x < sizeof(RowSums) / sizeof(float)) {
         // one value per thread: one atomic per CTA, and only while it raises the value
         const int q = threadIdx.x;
         float mx = 0.f;
@@ -290,8 +297,8 @@ __global__ void pack_atoms_kernel(__nv_bfloat16 *B, const float2 *atoms, long lo
 // to the fall list.  One warp per slot (WIDE: one CTA, whose warps take the
 // batches in turn); lane c carries candidate c's chain (kBatch of them at a
 // time) through samples that cp.async stages kDepth steps of kSteps ahead.
-// The chain is serial by definition: 57,600 voxels of about ten candidates
-// 0.80 ms, their rows 4.6 GB from L2 (8-byte copies and reads 0.88, waiting
+// The chain is serial by definition: 57,600 voxels of about eight candidates
+// 0.77 ms, their rows 4.6 GB from L2 (8-byte copies and reads 0.88, waiting
 // for each candidate's load in turn 2.4 ms).
 constexpr int kRescoreWarps = 4, kMaxCand = 96, kBatch = 16, kSteps = 16, kDepth = 3;
 struct alignas(16) RescoreSmem {
@@ -318,7 +325,7 @@ __global__ void __launch_bounds__(kRescoreWarps * 32, 7)
 rescore_kernel(unsigned long long *keys, tc::Lists lists, int list_cap, const int *list_n, const float *list_best,
                const long long *perm, const tc::VoxelStats *vstats, const long long *tile_start, int bin_lo, int bin_hi,
                const int *vox_bin, const float2 *atoms, long long atom_stride, const float2 *img,
-               long long img_stride, int nreps, long long bin_natoms, float chain, State *st, int *fall,
+               long long img_stride, int nreps, long long bin_natoms, int nk, State *st, int *fall,
                int *fall_counts) {
     __shared__ RescoreSmem smem[kRescoreWarps];
     __shared__ float wide_s[kRescoreWarps];
@@ -359,7 +366,7 @@ rescore_kernel(unsigned long long *keys, tc::Lists lists, int list_cap, const in
     const bool over = n == tc::LIST_OVER;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
-    const float low = sqrtf(best) - tc::screen_margin(as, vs, chain);
+    const float low = sqrtf(best) - tc::screen_margin(as, vs, nk);
     if (__any_sync(0xffffffffu, over) || !(low > 0.f) || best * vs.norm2 < kMinNorm2) return leave();
     const float thr = low * low * (1.f - 0x1p-20f);
     const float2 *x = img + v * img_stride;
@@ -541,11 +548,11 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
     const long long chunk = bin_natoms <= fit ? bin_natoms : fit / apt * apt;
     // Entries per list: the atoms within the bound grow in number with the
     // grid's density (T = 1000, imaginary / complex, mean and most of 512
-    // voxels: 6,938 atoms 9, 27 / 17, 49; 41,588 51, 153 / 99, 294; 164,551
-    // 201, 599 / 390, 1,169; 334,125 408, 1,214 / 793, 2,364), over four / two
+    // voxels: 6,938 atoms 8, 24 / 15, 44; 41,588 45, 136 / 86, 262; 164,551
+    // 175, 536 / 340, 1,036; 334,125 356, 1,089 / 690, 2,109), over four / two
     // lists.  Full lists send the voxel to the FP32 kernel after the screen:
     // 4,096 voxels, 164,551 atoms 58.2 / 111 ms by that kernel alone, 63.4 /
-    // 121 with lists for 64 entries, 5.9 / 11.5 with these.
+    // 121 with lists for 64 entries, 5.8 / 11.2 with these.
     const int nlists = tc::split_lists(q.imag);
     int list_cap = 64;
     while (list_cap < 2048 && list_cap * 256ll < bin_natoms) list_cap *= 2;
@@ -607,7 +614,6 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
     // (tests: as if a wait of every scoring launch had run out)
     const int wait_err = getenv("SNAPMRF_SCREEN_WAIT_ERROR") ? 1 : 0;
 
-    const float chain = 93.f * 0x1p-24f * (1.f + (float)K * 0x1p-22f);
     auto aligned = [](const void *p, long long stride) {
         return stride % 2 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0;
     };
@@ -658,7 +664,6 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
         a.top_i = reinterpret_cast<int *>(b + oTi);
         a.plan = reinterpret_cast<tc::TailPlan *>(b + oPlan);
         a.list_cap = list_cap;
-        a.chain = chain;
         a.atom_stats = &state->atoms;
         a.vox_stats = vstats;
         a.list_n = reinterpret_cast<int *>(b + oLn);
@@ -672,8 +677,12 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
         lists.plan = a.plan;
         lists.cap = cap;
         lists.vt = vt;
-        // (long lists are of fine grids: batch after batch per voxel)
-        const bool wide = list_cap > 64;
+        // A CTA per voxel where fine grids (long lists) and long rows (a wide
+        // bound) give it several batches.  ms, a warp / a CTA: 4,096 voxels,
+        // 18,687 complex atoms, T = 1000 (list_cap nk = 8,064) 1.60 / 1.45,
+        // imaginary (4,096) 0.87 / 0.84, 1,024 voxels 0.43 / 0.35; 19,600
+        // complex bSSFP atoms, T = 400 (3,200) 0.56 / 0.61.
+        const bool wide = (long long)list_cap * nk >= 4096;
         auto pick = [&](auto vec_wide, auto vec, auto wd, auto plain) {
             return avec && ivec ? (wide ? vec_wide : vec) : (wide ? wd : plain);
         };
@@ -702,7 +711,8 @@ int match_fp32_screened(const ScreenRequest &q, cudaStream_t st, bool *done) {
             // (the next bins' launch uses the split items' lists again)
             rk<<<nblk(cap, wide ? 1 : kRescoreWarps), kRescoreWarps * 32, 0, st>>>(
                 keys, lists, list_cap, a.list_n, a.list_best, perm, vstats, tile_start, b0, b0 + nb, b1 ? vox_bin : nullptr,
-                q.atoms, q.atom_stride, img, q.img_stride, (int)q.nreps, bin_natoms, chain, state, fall, fall_counts);
+                q.atoms, q.atom_stride, img, q.img_stride, (int)q.nreps, bin_natoms, (int)nk, state, fall,
+                fall_counts);
             SNAPMRF_LAUNCH_CHECK();
         }
         fall_bins_kernel<<<1, 1024, 0, st>>>(state, fall, fall_counts, b1 ? vox_bin : nullptr, fslot, ftile, fcursor,

@@ -174,8 +174,10 @@ match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                         }
                         sm100::mbar_arrive_expect_tx(&full[stage], STAGE_BYTES);
                         unsigned char *sa = smem + stage * STAGE_BYTES;
-                        sm100::tma_load_2d(sa, &tmA, &full[stage], kc * BKE, vrow);
-                        sm100::tma_load_2d(sa + A_BYTES, &tmB, &full[stage], kc * BKE, brow);
+                        // (SPLIT: last chunk first, see match_fp32_tc.cu)
+                        const int k0 = (SPLIT ? p.nk - 1 - kc : kc) * BKE;
+                        sm100::tma_load_2d(sa, &tmA, &full[stage], k0, vrow);
+                        sm100::tma_load_2d(sa + A_BYTES, &tmB, &full[stage], k0, brow);
                         issued[stage] = (int)phase;
                         if (++stage == STAGES) {
                             stage = 0;
@@ -335,7 +337,7 @@ match_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 lbase = list_offset(lid, p.cap * LISTS, p.list_cap, parts);
                 lcap = part_cap(p.list_cap, parts);
                 margin = screen_margin(*p.atom_stats,
-                                       p.vox_stats[(item0 + u.item) * VPT + (IMAG ? row / 2 : row)], p.chain);
+                                       p.vox_stats[(item0 + u.item) * VPT + (IMAG ? row / 2 : row)], p.nk);
                 if (p.resume) {
                     ln = p.list_n[lid];
                     best = p.list_best[lid];

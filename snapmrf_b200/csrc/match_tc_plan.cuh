@@ -36,22 +36,24 @@ static_assert(SMEM_BYTES + 2 * BM * 8 + 512 <= 227 * 1024, "shared memory of one
 constexpr uint32_t TMEM_COLS = 512;
 
 // What the FP32 form's screen knows of its operands.  v = hi + lo + rest, hi
-// and lo its BF16 parts; weighted: sum of (nk - k / 32) v_k^2, nk chunks of 32
-// elements.  Atoms: the largest value of any (the bits of floats >= 0 order as
-// integers); voxels: of the slot's voxel at unit norm.
+// and lo its BF16 parts; with c = k / 32 the chunk of element k of nk chunks,
+// forward: sum of (nk - c) v_k^2, backward: of (c + 1) v_k^2.  Atoms: the largest
+// value of any (the bits of floats >= 0 order as integers); voxels: of the
+// slot's voxel at unit norm.
 struct AtomStats {
-    unsigned norm2, weighted2, lo2, rest2;
+    unsigned norm2, forward2, backward2, lo2, rest2;
 };
 struct VoxelStats {
-    float norm2;                // 0: nothing scores above 0; < 0: left to the FP32 kernel
-    float weighted, lo, rest;   // square roots
+    float norm2;                          // 0: nothing scores above 0; < 0: left to the FP32 kernel
+    float forward, backward, lo, rest;    // square roots
 };
 // Twice a bound of |approximate score - FP32 score| (the argument: match_fp32_tc.cu).
-__device__ __forceinline__ float screen_margin(const AtomStats &a, const VoxelStats &v, float chain) {
+__device__ __forceinline__ float screen_margin(const AtomStats &a, const VoxelStats &v, int nk) {
     auto root = [](unsigned bits) { return sqrtf(__uint_as_float(bits)); };
-    const float first = chain * root(a.weighted2) * v.weighted;
-    const float second = root(a.lo2) * v.lo + root(a.rest2) + root(a.norm2) * (v.rest + 0x1p-20f);
-    return 2.002f * (first + second);
+    const float sums = 0x1p-24f * (1.f + (float)nk * 0x1p-17f) *
+                       (32.f * root(a.forward2) * v.forward + 61.f * root(a.backward2) * v.backward);
+    const float parts = root(a.lo2) * v.lo + root(a.rest2) + root(a.norm2) * (v.rest + 0x1p-20f);
+    return 2.002f * (sums + parts);
 }
 
 struct Args {
@@ -73,7 +75,6 @@ struct Args {
     int *err;
     // SPLIT: candidates within screen_margin of the best score
     int list_cap;                 // entries per list
-    float chain;                  // see screen_margin
     const AtomStats *atom_stats;  // of the atoms packed so far
     const VoxelStats *vox_stats;  // [slots]
     int *list_n;                  // [slots][lists] entries, LIST_OVER: more than the list holds
