@@ -16,6 +16,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <map>
 #include <vector>
 
@@ -186,20 +187,38 @@ namespace tc {
 __global__ void publish_error_kernel(const int *err);
 }
 
-// Whether the FP32 form's screen pays for its launches.  Measured, T = 1000
-// (FP32 kernel / screened, us).  One block, random rows: voxels x atoms 64 x
-// 256 (2^24 products) 244 / 134, 256 x 256 249 / 127, 4,096 x 64 248 / 141,
-// 1,024 x 1,024 254 / 135, 4,096 x 837 828 / 200.  Below 2^24 the FP32
-// kernel's 240 us take fewer launches and no operands; below 32 voxels the
-// candidates' chains take as long: 32 x 4,096 248 / 239, 4 x 4,096 244 / 235.
-// Several blocks: how the voxels fall on them is not known here, and the FP32
-// kernel reads only blocks with voxels.  All in one of 41 blocks of 6,938
-// atoms, imaginary: 32 voxels 191 / 293, 100 288 / 297, 1,000 731 / 318;
-// complex (twice the operand, in three passes): 32 280 / 530, 320 466 / 534,
-// 1,000 1,269 / 550.  Over all 41: 100 voxels 1,716 / 946 and 3,196 / 2,924.
-// The lines lie where the first of these cost nothing.
-static bool screen_pays(long long nvox, long long bin_natoms, long long nreps, bool blocks, bool imag) {
-    return nvox >= (!blocks ? 32 : imag ? 96 : 384) && nvox * bin_natoms * nreps >= (1ll << 24);
+// Whether the FP32 form's screen (match_fp32_tc.cu) pays for its launches, the
+// packing and the candidates' chains, from what both sides were measured to
+// take, us:
+//   FP32 kernel  31 + t (26 + t complex) up to one CTA (64 voxels x 128 atoms)
+//                per SM, then t (0.9 per CTA and SM + 0.35), t = 4 + 0.12 T
+//                (4 + 0.206 T), T samples
+//   screened     64 + 0.045 T + 0.0023 atoms + 1.1e-5 atoms T + products / 1.5e8
+//                (58 + 0.045 T + 0.0024 atoms + 2.9e-5 atoms T + products / 1.1e8),
+//                and 1.6e-4 (2.5e-4) per atom of all blocks where there are several
+// On 360 sizes of both forms (32 to 4,096 voxels, 341 to 18,687 atoms, T = 50 to
+// 1,000, in one block and in one of 3 and of 41) the faster side is taken in all
+// but 17 cases, which lose 4 to 34 %.  For instance (FP32 kernel / screened),
+// imaginary: 256 x 2,739, T = 200 60 / 83, 1,024 124 / 85; 64 x 6,938, T = 1000
+// 161 / 212, 512 461 / 221; complex: 4,096 x 837 828 / 200.  With several
+// blocks the FP32 kernel reads only those that voxels fall into, and how they
+// fall is not known here: one block is assumed, where the screen gains least.
+// All voxels in one of 41 blocks of 6,938 atoms, T = 1000: 32 imaginary 191 /
+// 293, 1,000 731 / 323; 320 complex 466 / 500, 1,000 1,269 / 522; over all 41
+// blocks 100 imaginary 1,716 / 948, 1,000 1,726 / 1,030.
+// SNAPMRF_SCREEN=0 / 1 takes one side whatever the size.
+static bool screen_pays(long long nvox, long long bin_natoms, long long NATOMS, long long nreps, bool imag, int sms) {
+    if (const char *e = getenv("SNAPMRF_SCREEN")) return atoi(e) != 0;
+    const double T = (double)nreps, atoms = (double)bin_natoms, products = (double)nvox * atoms * T;
+    const bool blocks = NATOMS > bin_natoms;
+    const long long ctas = ((nvox + 63) / 64) * ((bin_natoms + 127) / 128);
+    const double per_sm = (double)ctas / sms, t = 4 + (imag ? 0.12 : 0.206) * T;
+    const double plain = (imag ? 31 : 26) + t * (per_sm <= 1 ? 1 : 0.9 * per_sm + 0.35);
+    const double screened =
+        (imag ? 64 + 0.045 * T + 0.0023 * atoms + 1.1e-5 * atoms * T + products / 1.5e8
+              : 58 + 0.045 * T + 0.0024 * atoms + 2.9e-5 * atoms * T + products / 1.1e8) +
+        (blocks ? (imag ? 1.6e-4 : 2.5e-4) * (double)NATOMS : 0);
+    return screened < plain;
 }
 
 static inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -577,9 +596,12 @@ extern "C" int snapmrf_mrf_match(float *d_maps, const float *img, int img_on_hos
     // Screened on the tensor cores where that applies (see match_fp32_tc.cu):
     // not for compressed scores, blocks with several B1 values, or calls too
     // small to pay for its launches.
+    int num_sms = 0, dev = 0;
+    SNAPMRF_CUDA(cudaGetDevice(&dev));
+    SNAPMRF_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
     const bool screen = !comp && !general &&
-                        screen_pays(nvox, (long long)(d_b1 ? natoms : NATOMS), (long long)nreps, d_b1 && nblocks > 1,
-                                    (flags & SNAPMRF_MATCH_IMAG_ATOMS) != 0);
+                        screen_pays(nvox, (long long)(d_b1 ? natoms : NATOMS), (long long)NATOMS, (long long)nreps,
+                                    (flags & SNAPMRF_MATCH_IMAG_ATOMS) != 0, num_sms);
     auto range = [&](long long v0, long long n) -> int {
         float *maps = d_maps + 5 * v0;
         int64_t *index = d_index ? d_index + v0 : nullptr;

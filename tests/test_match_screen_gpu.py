@@ -15,6 +15,12 @@ from gpu_util import torch_cuda
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def take_the_screen(monkeypatch):
+    """Whatever a call's size (the rule keeps small calls with the FP32 kernel)."""
+    monkeypatch.setenv("SNAPMRF_SCREEN", "1")
+
+
 def _both(snap, img, atoms, params, nreps, natoms, b1map=None, imag=False):
     torch = torch_cuda()
     N, stride = atoms.shape
@@ -291,3 +297,24 @@ def test_host_image_in_two_ranges(snap, use_map):
            for dev in (False, True)]
     np.testing.assert_array_equal(out[0][1], out[1][1])
     np.testing.assert_array_equal(out[0][0], out[1][0])
+
+
+@pytest.mark.parametrize("nvox,natoms,T,imag,screened", [
+    (300, 400, 64, True, False), (300, 400, 64, False, False), (1024, 2800, 200, True, True),
+    (4096, 837, 1000, False, True), (40, 6900, 1000, True, False), (5000, 20, 100, True, False)])
+def test_rule(snap, monkeypatch, nvox, natoms, T, imag, screened):
+    """Small calls stay with the FP32 kernel, which takes half the launches."""
+    atoms, img, params = _inputs(nvox, natoms, T, 1, imag, seed=5)
+    count = []
+    for force in ("0", "1", None):
+        if force is None:
+            monkeypatch.delenv("SNAPMRF_SCREEN")
+        else:
+            monkeypatch.setenv("SNAPMRF_SCREEN", force)
+        before = snap.kernel_launches()
+        a, b = _both(snap, img, atoms, params, T, natoms, None, imag)
+        count.append(snap.kernel_launches() - before)
+        np.testing.assert_array_equal(a[1], b[1])
+        np.testing.assert_array_equal(a[0], b[0])
+    assert count[0] < count[1]
+    assert count[2] == count[int(screened)]
