@@ -345,14 +345,15 @@ __device__ __forceinline__ void gn_shift(Pair3<P> &x, int gl, int L, int w, int 
     for (int i = 0; i < P - 1; i++) x.m[i] = x.m[i + 1];
     x.m[P - 1] = make_float2(mid_m, (gl == L - 1) ? 0.f : dn);
     if (gl == 0) x.p[0].x = w == 1 ? old_m0 : x.m[0].x;
-    // (no slot w without padding: the last lane's F- takes a zero instead)
+    // (no slot w without padding: the last lane's F- takes a zero instead.  A
+    // multiply, whose factors the loop keeps: with a select per slot 256 voxels,
+    // T = 1000, w = 50 take 345 us instead of 243, 57,600, T = 300, w = 41 1.65
+    // ms instead of 1.43)
     if (PAD) {
         const int j = w - gl * 2 * P;  // slot w in this lane
 #pragma unroll
-        for (int i = 0; i < P; i++) {
-            if (j == i) x.p[i].x = 0.f;
-            if (j == i + P) x.p[i].y = 0.f;
-        }
+        for (int i = 0; i < P; i++)
+            x.p[i] = __fmul2_rn(x.p[i], make_float2(j == i ? 0.f : 1.f, j == i + P ? 0.f : 1.f));
     }
 }
 
