@@ -1396,9 +1396,9 @@ static void choose_crb(int w, size_t n, int *L, int *S) {
 static size_t crb_forward_smem(int L) {
     return (size_t)(kCrbThreads / L) * kCrbChunk * (sizeof(CrbConst) + 3 * sizeof(float));
 }
-static size_t crb_adjoint_smem(int L, int S, int C) {
+static size_t crb_adjoint_smem(int L, int S, int C, bool on_chip) {
     return (size_t)C * ((size_t)(kCrbThreads / L) * (sizeof(CrbConst) + 3 * sizeof(float)) + 33 * sizeof(float) +
-                        (L == 32 ? 9 * (size_t)L * S * sizeof(float) : 0));
+                        (on_chip ? 9 * (size_t)L * S * sizeof(float) : 0));
 }
 
 static void choose(int w, int *L, int *S) {
@@ -1421,9 +1421,9 @@ static void choose(int w, int *L, int *S) {
         SNAPMRF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM)));        \
         k<<<GRID, kCrbThreads, SMEM, ST>>>(ARGS);                                                              \
     } while (0)
-#define SNAPMRF_CRB_DISPATCH(KERNEL, S, GRID, SMEM, ST, ARGS)                                                     \
+#define SNAPMRF_CRB_DISPATCH(KERNEL, S, WIDE, GRID, SMEM, ST, ARGS)                                               \
     do {                                                                                                       \
-        if ((ARGS).L == 32) SNAPMRF_CRB_DISPATCH_W(KERNEL, S, true, GRID, SMEM, ST, ARGS);                      \
+        if (WIDE) SNAPMRF_CRB_DISPATCH_W(KERNEL, S, true, GRID, SMEM, ST, ARGS);                      \
         else SNAPMRF_CRB_DISPATCH_W(KERNEL, S, false, GRID, SMEM, ST, ARGS);                                    \
     } while (0)
 
@@ -1772,7 +1772,7 @@ extern "C" int snapmrf_epg_jvp(const float *d_params, int nparams, const float *
     a.nckpt = 1;
     const int apc = kCrbThreads / L;
     dim3 grid((unsigned)((natoms + apc - 1) / apc));
-    SNAPMRF_CRB_DISPATCH(crb_forward_kernel, S, grid, crb_forward_smem(L), st, a);
+    SNAPMRF_CRB_DISPATCH(crb_forward_kernel, S, L == 32, grid, crb_forward_smem(L), st, a);
     SNAPMRF_LAUNCH_CHECK();
     return SNAPMRF_OK;
 }
@@ -1800,9 +1800,20 @@ extern "C" int snapmrf_crb_gradient(const float *d_params, int nparams, const fl
     const size_t n = ntissues;
     // a segment's constants, and with one tissue per warp its states, are kept
     // in shared memory: C is halved until they fit (the results do not depend
-    // on it)
-    const bool on_chip = L == 32;
-    while (crb_adjoint_smem(L, S, C) > kMaxSmem) C = (C + 1) / 2;
+    // on it).  The states only while all tissues' warps are resident at once:
+    // they leave an SM two warps or even one (T = 1000, us, shared / global
+    // memory: 592 tissues w = 20 464 / 745, w = 50 (two warps) 937 / 776; 148
+    // tissues w = 256 1,459 / 2,138, 1,200 10,161 / 6,579).
+    int sms = 148, dev = 0;
+    SNAPMRF_CUDA(cudaGetDevice(&dev));
+    SNAPMRF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    constexpr size_t kSmPerSm = 228 * 1024, kSmReserved = 1024;
+    int C_chip = C;
+    while (crb_adjoint_smem(L, S, C_chip, true) > kMaxSmem) C_chip = (C_chip + 1) / 2;
+    const bool on_chip =
+        L == 32 && n <= (size_t)sms * (kSmPerSm / (crb_adjoint_smem(L, S, C_chip, true) + kSmReserved));
+    if (on_chip) C = C_chip;
+    while (crb_adjoint_smem(L, S, C, on_chip) > kMaxSmem) C = (C + 1) / 2;
     const int nckpt = (int)((nreps + C - 1) / C);
     const size_t nf = n * 3 * nreps, ck = n * (size_t)nckpt * 9 * LS, sg = on_chip ? 0 : n * (size_t)C * 9 * LS,
                  ga = n * nreps, part = (size_t)kSplits * nreps;
@@ -1827,11 +1838,11 @@ extern "C" int snapmrf_crb_gradient(const float *d_params, int nparams, const fl
     float *partial = a.galpha + ga;
     const int apc = kCrbThreads / L;
     dim3 grid((unsigned)((n + apc - 1) / apc));
-    SNAPMRF_CRB_DISPATCH(crb_forward_kernel, S, grid, crb_forward_smem(L), st, a);
+    SNAPMRF_CRB_DISPATCH(crb_forward_kernel, S, L == 32, grid, crb_forward_smem(L), st, a);
     SNAPMRF_LAUNCH_CHECK();
     crb_loss_kernel<<<(unsigned)n, 256, 0, st>>>(a.fvec, base + nf, d_loss, d_params, nparams, (int)nreps);
     SNAPMRF_LAUNCH_CHECK();
-    SNAPMRF_CRB_DISPATCH(crb_adjoint_kernel, S, grid, crb_adjoint_smem(L, S, C), st, a);
+    SNAPMRF_CRB_DISPATCH(crb_adjoint_kernel, S, on_chip, grid, crb_adjoint_smem(L, S, C, on_chip), st, a);
     SNAPMRF_LAUNCH_CHECK();
     return sum_columns(d_grad_alpha, partial, a.galpha, (long long)n, (int)nreps, st);
 }

@@ -127,3 +127,21 @@ def test_adjoint_of_a_vanished_t2(snap, n):
         out.append(_adjoint(snap, torch, p, g.contiguous(), h, 20, "epg_fisp"))
     for x, y in zip(*out):
         assert torch.isfinite(x).all() and torch.equal(x, y)
+
+
+@pytest.mark.parametrize("w,n", [(50, 450), (100, 390), (200, 160), (256, 200)])
+def test_crb_of_more_tissues_than_shared_memory_holds(snap, w, n):
+    """One tissue per warp, the segments' states in global memory: losses and
+    signals bit for bit those of a few tissues, whose states are on chip."""
+    torch = torch_cuda()
+    h = mrf_schedule(T, seed=w + 7, inversion=False)
+    out = []
+    p = torch.from_numpy(_params(2, w)).cuda()
+    for q in (p, p.repeat(n // 2, 1).contiguous()):
+        loss, ga, sig = (torch.empty(s, device="cuda") for s in ((len(q),), (T,), (len(q), 3, T)))
+        snap.crb_gradient(q, h, T, T, len(q), loss, ga, 4, w, "epg_fisp", d_signals=sig, checkpoint_every=T // 2)
+        out.append((loss, ga.double(), sig))
+    (loss, ga, sig), (loss_n, ga_n, sig_n) = out
+    assert torch.equal(sig_n[-2:], sig) and torch.equal(loss_n[:2], loss)
+    assert torch.isfinite(ga).all()
+    assert (ga_n / (n // 2) - ga).abs().max() <= 1e-5 * ga.abs().max()
