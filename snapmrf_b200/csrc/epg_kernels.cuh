@@ -455,13 +455,15 @@ __device__ __forceinline__ void rl2_relax(RealLane2<P> &s, float E1, float E2, b
 // so a pair moves as a whole: only the pair that takes the neighbour's state
 // is put together anew.
 //
-// TAIL: the layout pads at most two slots (w >= 2P L - 2).  Slots k >= w
-// then hold zeros before the shift, so F-[w-1] takes the zero of F-[w] and
-// only F+[w], which receives F+[w-1], must be cleared.  That slot is the
+// Slots k >= w hold zeros before the shift, so F-[w-1] takes the zero of F-[w]
+// and only F+[w], which receives F+[w-1], must be cleared: by a multiply per
+// pair whose factors the step loop keeps (a compare and a select per slot took
+// w = 49, 53 and 61 from 1.45, 1.43 and 1.59 to 2.16, 2.06 and 2.16 ms, 138,760
+// atoms, T = 500).
+// TAIL: the layout pads at most two slots (w >= 2P L - 2).  That slot is then the
 // second of the last lane's last pair (or of the one before it), and
 // tail_keep (0 there, 1 elsewhere; .x the pair before the last, .y the last)
-// clears it with a multiply instead of a compare per slot; every non-zero
-// value is the same as with the per-slot masks.
+// clears it with one multiply.
 // NEG: s.fm holds -F-.
 template <int P, bool TAIL, bool NEG>
 __device__ __forceinline__ void rl2_shift(RealLane2<P> &s, int gl, int L, int w, float2 tail_keep) {
@@ -487,14 +489,10 @@ __device__ __forceinline__ void rl2_shift(RealLane2<P> &s, int gl, int L, int w,
             s.fp[0].x *= tail_keep.x;
         return;
     }
-    const int k0 = gl * 2 * P;
+    const int j = w - gl * 2 * P;  // slot w in this lane
 #pragma unroll
-    for (int i = 0; i < P; i++) {
-        if (k0 + i >= w) s.fp[i].x = 0.f;
-        if (k0 + P + i >= w) s.fp[i].y = 0.f;
-        if (k0 + i == w - 1) s.fm[i].x = 0.f;
-        if (k0 + P + i == w - 1) s.fm[i].y = 0.f;
-    }
+    for (int i = 0; i < P; i++)
+        s.fp[i] = __fmul2_rn(s.fp[i], make_float2(j == i ? 0.f : 1.f, j == P + i ? 0.f : 1.f));
 }
 
 // The real-valued kernel: one warp per CTA, so that no CTA barrier makes the
@@ -514,11 +512,11 @@ constexpr int kRealChunk = 32;
 // and 144 registers spill and take 6.2-6.5 ms).
 constexpr int kRealUnroll = 4;
 // Resident CTAs per SM asked of the compiler (168 registers at 12).  With more
-// pairs a lane takes 208 to 254 registers, and still gains: 138,760 atoms, T =
+// pairs a lane takes 208 to 255 registers, and still gains: 138,760 atoms, T =
 // 500, ms with pairs of neighbours (148 to 180 registers) and now: w = 50 (13
-// pairs) 1.70 / 1.40, 53 (14, padded) 2.50 / 2.13, 56 (14) 1.75 / 1.46, 57 (15,
-// padded) 2.86 / 2.27, 64 (16) 1.95 / 1.58; 45 and 49 (spilling 12-36 bytes)
-// 2.22 / 2.13 and 2.58 / 2.23.
+// pairs) 1.63 / 1.28, 53 (14, padded) 2.43 / 1.43, 56 (14) 1.67 / 1.38, 57 (15,
+// padded) 2.79 / 1.51, 64 (16) 1.87 / 1.50; 45 and 49 (padded) 2.15 / 1.37 and
+// 2.51 / 1.45.
 constexpr int real_min_ctas(int P) { return P <= 13 ? 12 : 1; }
 constexpr int kRealFS = kRealChunk * 4 + 4;        // floats per atom of relaxation factors
 constexpr int kRealReadoutStride = kRealChunk + 1;  // floats per atom
