@@ -319,10 +319,11 @@ typedef struct snapmrf_match_opts {
  * largest |<atom, voxel>| wins; blocks are merged by nearest B1 when a B1
  * map is given (ties to the lower block, differences >= 10 to block 0),
  * otherwise by the largest PD (ties to the lower block).
- * Scratch: the tensor-core forms pack both operands.  FP32 matching does from
- * 2^24 products on (32 voxels; 96 or 384 against several B1 blocks): nreps
- * floats per purely imaginary atom, 4 nreps per complex atom, 2 nreps per
- * voxel, at most 2 GB and 1 GB in a pass, and up to 1 GB of candidate lists.
+ * Scratch: the tensor-core forms pack both operands.  FP32 matching does too,
+ * but for small calls (below some 1e8 products of an atom's and a voxel's
+ * samples): nreps floats per purely imaginary atom, 4 nreps per complex atom,
+ * 2 nreps per voxel, at most 2 GB and 1 GB in a pass, and up to 1 GB of
+ * candidate lists.
  * It comes from the library's pool, which keeps it for the next call
  * (snapmrf_release_scratch gives it back).  An FP32 call that cannot have it,
  * or whose tensor-core kernel gives up a wait, is matched without (a few MB). */
